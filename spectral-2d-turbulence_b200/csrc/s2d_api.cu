@@ -116,10 +116,10 @@ static int check_device(int dev) {
 struct GraphKey {
   int phase, slot, parity;
   unsigned flags;
-  int ptr, prof;
+  int ptr, prof, banded;
   bool operator<(const GraphKey& o) const {
-    return std::tie(phase, slot, parity, flags, ptr, prof) <
-           std::tie(o.phase, o.slot, o.parity, o.flags, o.ptr, o.prof);
+    return std::tie(phase, slot, parity, flags, ptr, prof, banded) <
+           std::tie(o.phase, o.slot, o.parity, o.flags, o.ptr, o.prof, o.banded);
   }
 };
 
@@ -184,6 +184,12 @@ struct s2d_solver {
   char* tctab = nullptr;              // tensor-core DFT32 planes + twiddle matrix (fft 'tc-f16')
   int* row_nz = nullptr;              // per ky row: the last row-kernel pass wrote a nonzero PA/PB row
   bool packs_flagged = false;         // PA/PB rows flagged zero were left unwritten
+  bool packs_pairs = false;           // ... by the pair kernel (rows outside the band)
+  bool packs_half = false;            // ... which also left the rows ky < 0 of PB unwritten
+  // every cell of the state ring outside the dealias band is zero (seeds, steps); a caller may
+  // store other states, which the pair kernels do not take
+  bool banded = true;
+  float4* ptw = nullptr;              // pass-ordered twiddles of the pair kernels
   uchar4* image = nullptr;            // headless render target, grown on demand
   size_t image_px = 0;
   ushort4* dye[3] = {nullptr, nullptr, nullptr};
@@ -302,7 +308,7 @@ static void free_solver(s2d_solver* s) {
   }
   s->prof_events.clear();
   void* dev_ptrs[] = {s->state[0], s->state[1], s->state[2], s->packA, s->packB, s->physZ, s->rhs,
-                      s->force, s->vel, s->tw, s->partials, s->ticket, s->dparams, s->diag, s->seed_parts,
+                      s->force, s->vel, s->tw, s->ptw, s->partials, s->ticket, s->dparams, s->diag, s->seed_parts,
                       s->step_counter, s->err, s->tctab, s->row_nz, s->image, s->dye[0], s->dye[1], s->dye[2]};
   for (void* p : dev_ptrs)
     if (p) cudaFree(p);
@@ -591,13 +597,33 @@ template <class P> static void tc_rows_launch(int mode, bool ptr, const SpecArgs
   }
 }
 static bool is_tc(const s2d_solver* s) { return s->fft_precision != S2D_FFT_FP32; }
+// The stage kernels of the next launch: the chosen shapes, except that the pair kernels need a
+// dealiased state, and the pair column kernel also rows written by the pair row kernel (it
+// reads PB's rows ky >= 0 as the Hermitian half they then are).
+static int spec_shape(const s2d_solver* s) {
+  return s->ops->spec[s->spec_choice].pairs && !s->banded ? kAnyState : s->spec_choice;
+}
+static bool pair_rows(const s2d_solver* s) { return !tc_rows(s) && s->ops->spec[spec_shape(s)].pairs; }
+static int phys_shape(const s2d_solver* s) {
+  return s->ops->phys[s->phys_choice].pairs && !pair_rows(s) ? kAnyState : s->phys_choice;
+}
+static bool pair_cols(const s2d_solver* s) { return !is_tc(s) && s->ops->phys[phys_shape(s)].pairs; }
+// the packs are now those a row-stage launch writes
+static void mark_packs(s2d_solver* s) {
+  s->packs_valid = true;
+  s->packs_flagged = true;
+  s->packs_pairs = pair_rows(s);
+  s->packs_half = s->packs_pairs && pair_cols(s);
+}
 // the row stage with the solver's chosen variant
-static void run_spec(s2d_solver* s, int mode, bool ptr, const SpecArgs& a) {
+static void run_spec(s2d_solver* s, int mode, bool ptr, SpecArgs a) {
+  a.ptw = s->ptw;
+  a.full_pb = pair_cols(s) ? 0 : 1;
   if (tc_rows(s)) {
     if (s->fft_precision == S2D_FFT_TC_BF16) tc_rows_launch<tc::PrecBF16>(mode, ptr, a, s->tctab, s->stream);
     else tc_rows_launch<tc::PrecF16>(mode, ptr, a, s->tctab, s->stream);
   } else {
-    s->ops->spec[s->spec_choice].run(mode, ptr, a, s->stream);
+    s->ops->spec[spec_shape(s)].run(mode, ptr, a, s->stream);
   }
 }
 
@@ -654,6 +680,7 @@ extern "C" int s2d_create(int n, int dye_scale, int fft_precision, int device, s
   TRY(cudaMalloc(&s->force, cbytes), "force");
   TRY(cudaMalloc(&s->vel, cbytes), "vel");
   TRY(cudaMalloc(&s->tw, sizeof(float2) * n), "twiddles");
+  TRY(cudaMalloc(&s->ptw, sizeof(float4) * ops->ptw_size), "twiddles");
   // column-kernel grids are at most n CTAs in every registered shape
   const int nparts = std::max(std::max(n, 256), seed_parts_count(n));
   TRY(cudaMalloc(&s->partials, sizeof(float) * nparts), "partials");
@@ -699,6 +726,8 @@ extern "C" int s2d_create(int n, int dye_scale, int fft_precision, int device, s
   TRY(cudaMemsetAsync(s->partials, 0, sizeof(float) * nparts, s->stream), "memset");
   for (int i = 0; i < 3; ++i) TRY(cudaMemsetAsync(s->dye[i], 0, dbytes, s->stream), "memset");
   k_twiddles<<<(n + 255) / 256, 256, 0, s->stream>>>(s->tw, n);
+  TRY(cudaGetLastError(), "twiddle kernel");
+  ops->make_ptw(s->ptw, s->tw, s->stream);
   TRY(cudaGetLastError(), "twiddle kernel");
   if (fft_precision != S2D_FFT_FP32 && n == 1024) {
     TRY(cudaMalloc(&s->tctab, tc::kTabBytes), "tensor-core tables");
@@ -906,10 +935,14 @@ static int enqueue_pack_prime(s2d_solver* s) {
   a.tw = s->tw;
   a.err = s->err;
   a.row_nz = s->row_nz;
+  if (pair_rows(s)) {
+    // the pair kernel writes the in-band rows whatever they hold: its flags do not change
+    k_band_flags<<<(s->n + 255) / 256, 256, 0, s->stream>>>(s->row_nz, s->n);
+    S2D_LAUNCHED();
+  }
   run_spec(s, -1, false, a);
   S2D_LAUNCHED();
-  s->packs_flagged = true;
-  s->packs_valid = true;
+  mark_packs(s);
   return S2D_OK;
 }
 
@@ -917,7 +950,10 @@ static int enqueue_pack_prime(s2d_solver* s) {
 // other than the fused stage kernels reads or writes the packs
 static int materialize_packs(s2d_solver* s) {
   if (!s->packs_flagged) return S2D_OK;
-  k_zero_flagged_rows<<<cells_grid(s->n), 256, 0, s->stream>>>(s->packA, s->packB, s->row_nz, s->n);
+  if (s->packs_pairs)
+    k_expand_packs<<<cells_grid(s->n), 256, 0, s->stream>>>(s->packA, s->packB, s->n, s->packs_half ? 1 : 0);
+  else
+    k_zero_flagged_rows<<<cells_grid(s->n), 256, 0, s->stream>>>(s->packA, s->packB, s->row_nz, s->n);
   S2D_LAUNCHED();
   s->packs_flagged = false;
   return S2D_OK;
@@ -934,6 +970,7 @@ static PhysArgs phys_args(s2d_solver* s, int reduce) {
   a.dt_out = dt_slot(s, s->slot ^ 1);
   a.params = s->dparams;
   a.tw = s->tw;
+  a.ptw = s->ptw;
   a.reduce = reduce;
   a.row_nz = s->row_nz;
   return a;
@@ -946,7 +983,7 @@ static void enqueue_phys_cols(s2d_solver* s, int mode, const PhysArgs& a) {
     if (s->fft_precision == S2D_FFT_TC_BF16) tc_cols_launch<tc::PrecBF16>(mode, a, s->tctab, s->err, s->stream);
     else tc_cols_launch<tc::PrecF16>(mode, a, s->tctab, s->err, s->stream);
   } else {
-    s->ops->phys[s->phys_choice].run(mode, a, s->stream);
+    s->ops->phys[phys_shape(s)].run(mode, a, s->stream);
   }
 }
 
@@ -1067,10 +1104,9 @@ extern "C" int s2d_encode_step(s2d_solver* s) {
     a.row_nz = s->row_nz;
     run_spec(s, st, ptr, a);
     S2D_LAUNCHED();
-    s->packs_flagged = true;
   }
   s->reduced_valid = true;
-  s->packs_valid = true;
+  mark_packs(s);
   s->phase = (p + 1) % 3;
   s->step_index += 1;
   return S2D_OK;
@@ -1192,7 +1228,7 @@ extern "C" int s2d_step_graph(s2d_solver* s, int substeps, unsigned flags) {
   if (flags & S2D_STEP_RELATCH)
     if (int rc = sync_step_counter(s)) return rc;
   for (int i = 0; i < substeps; ++i) {
-    const GraphKey key{s->phase, s->slot, s->dye_parity, flags, s->hs.count > 0 ? 1 : 0, s->profiling ? 1 : 0};
+    const GraphKey key{s->phase, s->slot, s->dye_parity, flags, s->hs.count > 0 ? 1 : 0, s->profiling ? 1 : 0, s->banded ? 1 : 0};
     auto it = s->graphs.find(key);
     if (it == s->graphs.end()) {
       // capture one substep from the current host state, then restore it
@@ -1246,7 +1282,8 @@ extern "C" int s2d_step_graph(s2d_solver* s, int substeps, unsigned flags) {
     // advance the host mirror exactly as the captured substep did
     s->phase = (s->phase + 1) % 3;
     s->step_index += 1;
-    s->packs_valid = true;
+    if (tc_unfused(s)) s->packs_valid = true;
+    else mark_packs(s);
     s->reduced_valid = true;
     if (flags & S2D_STEP_DYE) s->dye_parity ^= 1;
     if (flags & S2D_STEP_REDUCE) {
@@ -1354,7 +1391,9 @@ extern "C" int s2d_read_diagnostics_fixed(s2d_solver* s, float* spectrum, float*
 }
 
 // ------------------------------------------------------------------ seeding
+// the rest of the state ring after a seed (state 0, dealiased)
 static int zero_other_states(s2d_solver* s) {
+  s->banded = true;
   const size_t cbytes = (size_t)s->n * s->n * sizeof(float2);
   S2D_CUDA(cudaMemsetAsync(s->state[1], 0, cbytes, s->stream));
   S2D_CUDA(cudaMemsetAsync(s->state[2], 0, cbytes, s->stream));
@@ -1526,6 +1565,7 @@ extern "C" int s2d_tune_select(s2d_solver* s, int phys, int spec) {
   DeviceGuard guard(s->dev);
   s->phys_choice = phys;
   s->spec_choice = spec;
+  s->packs_valid = false;   // the packs are laid out for the previous shapes
   drop_graphs(s);   // captured steps hold the previous shapes' kernels
   return S2D_OK;
 }
@@ -1722,6 +1762,7 @@ extern "C" int s2d_set_buffer(s2d_solver* s, int id, const void* host, size_t by
     if (int rc = materialize_packs(s)) return rc;
   S2D_CUDA(cudaMemcpyAsync(p, host, bytes, cudaMemcpyHostToDevice, s->stream));
   S2D_CUDA(cudaStreamSynchronize(s->stream));
+  if (id <= S2D_BUF_STATE2 && !band_limited(static_cast<const float*>(host), bytes / sizeof(float), s->n)) s->banded = false;
   if (id <= S2D_BUF_PACKB) s->packs_valid = false;
   if (id == S2D_BUF_VEL) s->reduced_valid = false;
   return S2D_OK;
@@ -1790,6 +1831,7 @@ extern "C" int s2d_rk3_stage(s2d_solver* s, int stage) {
   else k_rk3<2><<<g, 256, 0, s->stream>>>(w0, wc, wo, s->rhs, dt, s->dparams, s->n);
   S2D_LAUNCHED();
   s->packs_valid = false;
+  s->banded = false;   // rhs is the caller's
   return S2D_OK;
 }
 

@@ -10,6 +10,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+
 #include <cstring>
 #include <map>
 #include <string>
@@ -18,6 +19,7 @@
 #include "../../include/s2d.h"
 #include "s2d_band.cuh"
 #include "s2d_kernels.cuh"
+#include "s2d_pairs.cuh"
 
 using namespace s2d;
 
@@ -43,10 +45,10 @@ struct EnsInst {
   DevParams p;           // per-instance coefficients
   float dt;              // fixed step
   int n;
-  int tiles_a, tiles_b;
   long long off;         // first cell in the pooled arrays
   long long roff;        // first row in the pooled row flags
   const float2* tw;      // twiddle table of this n
+  const float4* ptw;     // pass-ordered twiddles of this n (pair kernels)
 };
 
 constexpr int kEnsAThreads = 256;
@@ -73,6 +75,18 @@ constexpr size_t kEnsBBarOff =
          Tune<1024>::B_SMEM);
 constexpr size_t kEnsBSmem = kEnsBBarOff + 16;
 
+// Pair kernels (dealiased states): 128 threads at every size, so 128 / T row pairs or column
+// pairs per item -- a 128-thread CTA synchronises at most four warps, and four of them share
+// an SM.
+constexpr int kEnsPairThreads = 128, kEnsPairMinb = 4;
+template <int N>
+using EnsPair = PairTune<N, 8, kEnsPairThreads / (N / 8), kEnsPairThreads, kEnsPairMinb, kEnsPairMinb>;
+// the same bytes at every size: (9/8) N elements of 24 bytes for each of 1024 / N pairs
+constexpr size_t kEnsPairSmem = EnsPair<1024>::B_SMEM;
+static_assert(EnsPair<64>::A_SMEM == kEnsPairSmem && EnsPair<64>::B_SMEM == kEnsPairSmem &&
+                  EnsPair<256>::A_SMEM == kEnsPairSmem && EnsPair<1024>::A_SMEM == kEnsPairSmem,
+              "one shared-memory size for every grid size");
+
 struct Pools {
   float2* s[3];
   float2 *pa, *pb, *z;
@@ -80,6 +94,64 @@ struct Pools {
   // (the column pass reads no such row); starts at "may be nonzero"
   int* row_nz;
 };
+
+__global__ void __launch_bounds__(kEnsPairThreads, kEnsPairMinb)
+    k_ens_pair_cols(const EnsInst* __restrict__ inst, const int2* __restrict__ items, int nitems, Pools pool) {
+  extern __shared__ __align__(16) float4 smem4[];
+  for (int k = blockIdx.x; k < nitems; k += gridDim.x) {
+    const int2 it = items[k];
+    const EnsInst& I = inst[it.x];
+    PhysArgs a{};
+    a.pa = pool.pa + I.off;
+    a.pb = pool.pb + I.off;
+    a.z = pool.z + I.off;
+    a.ptw = I.ptw;
+    switch (I.n) {
+      case 64: pair_cols_tile<1, EnsPair<64>>(a, it.y, smem4); break;
+      case 128: pair_cols_tile<1, EnsPair<128>>(a, it.y, smem4); break;
+      case 256: pair_cols_tile<1, EnsPair<256>>(a, it.y, smem4); break;
+      case 512: pair_cols_tile<1, EnsPair<512>>(a, it.y, smem4); break;
+      default: pair_cols_tile<1, EnsPair<1024>>(a, it.y, smem4); break;
+    }
+    __syncthreads();
+  }
+}
+template <int MODE>
+__global__ void __launch_bounds__(kEnsPairThreads, kEnsPairMinb)
+    k_ens_pair_rows(const EnsInst* __restrict__ inst, const int2* __restrict__ items, int nitems, Pools pool, int phase,
+                    int full_pb) {
+  extern __shared__ __align__(16) float4 smem4[];
+  constexpr int st = MODE < 0 ? 0 : MODE;
+  for (int k = blockIdx.x; k < nitems; k += gridDim.x) {
+    const int2 it = items[k];
+    const EnsInst& I = inst[it.x];
+    SpecArgs a{};
+    a.z = pool.z + I.off;
+    a.w0 = pool.s[phase] + I.off;
+    a.wcur = pool.s[(phase + st) % 3] + I.off;
+    a.wout = pool.s[(phase + (st == 1 ? 2 : 1)) % 3] + I.off;
+    a.pa = pool.pa + I.off;
+    a.pb = pool.pb + I.off;
+    a.dt = &I.dt;
+    a.params = &I.p;
+    a.ptw = I.ptw;
+    a.stochastic = I.p.force_amp > 0.f ? 1 : 0;
+    a.full_pb = full_pb;
+    switch (I.n) {
+      case 64: pair_rows_tile<MODE, false, EnsPair<64>>(a, it.y, smem4); break;
+      case 128: pair_rows_tile<MODE, false, EnsPair<128>>(a, it.y, smem4); break;
+      case 256: pair_rows_tile<MODE, false, EnsPair<256>>(a, it.y, smem4); break;
+      case 512: pair_rows_tile<MODE, false, EnsPair<512>>(a, it.y, smem4); break;
+      default: pair_rows_tile<MODE, false, EnsPair<1024>>(a, it.y, smem4); break;
+    }
+    __syncthreads();
+  }
+}
+// row flags of packs written by the pair kernel: the in-band rows of every instance
+__global__ void k_ens_band_flags(const EnsInst* __restrict__ inst, int* row_nz) {
+  const EnsInst& I = inst[blockIdx.x];
+  for (int r = threadIdx.x; r < I.n; r += blockDim.x) row_nz[I.roff + r] = (r <= I.n / 3 || r >= I.n - I.n / 3) ? 1 : 0;
+}
 
 // MINB: resident CTAs per SM the register allocation must allow (a tuned choice)
 template <int MINB>
@@ -154,48 +226,63 @@ __global__ void __launch_bounds__(kEnsBThreads, MINB)
   }
 }
 
-// ---- launch-shape variants of the two persistent stage kernels (index 0 = default)
-constexpr int kEnsPhysMinb[] = {2, 3};      // resident CTAs per SM of each shape
-constexpr int kEnsSpecMinb[] = {6, 4, 5, 4};
-constexpr bool kEnsSpecPair[] = {false, false, false, true};
+// ---- launch shapes of the two stage kernels: 0 (default) = pair kernels, for dealiased
+// states; the others take any state
+constexpr int kEnsAnyState = 1;
+constexpr int kEnsPhysMinb[] = {kEnsPairMinb, 2};      // resident CTAs per SM of each shape
+constexpr int kEnsSpecMinb[] = {kEnsPairMinb, 6, 4, 4};
+constexpr const char* kEnsPhysNote[] = {", column pairs", ""};
+constexpr const char* kEnsSpecNote[] = {", row pairs", "", "", ", paired inverse transforms"};
 constexpr int kEnsNPhys = 2, kEnsNSpec = 4;
 
-template <int MINB> cudaError_t ens_phys_attrs() {
-  return cudaFuncSetAttribute(k_ens_phys<MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEnsASmem);
+template <class K> cudaError_t ens_smem(K k, size_t bytes) {
+  return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
-template <int MINB, bool PAIR = false> cudaError_t ens_spec_attrs() {
-  cudaError_t e = cudaFuncSetAttribute(k_ens_spec<-1, MINB, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEnsBSmem);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ens_spec<0, MINB, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEnsBSmem);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ens_spec<1, MINB, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEnsBSmem);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ens_spec<2, MINB, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEnsBSmem);
+template <int MODE> cudaError_t ens_spec_attrs() {
+  cudaError_t e = ens_smem(k_ens_pair_rows<MODE>, kEnsPairSmem);
+  if (e == cudaSuccess) e = ens_smem(k_ens_spec<MODE, 6>, kEnsBSmem);
+  if (e == cudaSuccess) e = ens_smem(k_ens_spec<MODE, 4>, kEnsBSmem);
+  if (e == cudaSuccess) e = ens_smem(k_ens_spec<MODE, 4, true>, kEnsBSmem);
   return e;
 }
-const void* ens_phys_fn(int v) {
-  return v == 1 ? (const void*)k_ens_phys<3> : (const void*)k_ens_phys<2>;
+cudaError_t ens_attrs() {
+  cudaError_t e = ens_smem(k_ens_pair_cols, kEnsPairSmem);
+  if (e == cudaSuccess) e = ens_smem(k_ens_phys<2>, kEnsASmem);
+  if (e == cudaSuccess) e = ens_spec_attrs<-1>();
+  if (e == cudaSuccess) e = ens_spec_attrs<0>();
+  if (e == cudaSuccess) e = ens_spec_attrs<1>();
+  if (e == cudaSuccess) e = ens_spec_attrs<2>();
+  return e;
 }
+const void* ens_phys_fn(int v) { return v == 0 ? (const void*)k_ens_pair_cols : (const void*)k_ens_phys<2>; }
 const void* ens_spec_fn(int v) {
-  return v == 1 ? (const void*)k_ens_spec<1, 4> : v == 2 ? (const void*)k_ens_spec<1, 5>
-         : v == 3 ? (const void*)k_ens_spec<1, 4, true> : (const void*)k_ens_spec<1, 6>;
+  return v == 0 ? (const void*)k_ens_pair_rows<1> : v == 1 ? (const void*)k_ens_spec<1, 6>
+         : v == 2 ? (const void*)k_ens_spec<1, 4> : (const void*)k_ens_spec<1, 4, true>;
 }
-void ens_launch_phys(int v, int grid, cudaStream_t st, const EnsInst* inst, const int2* items, int nitems, Pools pool) {
-  if (v == 1) k_ens_phys<3><<<grid, kEnsAThreads, kEnsASmem, st>>>(inst, items, nitems, pool);
-  else k_ens_phys<2><<<grid, kEnsAThreads, kEnsASmem, st>>>(inst, items, nitems, pool);
+// one shape's work list and persistent grid
+struct EnsWork {
+  const int2* items;
+  int nitems, grid;
+};
+void ens_launch_phys(int v, const EnsWork& w, cudaStream_t st, const EnsInst* inst, Pools pool) {
+  if (v == 0) k_ens_pair_cols<<<w.grid, kEnsPairThreads, kEnsPairSmem, st>>>(inst, w.items, w.nitems, pool);
+  else k_ens_phys<2><<<w.grid, kEnsAThreads, kEnsASmem, st>>>(inst, w.items, w.nitems, pool);
 }
 template <int MODE>
-void ens_launch_spec_m(int v, int grid, cudaStream_t st, const EnsInst* inst, const int2* items, int nitems, Pools pool,
-                       int phase, int* err) {
-  if (v == 1) k_ens_spec<MODE, 4><<<grid, kEnsBThreads, kEnsBSmem, st>>>(inst, items, nitems, pool, phase, err);
-  else if (v == 2) k_ens_spec<MODE, 5><<<grid, kEnsBThreads, kEnsBSmem, st>>>(inst, items, nitems, pool, phase, err);
-  else if (v == 3)
-    k_ens_spec<MODE, 4, true><<<grid, kEnsBThreads, kEnsBSmem, st>>>(inst, items, nitems, pool, phase, err);
-  else k_ens_spec<MODE, 6><<<grid, kEnsBThreads, kEnsBSmem, st>>>(inst, items, nitems, pool, phase, err);
+void ens_launch_spec_m(int v, const EnsWork& w, cudaStream_t st, const EnsInst* inst, Pools pool, int phase,
+                       int full_pb, int* err) {
+  if (v == 0)
+    k_ens_pair_rows<MODE><<<w.grid, kEnsPairThreads, kEnsPairSmem, st>>>(inst, w.items, w.nitems, pool, phase, full_pb);
+  else if (v == 1) k_ens_spec<MODE, 6><<<w.grid, kEnsBThreads, kEnsBSmem, st>>>(inst, w.items, w.nitems, pool, phase, err);
+  else if (v == 2) k_ens_spec<MODE, 4><<<w.grid, kEnsBThreads, kEnsBSmem, st>>>(inst, w.items, w.nitems, pool, phase, err);
+  else k_ens_spec<MODE, 4, true><<<w.grid, kEnsBThreads, kEnsBSmem, st>>>(inst, w.items, w.nitems, pool, phase, err);
 }
-void ens_launch_spec(int mode, int v, int grid, cudaStream_t st, const EnsInst* inst, const int2* items, int nitems,
-                     Pools pool, int phase, int* err) {
-  if (mode < 0) ens_launch_spec_m<-1>(v, grid, st, inst, items, nitems, pool, phase, err);
-  else if (mode == 0) ens_launch_spec_m<0>(v, grid, st, inst, items, nitems, pool, phase, err);
-  else if (mode == 1) ens_launch_spec_m<1>(v, grid, st, inst, items, nitems, pool, phase, err);
-  else ens_launch_spec_m<2>(v, grid, st, inst, items, nitems, pool, phase, err);
+void ens_launch_spec(int mode, int v, const EnsWork& w, cudaStream_t st, const EnsInst* inst, Pools pool, int phase,
+                     int full_pb, int* err) {
+  if (mode < 0) ens_launch_spec_m<-1>(v, w, st, inst, pool, phase, full_pb, err);
+  else if (mode == 0) ens_launch_spec_m<0>(v, w, st, inst, pool, phase, full_pb, err);
+  else if (mode == 1) ens_launch_spec_m<1>(v, w, st, inst, pool, phase, full_pb, err);
+  else ens_launch_spec_m<2>(v, w, st, inst, pool, phase, full_pb, err);
 }
 
 __global__ void k_ens_twiddles(float2* tw, int n) {
@@ -257,9 +344,26 @@ __global__ void k_ens_energy(const EnsInst* __restrict__ inst, const float2* __r
 
 bool ens_n_ok(int n) { return n == 64 || n == 128 || n == 256 || n == 512 || n == 1024; }
 
-template <int N> void tiles_of(int& a, int& b) {
-  a = Tune<N>::A_GRID;
-  b = Tune<N>::B_GRID;
+// tiles of the any-state kernels and of the pair kernels
+struct EnsTiles {
+  int a, b, pa, pb;
+};
+template <int N> EnsTiles tiles_of() {
+  return {Tune<N>::A_GRID, Tune<N>::B_GRID, EnsPair<N>::A_GRID, EnsPair<N>::B_GRID};
+}
+EnsTiles tiles_of(int n) {
+  return n == 64 ? tiles_of<64>() : n == 128 ? tiles_of<128>() : n == 256 ? tiles_of<256>()
+         : n == 512 ? tiles_of<512>() : tiles_of<1024>();
+}
+template <int N> cudaError_t ens_make_ptw(float4* out, const float2* tw, cudaStream_t st) {
+  constexpr int size = PassTw<N, EnsPair<N>::V>::SIZE;
+  k_pass_twiddles<N, EnsPair<N>::V><<<(size + 255) / 256, 256, 0, st>>>(out, tw);
+  return cudaGetLastError();
+}
+cudaError_t ens_make_ptw(int n, float4* out, const float2* tw, cudaStream_t st) {
+  return n == 64 ? ens_make_ptw<64>(out, tw, st) : n == 128 ? ens_make_ptw<128>(out, tw, st)
+         : n == 256 ? ens_make_ptw<256>(out, tw, st) : n == 512 ? ens_make_ptw<512>(out, tw, st)
+                                                               : ens_make_ptw<1024>(out, tw, st);
 }
 
 }  // namespace
@@ -271,12 +375,15 @@ struct s2d_ensemble {
   std::vector<uint32_t> seeds;
   EnsInst* dinst = nullptr;
   uint32_t* dseeds = nullptr;
-  int2 *items_a = nullptr, *items_b = nullptr;
-  int nitems_a = 0, nitems_b = 0;
-  int grid_a[kEnsNPhys] = {}, grid_b[kEnsNSpec] = {};   // persistent grids per launch shape
-  int pv = 0, sv = 0;                                   // launch shapes in use
+  int2* items = nullptr;                                // the four work lists, one after another
+  EnsWork work_a[kEnsNPhys] = {}, work_b[kEnsNSpec] = {};   // per launch shape
+  int pv = 0, sv = 0;                                   // launch shapes chosen
+  // every state is zero outside its dealias band (seeds, steps); a caller may store others,
+  // which the pair kernels do not take
+  bool banded = true;
   Pools pool{};
   float2* tw = nullptr;
+  float4* ptw = nullptr;
   double* sums = nullptr;    // 2 * count
   int* err = nullptr;        // device error word (bounded waits that gave up)
   long long cells = 0;
@@ -285,12 +392,27 @@ struct s2d_ensemble {
   std::map<int, std::pair<cudaGraph_t, cudaGraphExec_t>> graphs;   // by starting phase
 };
 
-static void ens_free(s2d_ensemble* e) {
+// the shapes of the next launches: pair kernels only on dealiased states, and pair columns
+// only after pair rows (which leave PB's rows ky < 0 unwritten for them)
+static int ens_sv(const s2d_ensemble* e) { return e->sv == 0 && !e->banded ? kEnsAnyState : e->sv; }
+static int ens_pv(const s2d_ensemble* e) { return e->pv == 0 && ens_sv(e) != 0 ? kEnsAnyState : e->pv; }
+static int ens_full_pb(const s2d_ensemble* e) { return ens_pv(e) != 0; }
+static void ens_drop_graphs(s2d_ensemble* e) {
   for (auto& kv : e->graphs) {
     if (kv.second.second) cudaGraphExecDestroy(kv.second.second);
     if (kv.second.first) cudaGraphDestroy(kv.second.first);
   }
-  void* ptrs[] = {e->dinst, e->dseeds, e->items_a, e->items_b, e->pool.s[0], e->pool.s[1], e->pool.s[2],
+  e->graphs.clear();
+}
+// captured steps hold the kernels of the previous kind of state
+static void ens_set_banded(s2d_ensemble* e, bool banded) {
+  if (banded != e->banded) ens_drop_graphs(e);
+  e->banded = banded;
+}
+
+static void ens_free(s2d_ensemble* e) {
+  ens_drop_graphs(e);
+  void* ptrs[] = {e->dinst, e->dseeds, e->items, e->ptw, e->pool.s[0], e->pool.s[1], e->pool.s[2],
                   e->pool.pa, e->pool.pb, e->pool.z, e->pool.row_nz, e->tw, e->sums, e->err};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -343,6 +465,10 @@ extern "C" int s2d_ensemble_create(const s2d_instance_desc* descs, int count, in
     k_ens_twiddles<<<(kv.first + 255) / 256, 256, 0, e->stream>>>(e->tw + kv.second, kv.first);
     TRY(cudaGetLastError(), "twiddle kernel");
   }
+  // SIZE of every pass-ordered table is below n
+  TRY(cudaMalloc(&e->ptw, sizeof(float4) * tw_len), "twiddles");
+  for (auto& kv : tw_off)
+    TRY(ens_make_ptw(kv.first, e->ptw + kv.second, e->tw + kv.second, e->stream), "twiddle kernel");
   // instances and work lists (largest grids first for balance)
   e->hinst.resize(count);
   e->seeds.resize(count);
@@ -366,16 +492,10 @@ extern "C" int s2d_ensemble_create(const s2d_instance_desc* descs, int count, in
     I.p.force_norm = (float)(0.01 * n * n);
     I.p.n = n;
     I.dt = d.dt;
-    switch (n) {
-      case 64: tiles_of<64>(I.tiles_a, I.tiles_b); break;
-      case 128: tiles_of<128>(I.tiles_a, I.tiles_b); break;
-      case 256: tiles_of<256>(I.tiles_a, I.tiles_b); break;
-      case 512: tiles_of<512>(I.tiles_a, I.tiles_b); break;
-      default: tiles_of<1024>(I.tiles_a, I.tiles_b); break;
-    }
     I.off = off;
     I.roff = roff;
     I.tw = e->tw + tw_off[n];
+    I.ptw = e->ptw + tw_off[n];
     off += (long long)n * n;
     roff += n;
     e->seeds[i] = d.seed;
@@ -384,17 +504,18 @@ extern "C" int s2d_ensemble_create(const s2d_instance_desc* descs, int count, in
   std::vector<int> order(count);
   for (int i = 0; i < count; ++i) order[i] = i;
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return e->hinst[a].n > e->hinst[b].n; });
-  std::vector<int2> ia, ib;
+  // work lists: any-state columns, rows; pair columns, rows
+  std::vector<int2> lists[4], all;
   for (int i : order) {
-    for (int t = 0; t < e->hinst[i].tiles_a; ++t) ia.push_back(make_int2(i, t));
-    for (int t = 0; t < e->hinst[i].tiles_b; ++t) ib.push_back(make_int2(i, t));
+    const EnsTiles t = tiles_of(e->hinst[i].n);
+    const int tiles[4] = {t.a, t.b, t.pa, t.pb};
+    for (int l = 0; l < 4; ++l)
+      for (int k = 0; k < tiles[l]; ++k) lists[l].push_back(make_int2(i, k));
   }
-  e->nitems_a = (int)ia.size();
-  e->nitems_b = (int)ib.size();
+  for (const auto& l : lists) all.insert(all.end(), l.begin(), l.end());
   TRY(cudaMalloc(&e->dinst, sizeof(EnsInst) * count), "instances");
   TRY(cudaMalloc(&e->dseeds, sizeof(uint32_t) * count), "seeds");
-  TRY(cudaMalloc(&e->items_a, sizeof(int2) * ia.size()), "items");
-  TRY(cudaMalloc(&e->items_b, sizeof(int2) * ib.size()), "items");
+  TRY(cudaMalloc(&e->items, sizeof(int2) * all.size()), "items");
   TRY(cudaMalloc(&e->sums, sizeof(double) * 2 * count), "sums");
   TRY(cudaMalloc(&e->err, sizeof(int)), "error word");
   TRY(cudaMemsetAsync(e->err, 0, sizeof(int), e->stream), "memset");
@@ -409,24 +530,24 @@ extern "C" int s2d_ensemble_create(const s2d_instance_desc* descs, int count, in
   TRY(cudaMemsetAsync(e->pool.z, 0, cbytes, e->stream), "memset");
   TRY(cudaMemcpyAsync(e->dinst, e->hinst.data(), sizeof(EnsInst) * count, cudaMemcpyHostToDevice, e->stream), "copy");
   TRY(cudaMemcpyAsync(e->dseeds, e->seeds.data(), sizeof(uint32_t) * count, cudaMemcpyHostToDevice, e->stream), "copy");
-  TRY(cudaMemcpyAsync(e->items_a, ia.data(), sizeof(int2) * ia.size(), cudaMemcpyHostToDevice, e->stream), "copy");
-  TRY(cudaMemcpyAsync(e->items_b, ib.data(), sizeof(int2) * ib.size(), cudaMemcpyHostToDevice, e->stream), "copy");
-  TRY(ens_phys_attrs<2>(), "attr");
-  TRY(ens_phys_attrs<3>(), "attr");
-  TRY(ens_spec_attrs<4>(), "attr");
-  TRY(ens_spec_attrs<5>(), "attr");
-  TRY(ens_spec_attrs<6>(), "attr");
-  TRY((ens_spec_attrs<4, true>()), "attr");
-  for (int v = 0; v < kEnsNPhys; ++v) {
+  TRY(cudaMemcpyAsync(e->items, all.data(), sizeof(int2) * all.size(), cudaMemcpyHostToDevice, e->stream), "copy");
+  TRY(ens_attrs(), "attr");
+  const int2* list_at[4] = {e->items, nullptr, nullptr, nullptr};
+  for (int l = 1; l < 4; ++l) list_at[l] = list_at[l - 1] + lists[l - 1].size();
+  auto work = [&](const void* fn, int threads, size_t smem, int l, EnsWork* w) {
     int occ = 0;
-    TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ens_phys_fn(v), kEnsAThreads, kEnsASmem), "occupancy");
-    e->grid_a[v] = std::min(e->nitems_a, std::max(1, occ) * prop.multiProcessorCount);
-  }
-  for (int v = 0; v < kEnsNSpec; ++v) {
-    int occ = 0;
-    TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ens_spec_fn(v), kEnsBThreads, kEnsBSmem), "occupancy");
-    e->grid_b[v] = std::min(e->nitems_b, std::max(1, occ) * prop.multiProcessorCount);
-  }
+    const cudaError_t r = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, threads, smem);
+    w->items = list_at[l];
+    w->nitems = (int)lists[l].size();
+    w->grid = std::min(w->nitems, std::max(1, occ) * prop.multiProcessorCount);
+    return r;
+  };
+  for (int v = 0; v < kEnsNPhys; ++v)
+    TRY(v == 0 ? work(ens_phys_fn(v), kEnsPairThreads, kEnsPairSmem, 2, &e->work_a[v])
+               : work(ens_phys_fn(v), kEnsAThreads, kEnsASmem, 0, &e->work_a[v]), "occupancy");
+  for (int v = 0; v < kEnsNSpec; ++v)
+    TRY(v == 0 ? work(ens_spec_fn(v), kEnsPairThreads, kEnsPairSmem, 3, &e->work_b[v])
+               : work(ens_spec_fn(v), kEnsBThreads, kEnsBSmem, 1, &e->work_b[v]), "occupancy");
   TRY(cudaStreamSynchronize(e->stream), "sync");
 #undef TRY
   cudaSetDevice(prev);
@@ -483,6 +604,7 @@ extern "C" int s2d_ensemble_seed_band(s2d_ensemble* e, float kmin, float kmax, f
   E_CUDA(cudaMemsetAsync(e->pool.s[2], 0, cbytes, e->stream));
   e->phase = 0;
   e->packs_valid = false;
+  ens_set_banded(e, true);
   return S2D_OK;
 }
 
@@ -496,6 +618,7 @@ extern "C" int s2d_ensemble_set_state(s2d_ensemble* e, int index, const float* s
   E_CUDA(cudaMemcpyAsync(e->pool.s[e->phase] + I.off, spectrum, bytes, cudaMemcpyHostToDevice, e->stream));
   E_CUDA(cudaStreamSynchronize(e->stream));
   e->packs_valid = false;
+  if (!band_limited(spectrum, bytes / sizeof(float), I.n)) ens_set_banded(e, false);
   return S2D_OK;
 }
 
@@ -510,11 +633,11 @@ extern "C" int s2d_ensemble_get_state(s2d_ensemble* e, int index, float* spectru
 }
 
 static int ens_enqueue_step(s2d_ensemble* e) {
-  const int p = e->phase;
+  const int p = e->phase, pv = ens_pv(e), sv = ens_sv(e);
   for (int st = 0; st < 3; ++st) {
-    ens_launch_phys(e->pv, e->grid_a[e->pv], e->stream, e->dinst, e->items_a, e->nitems_a, e->pool);
+    ens_launch_phys(pv, e->work_a[pv], e->stream, e->dinst, e->pool);
     E_LAUNCHED();
-    ens_launch_spec(st, e->sv, e->grid_b[e->sv], e->stream, e->dinst, e->items_b, e->nitems_b, e->pool, p, e->err);
+    ens_launch_spec(st, sv, e->work_b[sv], e->stream, e->dinst, e->pool, p, ens_full_pb(e), e->err);
     E_LAUNCHED();
   }
   e->phase = (p + 1) % 3;
@@ -529,8 +652,9 @@ extern "C" int s2d_ensemble_step(s2d_ensemble* e, int steps, int use_graph) {
   if (prev != e->dev) cudaSetDevice(e->dev);
   int rc = S2D_OK;
   if (!e->packs_valid) {
-    ens_launch_spec(-1, e->sv, e->grid_b[e->sv], e->stream, e->dinst, e->items_b, e->nitems_b, e->pool, e->phase,
-                    e->err);
+    const int sv = ens_sv(e);
+    if (sv == 0) k_ens_band_flags<<<e->count, 128, 0, e->stream>>>(e->dinst, e->pool.row_nz);
+    ens_launch_spec(-1, sv, e->work_b[sv], e->stream, e->dinst, e->pool, e->phase, ens_full_pb(e), e->err);
     if (cudaGetLastError() != cudaSuccess) rc = efail(S2D_ERR_CUDA, "prime launch failed");
     e->packs_valid = true;
   }
@@ -577,7 +701,7 @@ extern "C" int s2d_ensemble_tune_variant_name(s2d_ensemble* e, int kind, int ind
   const int count = kind == 0 ? kEnsNPhys : kind == 1 ? kEnsNSpec : -1;
   if (count < 0 || index < 0 || index >= count) return efail(S2D_ERR_ARG, "variant out of range");
   std::snprintf(out, (size_t)cap, "%d CTAs/SM%s", kind == 0 ? kEnsPhysMinb[index] : kEnsSpecMinb[index],
-                kind == 1 && kEnsSpecPair[index] ? ", paired inverse transforms" : "");
+                kind == 0 ? kEnsPhysNote[index] : kEnsSpecNote[index]);
   return S2D_OK;
 }
 
@@ -643,11 +767,7 @@ extern "C" int s2d_ensemble_autotune(s2d_ensemble* e, int steps, s2d_tune_report
   if (saved) cudaFree(saved);
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);
-  for (auto& kv : e->graphs) {          // captured with the previous shapes
-    if (kv.second.second) cudaGraphExecDestroy(kv.second.second);
-    if (kv.second.first) cudaGraphDestroy(kv.second.first);
-  }
-  e->graphs.clear();
+  ens_drop_graphs(e);   // captured with the previous shapes
   if (prev != e->dev) cudaSetDevice(prev);
   if (rc) return rc;
   rep.phys_choice = e->pv;
@@ -662,11 +782,8 @@ extern "C" int s2d_ensemble_tune_select(s2d_ensemble* e, int phys, int spec) {
     return efail(S2D_ERR_ARG, "ensemble shape index out of range");
   e->pv = phys;
   e->sv = spec;
-  for (auto& kv : e->graphs) {          // captured with the previous shapes
-    if (kv.second.second) cudaGraphExecDestroy(kv.second.second);
-    if (kv.second.first) cudaGraphDestroy(kv.second.first);
-  }
-  e->graphs.clear();
+  e->packs_valid = false;   // laid out for the previous shapes
+  ens_drop_graphs(e);   // captured with the previous shapes
   return S2D_OK;
 }
 

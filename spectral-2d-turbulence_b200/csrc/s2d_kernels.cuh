@@ -89,6 +89,7 @@ struct PhysArgs {
   DevParams* latch;     // non-null: latch step_index from *counter (and advance it) first
   uint32_t* counter;
   const int* row_nz;    // non-null: row ky of PA/PB is all zero (and need not be read) where 0
+  const float4* ptw;    // pass-ordered twiddles of the pair kernels (s2d_pairs.cuh)
 };
 
 // the per-substep stepIndex latch (S2D_STEP_RELATCH): params.step_index = counter++,
@@ -118,6 +119,8 @@ struct SpecArgs {
   int* err;             // device error word (bounded waits that gave up)
   int* row_nz;          // non-null: per row, 1 if the written PA/PB row holds a nonzero value;
                         // a CTA whose rows are all zero then skips its transforms and stores
+  const float4* ptw;    // pass-ordered twiddles of the pair kernels (s2d_pairs.cuh)
+  int full_pb;          // pair kernel: also write the rows ky < 0 of PB (readers other than k_pair_cols)
 };
 
 // rows held by the 2*PPB row slots of tile `tile`: pair p = rows (p, N-p); pair 0 = rows (0, N/2)

@@ -7,6 +7,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include "s2d_kernels.cuh"
+#include "s2d_pairs.cuh"
 
 namespace s2d {
 
@@ -15,17 +16,23 @@ template <class K> inline cudaError_t set_smem(K kernel, size_t bytes) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
+// `pairs`: a shape of the pair kernels, for dealiased states only (s2d_pairs.cuh)
 struct PhysVariant {
   const char* name;
   cudaError_t (*set_attrs)();
   void (*run)(int mode, const PhysArgs& a, cudaStream_t st);
+  bool pairs = false;
 };
 struct SpecVariant {
   const char* name;
   cudaError_t (*set_attrs)();
   void (*run)(int mode, bool ptr, const SpecArgs& a, cudaStream_t st);
+  bool pairs = false;
 };
-constexpr int kMaxVariants = 4;
+constexpr int kMaxVariants = 6;
+// variant 0 of each stage is the pair kernel, variant 1 the first of the kernels that take
+// any state
+constexpr int kAnyState = 1;
 
 struct NOps {
   int n;
@@ -35,6 +42,9 @@ struct NOps {
   cudaError_t (*set_attrs)();   // FFT passes and every registered stage variant
   void (*fft_rows)(int sign, float2* data, const float2* tw, cudaStream_t st);
   void (*fft_cols)(int sign, float2* data, const float2* tw, cudaStream_t st);
+  // pass-ordered twiddles of the pair kernels
+  int ptw_size;
+  void (*make_ptw)(float4* out, const float2* tw, cudaStream_t st);
   int n_phys = 0, n_spec = 0;
   PhysVariant phys[kMaxVariants];
   SpecVariant spec[kMaxVariants];
@@ -90,9 +100,51 @@ template <int N, class TU> struct SpecImpl {
   static SpecVariant make(const char* name) { return SpecVariant{name, &set_attrs, &run}; }
 };
 
+// ---------------------------------------------------------------- pair-kernel variants
+template <class TU> struct PairImpl {
+  static cudaError_t phys_attrs() {
+    cudaError_t e = set_smem(k_pair_cols<0, TU>, TU::A_SMEM);
+    if (e == cudaSuccess) e = set_smem(k_pair_cols<1, TU>, TU::A_SMEM);
+    if (e == cudaSuccess) e = set_smem(k_pair_cols<2, TU>, TU::A_SMEM);
+    return e;
+  }
+  static void phys_run(int mode, const PhysArgs& a, cudaStream_t st) {
+    const dim3 g(TU::A_GRID), b(TU::A_THREADS);
+    if (mode == 0) k_pair_cols<0, TU><<<g, b, TU::A_SMEM, st>>>(a);
+    else if (mode == 1) k_pair_cols<1, TU><<<g, b, TU::A_SMEM, st>>>(a);
+    else k_pair_cols<2, TU><<<g, b, TU::A_SMEM, st>>>(a);
+  }
+  template <int MODE, bool PTR> static cudaError_t attr() { return set_smem(k_pair_rows<MODE, PTR, TU>, TU::B_SMEM); }
+  static cudaError_t spec_attrs() {
+    cudaError_t e = cudaSuccess;
+    for (cudaError_t r : {attr<-1, false>(), attr<0, false>(), attr<1, false>(), attr<2, false>(), attr<0, true>(),
+                          attr<1, true>(), attr<2, true>()})
+      if (r != cudaSuccess && e == cudaSuccess) e = r;
+    return e;
+  }
+  template <int MODE, bool PTR> static void launch(const SpecArgs& a, cudaStream_t st) {
+    k_pair_rows<MODE, PTR, TU><<<dim3(TU::B_GRID), dim3(TU::B_THREADS), TU::B_SMEM, st>>>(a);
+  }
+  static void spec_run(int mode, bool ptr, const SpecArgs& a, cudaStream_t st) {
+    switch (mode) {
+      case -1: launch<-1, false>(a, st); break;
+      case 0: ptr ? launch<0, true>(a, st) : launch<0, false>(a, st); break;
+      case 1: ptr ? launch<1, true>(a, st) : launch<1, false>(a, st); break;
+      default: ptr ? launch<2, true>(a, st) : launch<2, false>(a, st); break;
+    }
+  }
+  static PhysVariant phys() { return PhysVariant{"column pairs", &phys_attrs, &phys_run, true}; }
+  static SpecVariant spec() { return SpecVariant{"row pairs", &spec_attrs, &spec_run, true}; }
+};
+
 // ---------------------------------------------------------------- per-size table
 template <int N> struct OpsImpl {
   using TU = Tune<N>;
+  using PT = PairShape<N>;
+  static void make_ptw(float4* out, const float2* tw, cudaStream_t st) {
+    constexpr int size = PassTw<N, PT::V>::SIZE;
+    k_pass_twiddles<N, PT::V><<<(size + 255) / 256, 256, 0, st>>>(out, tw);
+  }
   static cudaError_t fft_attrs() {
     cudaError_t e = cudaSuccess;
     auto chk = [&](cudaError_t r) { if (r != cudaSuccess && e == cudaSuccess) e = r; };
@@ -128,6 +180,10 @@ template <int N> struct OpsImpl {
     o.set_attrs = &fft_attrs;
     o.fft_rows = &fft_rows;
     o.fft_cols = &fft_cols;
+    o.ptw_size = PassTw<N, PT::V>::SIZE;
+    o.make_ptw = &make_ptw;
+    o.phys[o.n_phys++] = PairImpl<PT>::phys();
+    o.spec[o.n_spec++] = PairImpl<PT>::spec();
     o.phys[o.n_phys++] = PhysImpl<N, TU>::make("V=16");
     o.spec[o.n_spec++] = SpecImpl<N, TU>::make("V=16");
     for (const PhysVariant& v : extra_phys)

@@ -171,7 +171,7 @@ struct s2d_solver {
          *vel = nullptr, *tw = nullptr;
   float* dtbuf = nullptr;      // 2 slots x [dt, speed], at the end of diag's allocation
   float* partials = nullptr;
-  unsigned* ticket = nullptr;
+  unsigned* ticket = nullptr;   // CTA counter, then max |u|+|v| (bits) of the pair column kernel
   DevParams* dparams = nullptr;
   DevSplats* dsplats = nullptr;   // inside dparams' allocation, right after the parameters
   // the two diagnostics blocks and the dt slots in one allocation (diag_block_offset)
@@ -479,10 +479,9 @@ static const char* dye_axis_check(int n, int m, int t0, int T, int W1, int W2, i
   return nullptr;
 }
 
-template <int TX> static int dye_fast_path_check_tx(int n, int m) {
-  using G = DyeGeom<TX>;
-  for (int t0 = 0; t0 < m; t0 += TX)
-    if (const char* why = dye_axis_check(n, m, t0, TX, G::W1X, G::W2X, G::W3X, 3 * kDyeLo + 1, G::vel_x(n, m)))
+template <class G> static int dye_fast_path_check_geom(int n, int m) {
+  for (int t0 = 0; t0 < m; t0 += G::TX)
+    if (const char* why = dye_axis_check(n, m, t0, G::TX, G::W1X, G::W2X, G::W3X, 3 * kDyeLo + 1, G::vel_x(n, m)))
       return fail(S2D_ERR_ARG, std::string("x tile at ") + std::to_string(t0) + ": " + why);
   for (int t0 = 0; t0 < m; t0 += G::TY)
     if (const char* why = dye_axis_check(n, m, t0, G::TY, G::W1Y, G::W2Y, G::W3Y, 3 * kDyeLo, G::vel_y(n, m)))
@@ -494,7 +493,11 @@ extern "C" int s2d_dye_fast_path_check(int n, int dye_scale) {
   if (n < S2D_MIN_N || n > S2D_MAX_N || (n & (n - 1)) != 0) return fail(S2D_ERR_UNSUPPORTED_N, "n");
   if (dye_scale != 1 && dye_scale != 2 && dye_scale != 4) return fail(S2D_ERR_ARG, "dye_scale must be 1, 2 or 4");
   const int m = n * dye_scale;
-  return dye_wide_tile(n, m) ? dye_fast_path_check_tx<64>(n, m) : dye_fast_path_check_tx<32>(n, m);
+  switch (dye_tile(n, m)) {
+    case 0: return dye_fast_path_check_geom<DyeWide>(n, m);
+    case 1: return dye_fast_path_check_geom<DyeSquare>(n, m);
+    default: return dye_fast_path_check_geom<DyeSmall>(n, m);
+  }
 }
 
 static int table_prelude(int n) {
@@ -596,6 +599,7 @@ template <class P> static void tc_rows_launch(int mode, bool ptr, const SpecArgs
     else tc::k_spec_rows_tc2<2, true, P><<<g, b, sm, st>>>(a, tab);
   }
 }
+static float* dt_slot(s2d_solver* s, int slot) { return s->dtbuf + 2 * slot; }
 static bool is_tc(const s2d_solver* s) { return s->fft_precision != S2D_FFT_FP32; }
 // The stage kernels of the next launch: the chosen shapes, except that the pair kernels need a
 // dealiased state, and the pair column kernel also rows written by the pair row kernel (it
@@ -617,7 +621,9 @@ static void mark_packs(s2d_solver* s) {
 }
 // the row stage with the solver's chosen variant
 static void run_spec(s2d_solver* s, int mode, bool ptr, SpecArgs a) {
-  a.ptw = s->ptw;
+  a.ptw = s->ptw + s->ops->ptw_rows;
+  a.top = pair_cols(s) ? s->ticket + 1 : nullptr;
+  a.dt_out = dt_slot(s, s->slot ^ 1);
   a.full_pb = pair_cols(s) ? 0 : 1;
   if (tc_rows(s)) {
     if (s->fft_precision == S2D_FFT_TC_BF16) tc_rows_launch<tc::PrecBF16>(mode, ptr, a, s->tctab, s->stream);
@@ -684,7 +690,7 @@ extern "C" int s2d_create(int n, int dye_scale, int fft_precision, int device, s
   // column-kernel grids are at most n CTAs in every registered shape
   const int nparts = std::max(std::max(n, 256), seed_parts_count(n));
   TRY(cudaMalloc(&s->partials, sizeof(float) * nparts), "partials");
-  TRY(cudaMalloc(&s->ticket, sizeof(unsigned)), "ticket");
+  TRY(cudaMalloc(&s->ticket, 2 * sizeof(unsigned)), "ticket");
   TRY(cudaMalloc(&s->row_nz, sizeof(int) * n), "row flags");
   TRY(cudaMalloc(&s->dparams, kConstBytes), "params");
   s->dsplats = reinterpret_cast<DevSplats*>(reinterpret_cast<char*>(s->dparams) + sizeof(DevParams));
@@ -704,11 +710,11 @@ extern "C" int s2d_create(int n, int dye_scale, int fft_precision, int device, s
   TRY(cudaMallocHost(&s->h_upload, kUploadSlotBytes * kUploadSlots), "pinned upload ring");
   for (cudaEvent_t& ev : s->upload_ev) TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "event");
   TRY(set_all_attrs(*ops), "kernel attributes");
-  if (dye_wide_tile(n, s->m))
-    TRY(cudaFuncSetAttribute(k_dye_fused<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)DyeGeom<64>::smem(n, s->m)), "dye kernel attributes");
-  TRY(cudaFuncSetAttribute(k_dye_fused<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)DyeGeom<32>::smem(n, s->m)), "dye kernel attributes");
+  switch (dye_tile(n, s->m)) {
+    case 0: TRY(set_smem(k_dye_fused<DyeWide>, DyeWide::smem(n, s->m)), "dye kernel attributes"); break;
+    case 1: TRY(set_smem(k_dye_fused<DyeSquare>, DyeSquare::smem(n, s->m)), "dye kernel attributes"); break;
+    default: TRY(set_smem(k_dye_fused<DyeSmall>, DyeSmall::smem(n, s->m)), "dye kernel attributes"); break;
+  }
   if (fft_precision == S2D_FFT_TC_F16 && n == 1024) TRY(tc_attrs<tc::PrecF16>(), "tensor-core kernel attributes");
   if (fft_precision == S2D_FFT_TC_BF16 && n == 1024) TRY(tc_attrs<tc::PrecBF16>(), "tensor-core kernel attributes");
   if (fft_precision != S2D_FFT_FP32 && n != 1024)
@@ -722,7 +728,7 @@ extern "C" int s2d_create(int n, int dye_scale, int fft_precision, int device, s
   TRY(cudaMemsetAsync(s->force, 0, cbytes, s->stream), "memset");
   TRY(cudaMemsetAsync(s->vel, 0, cbytes, s->stream), "memset");
   TRY(cudaMemsetAsync(s->dtbuf, 0, sizeof(float) * 4, s->stream), "memset");
-  TRY(cudaMemsetAsync(s->ticket, 0, sizeof(unsigned), s->stream), "memset");
+  TRY(cudaMemsetAsync(s->ticket, 0, 2 * sizeof(unsigned), s->stream), "memset");
   TRY(cudaMemsetAsync(s->partials, 0, sizeof(float) * nparts, s->stream), "memset");
   for (int i = 0; i < 3; ++i) TRY(cudaMemsetAsync(s->dye[i], 0, dbytes, s->stream), "memset");
   k_twiddles<<<(n + 255) / 256, 256, 0, s->stream>>>(s->tw, n);
@@ -922,8 +928,6 @@ static int enqueue_fft2(s2d_solver* s, float2* buf, int sign) {
   return S2D_OK;
 }
 
-static float* dt_slot(s2d_solver* s, int slot) { return s->dtbuf + 2 * slot; }
-
 // prime packs from state[phase]: PA/PB = FFT_x^-1 of the scaled packs
 static int enqueue_pack_prime(s2d_solver* s) {
   SpecArgs a{};
@@ -950,6 +954,17 @@ static int enqueue_pack_prime(s2d_solver* s) {
 // other than the fused stage kernels reads or writes the packs
 static int materialize_packs(s2d_solver* s) {
   if (!s->packs_flagged) return S2D_OK;
+  if (s->packs_half && s->ops->blocked_packs) {
+    const size_t cbytes = (size_t)s->n * s->n * sizeof(float2);
+    float2* tmp = nullptr;
+    S2D_CUDA(cudaMallocAsync(&tmp, cbytes, s->stream));
+    for (float2* p : {s->packA, s->packB}) {
+      S2D_CUDA(cudaMemcpyAsync(tmp, p, cbytes, cudaMemcpyDeviceToDevice, s->stream));
+      k_unblock_pack<<<cells_grid(s->n), 256, 0, s->stream>>>(p, tmp, s->n);
+      S2D_LAUNCHED();
+    }
+    S2D_CUDA(cudaFreeAsync(tmp, s->stream));
+  }
   if (s->packs_pairs)
     k_expand_packs<<<cells_grid(s->n), 256, 0, s->stream>>>(s->packA, s->packB, s->n, s->packs_half ? 1 : 0);
   else
@@ -1114,6 +1129,12 @@ extern "C" int s2d_encode_step(s2d_solver* s) {
 
 static uint2* tex(s2d_solver* s, int i) { return reinterpret_cast<uint2*>(s->dye[i]); }
 
+template <class G> static void launch_dye(s2d_solver* s) {
+  const int p = s->dye_parity, m = s->m;
+  k_dye_fused<G><<<dim3(m / G::TX, m / G::TY), G::THREADS, G::smem(s->n, m), s->stream>>>(
+      s->vel, tex(s, p), tex(s, 1 - p), dt_slot(s, s->slot), s->dparams, s->dsplats, s->n, m);
+}
+
 // encodeDye (solver.js:523-536) as one fused launch: forward, backward and
 // corrected passes of a tile computed from on-chip halos (s2d_dye.cuh)
 extern "C" int s2d_encode_dye(s2d_solver* s) {
@@ -1121,14 +1142,10 @@ extern "C" int s2d_encode_dye(s2d_solver* s) {
   DeviceGuard guard(s->dev);
   const int p = s->dye_parity, m = s->m;
   ProfScope ps(s, S2D_PROF_DYE);
-  if (dye_wide_tile(s->n, m)) {
-    using G = DyeGeom<64>;
-    k_dye_fused<64><<<dim3(m / 64, m / G::TY), G::THREADS, G::smem(s->n, m), s->stream>>>(
-        s->vel, tex(s, p), tex(s, 1 - p), dt_slot(s, s->slot), s->dparams, s->dsplats, s->n, m);
-  } else {
-    using G = DyeGeom<32>;
-    k_dye_fused<32><<<dim3(m / 32, m / G::TY), G::THREADS, G::smem(s->n, m), s->stream>>>(
-        s->vel, tex(s, p), tex(s, 1 - p), dt_slot(s, s->slot), s->dparams, s->dsplats, s->n, m);
+  switch (dye_tile(s->n, m)) {
+    case 0: launch_dye<DyeWide>(s); break;
+    case 1: launch_dye<DyeSquare>(s); break;
+    default: launch_dye<DyeSmall>(s); break;
   }
   S2D_LAUNCHED();
   s->dye_parity = 1 - p;

@@ -76,15 +76,16 @@ constexpr size_t kEnsBBarOff =
 constexpr size_t kEnsBSmem = kEnsBBarOff + 16;
 
 // Pair kernels (dealiased states): 128 threads at every size, so 128 / T row pairs or column
-// pairs per item -- a 128-thread CTA synchronises at most four warps, and four of them share
-// an SM.
-constexpr int kEnsPairThreads = 128, kEnsPairMinb = 4;
-template <int N>
-using EnsPair = PairTune<N, 8, kEnsPairThreads / (N / 8), kEnsPairThreads, kEnsPairMinb, kEnsPairMinb>;
+// pairs per item -- a 128-thread CTA synchronises at most four warps.  The row kernel runs three
+// CTAs per SM at 168 registers: at four and 128 it spills (256 x 256^2: 593 against 645 us per
+// step; two CTAs 678), and the column kernel four (three 628).
+constexpr int kEnsPairThreads = 128, kEnsColsMinb = 4, kEnsRowsMinb = 3;
+template <int N> using EnsCols = PairCols<N, 8, kEnsPairThreads / (N / 8), kEnsColsMinb>;
+template <int N> using EnsRows = PairRows<N, 8, kEnsPairThreads, kEnsRowsMinb>;
 // the same bytes at every size: (9/8) N elements of 24 bytes for each of 1024 / N pairs
-constexpr size_t kEnsPairSmem = EnsPair<1024>::B_SMEM;
-static_assert(EnsPair<64>::A_SMEM == kEnsPairSmem && EnsPair<64>::B_SMEM == kEnsPairSmem &&
-                  EnsPair<256>::A_SMEM == kEnsPairSmem && EnsPair<1024>::A_SMEM == kEnsPairSmem,
+constexpr size_t kEnsPairSmem = EnsRows<1024>::SMEM;
+static_assert(EnsCols<64>::SMEM == kEnsPairSmem && EnsRows<64>::SMEM == kEnsPairSmem &&
+                  EnsCols<256>::SMEM == kEnsPairSmem && EnsCols<1024>::SMEM == kEnsPairSmem,
               "one shared-memory size for every grid size");
 
 struct Pools {
@@ -95,54 +96,41 @@ struct Pools {
   int* row_nz;
 };
 
-__global__ void __launch_bounds__(kEnsPairThreads, kEnsPairMinb)
-    k_ens_pair_cols(const EnsInst* __restrict__ inst, const int2* __restrict__ items, int nitems, Pools pool) {
+// `a` holds the pooled arrays; an item adds its instance's offset, parameters and twiddles
+__global__ void __launch_bounds__(kEnsPairThreads, kEnsColsMinb)
+    k_ens_pair_cols(const EnsInst* __restrict__ inst, const int2* __restrict__ items, int nitems, PhysArgs a) {
   extern __shared__ __align__(16) float4 smem4[];
+  pdl_wait();
   for (int k = blockIdx.x; k < nitems; k += gridDim.x) {
     const int2 it = items[k];
     const EnsInst& I = inst[it.x];
-    PhysArgs a{};
-    a.pa = pool.pa + I.off;
-    a.pb = pool.pb + I.off;
-    a.z = pool.z + I.off;
-    a.ptw = I.ptw;
     switch (I.n) {
-      case 64: pair_cols_tile<1, EnsPair<64>>(a, it.y, smem4); break;
-      case 128: pair_cols_tile<1, EnsPair<128>>(a, it.y, smem4); break;
-      case 256: pair_cols_tile<1, EnsPair<256>>(a, it.y, smem4); break;
-      case 512: pair_cols_tile<1, EnsPair<512>>(a, it.y, smem4); break;
-      default: pair_cols_tile<1, EnsPair<1024>>(a, it.y, smem4); break;
+      case 64: pair_cols_tile<EnsCols<64>>(a, I.off, I.ptw, 1, it.y, smem4); break;
+      case 128: pair_cols_tile<EnsCols<128>>(a, I.off, I.ptw, 1, it.y, smem4); break;
+      case 256: pair_cols_tile<EnsCols<256>>(a, I.off, I.ptw, 1, it.y, smem4); break;
+      case 512: pair_cols_tile<EnsCols<512>>(a, I.off, I.ptw, 1, it.y, smem4); break;
+      default: pair_cols_tile<EnsCols<1024>>(a, I.off, I.ptw, 1, it.y, smem4); break;
     }
     __syncthreads();
   }
 }
-template <int MODE>
-__global__ void __launch_bounds__(kEnsPairThreads, kEnsPairMinb)
-    k_ens_pair_rows(const EnsInst* __restrict__ inst, const int2* __restrict__ items, int nitems, Pools pool, int phase,
-                    int full_pb) {
+template <int N>
+__device__ __forceinline__ void ens_pair_rows(const SpecArgs& a, const EnsInst& I, int stage, int tile, float4* smem4) {
+  pair_rows_tile<EnsRows<N>>(a, I.off, &I.p, I.dt, I.p.force_amp > 0.f, I.ptw, stage, tile, smem4);
+}
+__global__ void __launch_bounds__(kEnsPairThreads, kEnsRowsMinb)
+    k_ens_pair_rows(const EnsInst* __restrict__ inst, const int2* __restrict__ items, int nitems, SpecArgs a, int stage) {
   extern __shared__ __align__(16) float4 smem4[];
-  constexpr int st = MODE < 0 ? 0 : MODE;
+  pdl_wait();
   for (int k = blockIdx.x; k < nitems; k += gridDim.x) {
     const int2 it = items[k];
     const EnsInst& I = inst[it.x];
-    SpecArgs a{};
-    a.z = pool.z + I.off;
-    a.w0 = pool.s[phase] + I.off;
-    a.wcur = pool.s[(phase + st) % 3] + I.off;
-    a.wout = pool.s[(phase + (st == 1 ? 2 : 1)) % 3] + I.off;
-    a.pa = pool.pa + I.off;
-    a.pb = pool.pb + I.off;
-    a.dt = &I.dt;
-    a.params = &I.p;
-    a.ptw = I.ptw;
-    a.stochastic = I.p.force_amp > 0.f ? 1 : 0;
-    a.full_pb = full_pb;
     switch (I.n) {
-      case 64: pair_rows_tile<MODE, false, EnsPair<64>>(a, it.y, smem4); break;
-      case 128: pair_rows_tile<MODE, false, EnsPair<128>>(a, it.y, smem4); break;
-      case 256: pair_rows_tile<MODE, false, EnsPair<256>>(a, it.y, smem4); break;
-      case 512: pair_rows_tile<MODE, false, EnsPair<512>>(a, it.y, smem4); break;
-      default: pair_rows_tile<MODE, false, EnsPair<1024>>(a, it.y, smem4); break;
+      case 64: ens_pair_rows<64>(a, I, stage, it.y, smem4); break;
+      case 128: ens_pair_rows<128>(a, I, stage, it.y, smem4); break;
+      case 256: ens_pair_rows<256>(a, I, stage, it.y, smem4); break;
+      case 512: ens_pair_rows<512>(a, I, stage, it.y, smem4); break;
+      default: ens_pair_rows<1024>(a, I, stage, it.y, smem4); break;
     }
     __syncthreads();
   }
@@ -229,8 +217,8 @@ __global__ void __launch_bounds__(kEnsBThreads, MINB)
 // ---- launch shapes of the two stage kernels: 0 (default) = pair kernels, for dealiased
 // states; the others take any state
 constexpr int kEnsAnyState = 1;
-constexpr int kEnsPhysMinb[] = {kEnsPairMinb, 2};      // resident CTAs per SM of each shape
-constexpr int kEnsSpecMinb[] = {kEnsPairMinb, 6, 4, 4};
+constexpr int kEnsPhysMinb[] = {kEnsColsMinb, 2};      // resident CTAs per SM of each shape
+constexpr int kEnsSpecMinb[] = {kEnsRowsMinb, 6, 4, 4};
 constexpr const char* kEnsPhysNote[] = {", column pairs", ""};
 constexpr const char* kEnsSpecNote[] = {", row pairs", "", "", ", paired inverse transforms"};
 constexpr int kEnsNPhys = 2, kEnsNSpec = 4;
@@ -239,14 +227,14 @@ template <class K> cudaError_t ens_smem(K k, size_t bytes) {
   return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 template <int MODE> cudaError_t ens_spec_attrs() {
-  cudaError_t e = ens_smem(k_ens_pair_rows<MODE>, kEnsPairSmem);
-  if (e == cudaSuccess) e = ens_smem(k_ens_spec<MODE, 6>, kEnsBSmem);
+  cudaError_t e = ens_smem(k_ens_spec<MODE, 6>, kEnsBSmem);
   if (e == cudaSuccess) e = ens_smem(k_ens_spec<MODE, 4>, kEnsBSmem);
   if (e == cudaSuccess) e = ens_smem(k_ens_spec<MODE, 4, true>, kEnsBSmem);
   return e;
 }
 cudaError_t ens_attrs() {
   cudaError_t e = ens_smem(k_ens_pair_cols, kEnsPairSmem);
+  if (e == cudaSuccess) e = ens_smem(k_ens_pair_rows, kEnsPairSmem);
   if (e == cudaSuccess) e = ens_smem(k_ens_phys<2>, kEnsASmem);
   if (e == cudaSuccess) e = ens_spec_attrs<-1>();
   if (e == cudaSuccess) e = ens_spec_attrs<0>();
@@ -256,7 +244,7 @@ cudaError_t ens_attrs() {
 }
 const void* ens_phys_fn(int v) { return v == 0 ? (const void*)k_ens_pair_cols : (const void*)k_ens_phys<2>; }
 const void* ens_spec_fn(int v) {
-  return v == 0 ? (const void*)k_ens_pair_rows<1> : v == 1 ? (const void*)k_ens_spec<1, 6>
+  return v == 0 ? (const void*)k_ens_pair_rows : v == 1 ? (const void*)k_ens_spec<1, 6>
          : v == 2 ? (const void*)k_ens_spec<1, 4> : (const void*)k_ens_spec<1, 4, true>;
 }
 // one shape's work list and persistent grid
@@ -264,25 +252,55 @@ struct EnsWork {
   const int2* items;
   int nitems, grid;
 };
+// pair kernels with programmatic stream serialisation (pdl_wait)
+template <class... P, class... A>
+void ens_launch_pair(void (*kernel)(P...), int threads, size_t smem, const EnsWork& w, cudaStream_t st, A... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(w.grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, args...);
+}
 void ens_launch_phys(int v, const EnsWork& w, cudaStream_t st, const EnsInst* inst, Pools pool) {
-  if (v == 0) k_ens_pair_cols<<<w.grid, kEnsPairThreads, kEnsPairSmem, st>>>(inst, w.items, w.nitems, pool);
+  if (v == 0) {
+    PhysArgs a{};
+    a.pa = pool.pa;
+    a.pb = pool.pb;
+    a.z = pool.z;
+    ens_launch_pair(k_ens_pair_cols, kEnsPairThreads, kEnsPairSmem, w, st, inst, w.items, w.nitems, a);
+  }
   else k_ens_phys<2><<<w.grid, kEnsAThreads, kEnsASmem, st>>>(inst, w.items, w.nitems, pool);
 }
 template <int MODE>
 void ens_launch_spec_m(int v, const EnsWork& w, cudaStream_t st, const EnsInst* inst, Pools pool, int phase,
-                       int full_pb, int* err) {
-  if (v == 0)
-    k_ens_pair_rows<MODE><<<w.grid, kEnsPairThreads, kEnsPairSmem, st>>>(inst, w.items, w.nitems, pool, phase, full_pb);
-  else if (v == 1) k_ens_spec<MODE, 6><<<w.grid, kEnsBThreads, kEnsBSmem, st>>>(inst, w.items, w.nitems, pool, phase, err);
+                       int* err) {
+  if (v == 1) k_ens_spec<MODE, 6><<<w.grid, kEnsBThreads, kEnsBSmem, st>>>(inst, w.items, w.nitems, pool, phase, err);
   else if (v == 2) k_ens_spec<MODE, 4><<<w.grid, kEnsBThreads, kEnsBSmem, st>>>(inst, w.items, w.nitems, pool, phase, err);
   else k_ens_spec<MODE, 4, true><<<w.grid, kEnsBThreads, kEnsBSmem, st>>>(inst, w.items, w.nitems, pool, phase, err);
 }
 void ens_launch_spec(int mode, int v, const EnsWork& w, cudaStream_t st, const EnsInst* inst, Pools pool, int phase,
                      int full_pb, int* err) {
-  if (mode < 0) ens_launch_spec_m<-1>(v, w, st, inst, pool, phase, full_pb, err);
-  else if (mode == 0) ens_launch_spec_m<0>(v, w, st, inst, pool, phase, full_pb, err);
-  else if (mode == 1) ens_launch_spec_m<1>(v, w, st, inst, pool, phase, full_pb, err);
-  else ens_launch_spec_m<2>(v, w, st, inst, pool, phase, full_pb, err);
+  if (v == 0) {
+    const int s = mode < 0 ? 0 : mode;
+    SpecArgs a{};
+    a.z = pool.z;
+    a.w0 = pool.s[phase];
+    a.wcur = pool.s[(phase + s) % 3];
+    a.wout = pool.s[(phase + (s == 1 ? 2 : 1)) % 3];
+    a.pa = pool.pa;
+    a.pb = pool.pb;
+    a.full_pb = full_pb;
+    ens_launch_pair(k_ens_pair_rows, kEnsPairThreads, kEnsPairSmem, w, st, inst, w.items, w.nitems, a, mode);
+  } else if (mode < 0) ens_launch_spec_m<-1>(v, w, st, inst, pool, phase, err);
+  else if (mode == 0) ens_launch_spec_m<0>(v, w, st, inst, pool, phase, err);
+  else if (mode == 1) ens_launch_spec_m<1>(v, w, st, inst, pool, phase, err);
+  else ens_launch_spec_m<2>(v, w, st, inst, pool, phase, err);
 }
 
 __global__ void k_ens_twiddles(float2* tw, int n) {
@@ -349,15 +367,15 @@ struct EnsTiles {
   int a, b, pa, pb;
 };
 template <int N> EnsTiles tiles_of() {
-  return {Tune<N>::A_GRID, Tune<N>::B_GRID, EnsPair<N>::A_GRID, EnsPair<N>::B_GRID};
+  return {Tune<N>::A_GRID, Tune<N>::B_GRID, EnsCols<N>::GRID, EnsRows<N>::GRID};
 }
 EnsTiles tiles_of(int n) {
   return n == 64 ? tiles_of<64>() : n == 128 ? tiles_of<128>() : n == 256 ? tiles_of<256>()
          : n == 512 ? tiles_of<512>() : tiles_of<1024>();
 }
 template <int N> cudaError_t ens_make_ptw(float4* out, const float2* tw, cudaStream_t st) {
-  constexpr int size = PassTw<N, EnsPair<N>::V>::SIZE;
-  k_pass_twiddles<N, EnsPair<N>::V><<<(size + 255) / 256, 256, 0, st>>>(out, tw);
+  static_assert(PassTw<N, EnsCols<N>::V>::SIZE <= N && EnsCols<N>::V == EnsRows<N>::V, "one table below n entries");
+  k_pass_twiddles<N, EnsCols<N>::V><<<(N + 255) / 256, 256, 0, st>>>(out, tw);
   return cudaGetLastError();
 }
 cudaError_t ens_make_ptw(int n, float4* out, const float2* tw, cudaStream_t st) {

@@ -81,7 +81,7 @@ struct PhysArgs {
   float2* z;            // product spectrum after the y-FFT, [ky][x], in-band rows
   float2* vel;          // physical (u, v), [y][x]
   float* partials;      // per-CTA max |u|+|v|
-  unsigned* ticket;     // last-CTA-done counter
+  unsigned* ticket;     // last-CTA-done counter, then the maximum k_pair_cols accumulates
   float* dt_out;        // dt slot written by the last CTA: [dt, speed]
   const DevParams* params;
   const float2* tw;
@@ -120,6 +120,8 @@ struct SpecArgs {
   int* row_nz;          // non-null: per row, 1 if the written PA/PB row holds a nonzero value;
                         // a CTA whose rows are all zero then skips its transforms and stores
   const float4* ptw;    // pass-ordered twiddles of the pair kernels (s2d_pairs.cuh)
+  unsigned* top;        // pair kernel, last stage: max |u|+|v| (bits) left by k_pair_cols, or null
+  float* dt_out;        // ... and the dt slot it goes to: [dt, speed]
   int full_pb;          // pair kernel: also write the rows ky < 0 of PB (readers other than k_pair_cols)
 };
 

@@ -42,8 +42,9 @@ struct NOps {
   cudaError_t (*set_attrs)();   // FFT passes and every registered stage variant
   void (*fft_rows)(int sign, float2* data, const float2* tw, cudaStream_t st);
   void (*fft_cols)(int sign, float2* data, const float2* tw, cudaStream_t st);
-  // pass-ordered twiddles of the pair kernels
-  int ptw_size;
+  // pass-ordered twiddles of the pair kernels: entries, and where the rows' table starts
+  int ptw_size, ptw_rows;
+  bool blocked_packs;   // the pair kernels keep the packs in blocks of four columns
   void (*make_ptw)(float4* out, const float2* tw, cudaStream_t st);
   int n_phys = 0, n_spec = 0;
   PhysVariant phys[kMaxVariants];
@@ -101,50 +102,47 @@ template <int N, class TU> struct SpecImpl {
 };
 
 // ---------------------------------------------------------------- pair-kernel variants
-template <class TU> struct PairImpl {
-  static cudaError_t phys_attrs() {
-    cudaError_t e = set_smem(k_pair_cols<0, TU>, TU::A_SMEM);
-    if (e == cudaSuccess) e = set_smem(k_pair_cols<1, TU>, TU::A_SMEM);
-    if (e == cudaSuccess) e = set_smem(k_pair_cols<2, TU>, TU::A_SMEM);
-    return e;
-  }
+// launched with programmatic stream serialisation (pdl_wait)
+template <class A> inline void launch_pdl(void (*kernel)(A, int), int grid, int threads, size_t smem, cudaStream_t st,
+                                          const A& a, int mode) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, a, mode);
+}
+template <int N> struct PairImpl {
+  using C = typename PairShape<N>::C;
+  using R = typename PairShape<N>::R;
+  static_assert(C::BP == R::BP, "one pack layout");
+  static cudaError_t phys_attrs() { return set_smem(k_pair_cols<C>, C::SMEM); }
   static void phys_run(int mode, const PhysArgs& a, cudaStream_t st) {
-    const dim3 g(TU::A_GRID), b(TU::A_THREADS);
-    if (mode == 0) k_pair_cols<0, TU><<<g, b, TU::A_SMEM, st>>>(a);
-    else if (mode == 1) k_pair_cols<1, TU><<<g, b, TU::A_SMEM, st>>>(a);
-    else k_pair_cols<2, TU><<<g, b, TU::A_SMEM, st>>>(a);
+    launch_pdl<PhysArgs>(k_pair_cols<C>, C::GRID, C::THREADS, C::SMEM, st, a, mode);
   }
-  template <int MODE, bool PTR> static cudaError_t attr() { return set_smem(k_pair_rows<MODE, PTR, TU>, TU::B_SMEM); }
-  static cudaError_t spec_attrs() {
-    cudaError_t e = cudaSuccess;
-    for (cudaError_t r : {attr<-1, false>(), attr<0, false>(), attr<1, false>(), attr<2, false>(), attr<0, true>(),
-                          attr<1, true>(), attr<2, true>()})
-      if (r != cudaSuccess && e == cudaSuccess) e = r;
-    return e;
-  }
-  template <int MODE, bool PTR> static void launch(const SpecArgs& a, cudaStream_t st) {
-    k_pair_rows<MODE, PTR, TU><<<dim3(TU::B_GRID), dim3(TU::B_THREADS), TU::B_SMEM, st>>>(a);
-  }
-  static void spec_run(int mode, bool ptr, const SpecArgs& a, cudaStream_t st) {
-    switch (mode) {
-      case -1: launch<-1, false>(a, st); break;
-      case 0: ptr ? launch<0, true>(a, st) : launch<0, false>(a, st); break;
-      case 1: ptr ? launch<1, true>(a, st) : launch<1, false>(a, st); break;
-      default: ptr ? launch<2, true>(a, st) : launch<2, false>(a, st); break;
-    }
+  static cudaError_t spec_attrs() { return set_smem(k_pair_rows<R>, R::SMEM); }
+  static void spec_run(int mode, bool, const SpecArgs& a, cudaStream_t st) {
+    launch_pdl<SpecArgs>(k_pair_rows<R>, R::GRID, R::THREADS, R::SMEM, st, a, mode);
   }
   static PhysVariant phys() { return PhysVariant{"column pairs", &phys_attrs, &phys_run, true}; }
   static SpecVariant spec() { return SpecVariant{"row pairs", &spec_attrs, &spec_run, true}; }
+  // pass-ordered twiddles: the columns' table, then the rows'
+  static constexpr int CTW = PassTw<N, C::V>::SIZE, RTW = PassTw<N, R::V>::SIZE;
+  static void make_ptw(float4* out, const float2* tw, cudaStream_t st) {
+    k_pass_twiddles<N, C::V><<<(CTW + 255) / 256, 256, 0, st>>>(out, tw);
+    k_pass_twiddles<N, R::V><<<(RTW + 255) / 256, 256, 0, st>>>(out + CTW, tw);
+  }
 };
 
 // ---------------------------------------------------------------- per-size table
 template <int N> struct OpsImpl {
   using TU = Tune<N>;
-  using PT = PairShape<N>;
-  static void make_ptw(float4* out, const float2* tw, cudaStream_t st) {
-    constexpr int size = PassTw<N, PT::V>::SIZE;
-    k_pass_twiddles<N, PT::V><<<(size + 255) / 256, 256, 0, st>>>(out, tw);
-  }
+  using PT = PairImpl<N>;
   static cudaError_t fft_attrs() {
     cudaError_t e = cudaSuccess;
     auto chk = [&](cudaError_t r) { if (r != cudaSuccess && e == cudaSuccess) e = r; };
@@ -180,10 +178,12 @@ template <int N> struct OpsImpl {
     o.set_attrs = &fft_attrs;
     o.fft_rows = &fft_rows;
     o.fft_cols = &fft_cols;
-    o.ptw_size = PassTw<N, PT::V>::SIZE;
-    o.make_ptw = &make_ptw;
-    o.phys[o.n_phys++] = PairImpl<PT>::phys();
-    o.spec[o.n_spec++] = PairImpl<PT>::spec();
+    o.ptw_size = PT::CTW + PT::RTW;
+    o.ptw_rows = PT::CTW;
+    o.make_ptw = &PT::make_ptw;
+    o.blocked_packs = PT::C::BP;
+    o.phys[o.n_phys++] = PT::phys();
+    o.spec[o.n_spec++] = PT::spec();
     o.phys[o.n_phys++] = PhysImpl<N, TU>::make("V=16");
     o.spec[o.n_spec++] = SpecImpl<N, TU>::make("V=16");
     for (const PhysVariant& v : extra_phys)

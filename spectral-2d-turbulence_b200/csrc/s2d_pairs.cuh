@@ -127,34 +127,52 @@ template <int N, int V> __global__ void k_pass_twiddles(float4* out, const float
 }
 
 // ------------------------------------------------------------------ launch shapes
-// V values per thread and line; GP column pairs per column CTA; BTHREADS threads per row CTA
-// (a multiple of T = N/V: whole row pairs); resident CTAs the register budget must allow.
-template <int N_, int V_, int GP_, int BTHREADS_, int AMINB_, int BMINB_> struct PairTune {
+// Column kernels run GP column pairs of T = N/V threads per CTA, row kernels THREADS / T whole
+// row pairs; MINB is the number of resident CTAs the register budget must allow.  BP_: the
+// packs between the two are stored in blocks of four columns, [x/4][ky][4], so that a column
+// CTA reads contiguous lines (and a row CTA writes 32-byte sectors).
+template <int N_, int V_, bool BP_ = false> struct PairLine {
   static constexpr int N = N_, V = V_, T = N / V;
+  static constexpr bool BP = BP_;
   using PL = LinePlan<N, V>;
   static constexpr int KMAX = N / 3;          // largest in-band wavenumber: |k| < N/3, N a power of two
   static constexpr int BAND = KMAX + 1;       // in-band k = 0..KMAX: row pairs, and columns of a thread quad
   __host__ __device__ static constexpr int pad(int i) { return i + i / V; }
   static constexpr int PADDED = N + T;
-  // columns
-  static constexpr int GP = GP_, A_THREADS = GP * T, A_GRID = N / 2 / GP, A_MINB = AMINB_;
-  static constexpr size_t A_SMEM = (size_t)PADDED * GP * (sizeof(float4) + sizeof(float2));
-  // rows
-  static constexpr int B_THREADS = BTHREADS_, PPB = B_THREADS / T, B_MINB = BMINB_;
-  static constexpr int B_GRID = (BAND + PPB - 1) / PPB;
-  static constexpr size_t B_SMEM = (size_t)PADDED * PPB * (sizeof(float4) + sizeof(float2));
-  static_assert(B_THREADS % T == 0 && (N / 2) % GP == 0, "whole lines");
 };
-template <int N> struct PairShapeOf;
-template <> struct PairShapeOf<32> { using type = PairTune<32, 8, 8, 32, 16, 16>; };
-template <> struct PairShapeOf<64> { using type = PairTune<64, 8, 4, 32, 16, 16>; };
-template <> struct PairShapeOf<128> { using type = PairTune<128, 8, 2, 32, 16, 16>; };
-template <> struct PairShapeOf<256> { using type = PairTune<256, 8, 2, 32, 8, 16>; };
-template <> struct PairShapeOf<512> { using type = PairTune<512, 8, 2, 64, 4, 8>; };
-template <> struct PairShapeOf<1024> { using type = PairTune<1024, 8, 2, 128, 2, 4>; };
-template <> struct PairShapeOf<2048> { using type = PairTune<2048, 8, 2, 256, 1, 2>; };
-template <> struct PairShapeOf<4096> { using type = PairTune<4096, 8, 1, 512, 1, 1>; };
-template <int N> using PairShape = typename PairShapeOf<N>::type;
+template <int N_, int V_, int GP_, int MINB_, bool BP_ = false> struct PairCols : PairLine<N_, V_, BP_> {
+  using L = PairLine<N_, V_, BP_>;
+  static constexpr int GP = GP_, THREADS = GP * L::T, GRID = N_ / 2 / GP, MINB = MINB_;
+  static constexpr size_t SMEM = (size_t)L::PADDED * GP * (sizeof(float4) + sizeof(float2));
+  static_assert((N_ / 2) % GP == 0 && (!BP_ || GP >= 2), "whole lines and blocks");
+};
+template <int N_, int V_, int THREADS_, int MINB_, bool BP_ = false> struct PairRows : PairLine<N_, V_, BP_> {
+  using L = PairLine<N_, V_, BP_>;
+  static constexpr int THREADS = THREADS_, PPB = THREADS / L::T, GRID = (L::BAND + PPB - 1) / PPB, MINB = MINB_;
+  static constexpr size_t SMEM = (size_t)L::PADDED * PPB * (sizeof(float4) + sizeof(float2));
+  static_assert(THREADS % L::T == 0, "whole lines");
+};
+// The shapes in use, each the fastest of those timed in turn on a B200 (us per launch, graph
+// replayed, columns / rows of stage 1):
+//   64     V=4  1.7 /  3.7     V=8  1.8 /  5.1
+//   256    V=4  2.6 /  4.1     V=8  2.6 /  5.4
+//   512    V=8  3.3 /  5.7     V=4  4.3 /  6.0    V=16  5.3 / 10
+//   1024   columns V=16, 8 columns a CTA 7.4 (4 columns 8.1, V=8 9.3); rows V=8, 3 CTAs/SM 10.0
+//          (4 CTAs/SM 11.9, V=16 11, V=4 15)
+//   2048   V=16 34 / 29 (4 row CTAs/SM 32.5)    V=8 43 / 33
+//   4096   V=16 in blocks 129 / 134, in rows 189 / 125    V=8 183 / 173
+// Small grids want more threads per line (the chain of a thread's cells sets the time), large
+// ones fewer, longer passes (shared-memory traffic does).  Blocked packs pay where a column's
+// rows lie 32 KB apart (4096); at 2048 the row kernel loses what the column kernel gains.
+template <int N> struct PairShape;
+template <> struct PairShape<32> { using C = PairCols<32, 4, 4, 16>; using R = PairRows<32, 4, 32, 16>; };
+template <> struct PairShape<64> { using C = PairCols<64, 4, 2, 16>; using R = PairRows<64, 4, 32, 16>; };
+template <> struct PairShape<128> { using C = PairCols<128, 4, 1, 16>; using R = PairRows<128, 4, 32, 16>; };
+template <> struct PairShape<256> { using C = PairCols<256, 4, 1, 8>; using R = PairRows<256, 4, 64, 8>; };
+template <> struct PairShape<512> { using C = PairCols<512, 8, 2, 4>; using R = PairRows<512, 8, 64, 8>; };
+template <> struct PairShape<1024> { using C = PairCols<1024, 16, 4, 1>; using R = PairRows<1024, 8, 128, 3>; };
+template <> struct PairShape<2048> { using C = PairCols<2048, 16, 4, 1>; using R = PairRows<2048, 16, 128, 3>; };
+template <> struct PairShape<4096> { using C = PairCols<4096, 16, 2, 1, true>; using R = PairRows<4096, 16, 256, 2, true>; };
 template <class TU> __device__ __forceinline__ bool pair_inband(int i) { return i <= TU::KMAX || i >= TU::N - TU::KMAX; }
 // whether register slot m (indices T m .. T m + T - 1) holds no in-band index
 template <class TU> __host__ __device__ constexpr bool slot_empty(int m) {
@@ -170,11 +188,11 @@ template <int T, int NTHREADS> struct GroupSync {
   }
 };
 
-// One packed pair of lines and, with HASV, one more single line, transformed in lockstep.
+// A packed pair of lines (HASX) and/or one single line (HASY), transformed in lockstep.
 // Element i of the pair is at l4[pad(i) * ST], of the single line at l2[pad(i) * ST].
-template <class TU, int SIGN, bool HASV, int ST, class Sync>
-__device__ __forceinline__ void pair_fft(C2 (&x)[TU::V], float2 (&y)[TU::V], float4* l4, float2* l2, int t,
-                                         const float4* __restrict__ tw, const Sync& sync) {
+template <class TU, int SIGN, bool HASX, bool HASY, int ST, class Sync>
+__device__ __forceinline__ void lines_fft(C2 (&x)[TU::V], float2 (&y)[TU::V], float4* l4, float2* l2, int t,
+                                          const float4* __restrict__ tw, const Sync& sync) {
   using PL = typename TU::PL;
   constexpr int N = TU::N, V = TU::V, T = TU::T;
   sfor<PL::P>([&](auto pc) {
@@ -187,40 +205,36 @@ __device__ __forceinline__ void pair_fft(C2 (&x)[TU::V], float2 (&y)[TU::V], flo
       for (int b = 0; b < B; ++b)
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-          v[b * R + r] = x[b + B * r];
-          if constexpr (HASV) w[b * R + r] = y[b + B * r];
+          if constexpr (HASX) v[b * R + r] = x[b + B * r];
+          if constexpr (HASY) w[b * R + r] = y[b + B * r];
         }
     } else {
-      float4 f[V];
-#pragma unroll
-      for (int b = 0; b < B; ++b)
-#pragma unroll
-        for (int r = 1; r < R; ++r)
-          f[b * R + r] = __ldg(tw + PassTw<N, V>::offset(p) + (r - 1) * NS + ((t + T * b) & (NS - 1)));
 #pragma unroll
       for (int b = 0; b < B; ++b)
 #pragma unroll
         for (int r = 0; r < R; ++r) {
           const int i = TU::pad(t + T * b + r * (N / R)) * ST;
-          const float4 q = l4[i];
-          v[b * R + r] = {make_float2(q.x, q.y), make_float2(q.z, q.w)};
-          if constexpr (HASV) w[b * R + r] = l2[i];
+          if constexpr (HASX) {
+            const float4 q = l4[i];
+            v[b * R + r] = {make_float2(q.x, q.y), make_float2(q.z, q.w)};
+          }
+          if constexpr (HASY) w[b * R + r] = l2[i];
         }
       sync();
 #pragma unroll
       for (int b = 0; b < B; ++b)
 #pragma unroll
         for (int r = 1; r < R; ++r) {
-          const float4 q = f[b * R + r];
+          const float4 q = __ldg(tw + PassTw<N, V>::offset(p) + (r - 1) * NS + ((t + T * b) & (NS - 1)));
           const float2 c = make_float2(q.x, q.y), s = make_float2(q.z, q.w);
-          v[b * R + r] = cmul_cs(v[b * R + r], c, SIGN > 0 ? s : neg2(s));
-          if constexpr (HASV) w[b * R + r] = cmul(w[b * R + r], make_float2(q.x, SIGN > 0 ? q.z : -q.z));
+          if constexpr (HASX) v[b * R + r] = cmul_cs(v[b * R + r], c, SIGN > 0 ? s : neg2(s));
+          if constexpr (HASY) w[b * R + r] = cmul(w[b * R + r], make_float2(q.x, SIGN > 0 ? q.z : -q.z));
         }
     }
 #pragma unroll
     for (int b = 0; b < B; ++b) {
-      DftE<R, SIGN, C2>::run(&v[b * R]);
-      if constexpr (HASV) DftE<R, SIGN, float2>::run(&w[b * R]);
+      if constexpr (HASX) DftE<R, SIGN, C2>::run(&v[b * R]);
+      if constexpr (HASY) DftE<R, SIGN, float2>::run(&w[b * R]);
     }
     if constexpr (p < PL::P - 1) {
 #pragma unroll
@@ -230,9 +244,11 @@ __device__ __forceinline__ void pair_fft(C2 (&x)[TU::V], float2 (&y)[TU::V], flo
 #pragma unroll
         for (int r = 0; r < R; ++r) {
           const int i = TU::pad(base + r * NS) * ST;
-          const C2 q = v[b * R + r];
-          l4[i] = make_float4(q.re.x, q.re.y, q.im.x, q.im.y);
-          if constexpr (HASV) l2[i] = w[b * R + r];
+          if constexpr (HASX) {
+            const C2 q = v[b * R + r];
+            l4[i] = make_float4(q.re.x, q.re.y, q.im.x, q.im.y);
+          }
+          if constexpr (HASY) l2[i] = w[b * R + r];
         }
       }
       sync();
@@ -241,18 +257,22 @@ __device__ __forceinline__ void pair_fft(C2 (&x)[TU::V], float2 (&y)[TU::V], flo
       for (int b = 0; b < B; ++b)
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-          x[b + B * r] = v[b * R + r];
-          if constexpr (HASV) y[b + B * r] = w[b * R + r];
+          if constexpr (HASX) x[b + B * r] = v[b * R + r];
+          if constexpr (HASY) y[b + B * r] = w[b * R + r];
         }
     }
   });
 }
 
 // ------------------------------------------------------------------ columns
-// MODE as phys_cols_tile.  One column pair per group; groups interleave over lanes (two
-// pairs are one 32-byte sector per row).  Returns this thread's max |u|+|v| (MODE != 1).
-template <int MODE, class TU>
-__device__ __forceinline__ float pair_cols_tile(const PhysArgs& a, int tile, float4* smem) {
+// `mode` as phys_cols_tile's MODE, at run time: the stages of a step then share one kernel's
+// code, which stays in the instruction caches from launch to launch.  `base` is the grid's first
+// cell in the arrays of `a` (kernel arguments: pointers in registers cost spills) and ptw
+// its twiddles.  One column pair per group; groups interleave over lanes (two pairs are one 32-byte sector per row).  Returns
+// this thread's max |u|+|v| (mode != 1).
+template <class TU>
+__device__ __forceinline__ float pair_cols_tile(const PhysArgs& a, size_t base, const float4* ptw, int mode, int tile,
+                                                float4* smem) {
   constexpr int N = TU::N, V = TU::V, T = TU::T, GP = TU::GP;
   const int g = threadIdx.x % GP, t = threadIdx.x / GP;
   const int x0 = 2 * (tile * GP + g);
@@ -260,31 +280,44 @@ __device__ __forceinline__ float pair_cols_tile(const PhysArgs& a, int tile, flo
   float2* const l2 = reinterpret_cast<float2*>(smem + TU::PADDED * GP) + g;
   struct Sync {
     __device__ __forceinline__ void operator()() const {
-      if constexpr (TU::A_THREADS <= 32) __syncwarp();
+      if constexpr (TU::THREADS <= 32) __syncwarp();
       else __syncthreads();
     }
   };
   C2 x[V];
   float2 y[V];
+  auto at = [&](int r) { return base + (TU::BP ? ((size_t)(x0 >> 2) * N + r) * 4 + (x0 & 3) : (size_t)r * N + x0); };
+  auto load_x = [&] {
 #pragma unroll
-  for (int m = 0; m < V; ++m) {
-    x[m] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-    y[m] = make_float2(0.f, 0.f);
-    const int row = t + T * m;
-    if (!slot_empty<TU>(m) && pair_inband<TU>(row)) {
-      const float4 p = __ldcs(reinterpret_cast<const float4*>(a.pa + (size_t)row * N + x0));
-      const bool up = row < N / 2;
-      const float4 q = __ldg(reinterpret_cast<const float4*>(a.pb + (size_t)(up ? row : N - row) * N + x0));
-      x[m] = {make_float2(p.x, p.z), make_float2(p.y, p.w)};
-      // V(x) + i V(x+1), conjugated spectra for -ky; row 0 is real
-      if (row == 0) y[m] = make_float2(q.x, q.z);
-      else y[m] = up ? make_float2(q.x - q.w, q.y + q.z) : make_float2(q.x + q.w, q.z - q.y);
+    for (int m = 0; m < V; ++m) {
+      const int row = t + T * m;
+      x[m] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+      if (!slot_empty<TU>(m) && pair_inband<TU>(row)) {
+        const float4 p = __ldcs(reinterpret_cast<const float4*>(a.pa + at(row)));
+        x[m] = {make_float2(p.x, p.z), make_float2(p.y, p.w)};
+      }
     }
-  }
-  pair_fft<TU, +1, true, GP>(x, y, l4, l2, t, a.ptw, Sync{});
+  };
+  auto load_y = [&] {
+#pragma unroll
+    for (int m = 0; m < V; ++m) {
+      const int row = t + T * m;
+      y[m] = make_float2(0.f, 0.f);
+      if (!slot_empty<TU>(m) && pair_inband<TU>(row)) {
+        const bool up = row < N / 2;
+        const float4 q = __ldg(reinterpret_cast<const float4*>(a.pb + at(up ? row : N - row)));
+        // V(x) + i V(x+1), conjugated spectra for -ky; row 0 is real
+        if (row == 0) y[m] = make_float2(q.x, q.z);
+        else y[m] = up ? make_float2(q.x - q.w, q.y + q.z) : make_float2(q.x + q.w, q.z - q.y);
+      }
+    }
+  };
+  load_x();
+  load_y();
+  lines_fft<TU, +1, true, true, GP>(x, y, l4, l2, t, ptw, Sync{});
   // re = omega, im = u at (x, x+1); y = v at (x, x+1)
   float speed = 0.f;
-  if constexpr (MODE != 1) {
+  if (mode != 1) {
 #pragma unroll
     for (int m = 0; m < V; ++m) {
       const float2 u = x[m].im, v = y[m];
@@ -292,216 +325,297 @@ __device__ __forceinline__ float pair_cols_tile(const PhysArgs& a, int tile, flo
       speed = fmaxf(speed, fmaxf(fabsf(u.x) + fabsf(v.x), fabsf(u.y) + fabsf(v.y)));
     }
   }
-  if constexpr (MODE != 0) {
+  if (mode != 0) {
 #pragma unroll
     for (int m = 0; m < V; ++m) {
       const float2 om = x[m].re;
       x[m] = {__fmul2_rn(x[m].im, om), __fmul2_rn(y[m], om)};
     }
-    pair_fft<TU, -1, false, GP>(x, y, l4, l2, t, a.ptw, Sync{});
+    lines_fft<TU, -1, true, false, GP>(x, y, l4, l2, t, ptw, Sync{});
 #pragma unroll
     for (int m = 0; m < V; ++m) {
       const int row = t + T * m;
       if (!slot_empty<TU>(m) && pair_inband<TU>(row))
-        *reinterpret_cast<float4*>(a.z + (size_t)row * N + x0) =
+        *reinterpret_cast<float4*>(a.z + base + (size_t)row * N + x0) =
             make_float4(x[m].re.x, x[m].im.x, x[m].re.y, x[m].im.y);
     }
   }
   return speed;
 }
 
-template <int MODE, class TU>
-__global__ void __launch_bounds__(TU::A_THREADS, TU::A_MINB) k_pair_cols(PhysArgs a) {
+// Programmatic dependent launch: a stage kernel may start while the one before it drains.
+// pdl_wait returns once that kernel has finished (and its writes are visible); every kernel
+// lets its successor start only after its own wait, so whatever ran two or more launches
+// back is complete when a kernel starts -- its prologue may read that, and nothing newer.
+__device__ __forceinline__ void pdl_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// CTA maximum of |u|+|v| into *top (bits of a non-negative float order as integers); the row
+// kernel behind it forms the next dt from the total (pair_cfl)
+template <int NTHREADS> __device__ __forceinline__ void cols_speed_max(unsigned* top, float speed) {
+  unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(speed));
+  if constexpr (NTHREADS > 32) {
+    __shared__ unsigned red[NTHREADS / 32];
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x < 32) m = __reduce_max_sync(0xffffffffu, threadIdx.x < NTHREADS / 32 ? red[threadIdx.x] : 0u);
+  }
+  if (threadIdx.x == 0) atomicMax(top, m);
+}
+
+template <class TU>
+__global__ void __launch_bounds__(TU::THREADS, TU::MINB) k_pair_cols(PhysArgs a, int mode) {
   extern __shared__ __align__(16) float4 smem4[];
+  pdl_wait();
   phys_latch(a);
-  const float speed = pair_cols_tile<MODE, TU>(a, blockIdx.x, smem4);
-  if constexpr (MODE != 1) cols_speed_finalize<TU::A_THREADS>(a, speed);
+  const float speed = pair_cols_tile<TU>(a, 0, a.ptw, mode, blockIdx.x, smem4);
+  if (mode == 2) cols_speed_max<TU::THREADS>(a.ticket + 1, speed);
+  else if (mode == 0) cols_speed_finalize<TU::THREADS>(a, speed);
 }
 
 // ------------------------------------------------------------------ rows
-// the state cells of one quad: (row a, col c), (a, -c), (b, c), (b, -c)
-struct Quad {
-  float2 v[4];
-};
-__device__ __forceinline__ Quad load_quad(const float2* s, size_t ra, size_t rb, int c, int mc) {
-  return {{s[ra + c], s[ra + mc], s[rb + c], s[rb + mc]}};
-}
 __device__ __forceinline__ C2 pair_of(float2 a, float2 b) { return {make_float2(a.x, b.x), make_float2(a.y, b.y)}; }
-// w + e w, w + conj(e) w
+// w + e w
 __device__ __forceinline__ C2 grow(C2 w, float2 e) { return cadd(w, cmul_w(w, e)); }
 
-// out of the stage update rk_update<S> for the two cells of a column, all factors finite
-template <int S> __device__ __forceinline__ C2 rk_pair(float2 e, float2 full, float2 mhalf, C2 w0, C2 adv) {
-  if constexpr (S == 0) {
-    return grow(adv, full);
-  } else if constexpr (S == 1) {
-    const C2 p = grow(w0, e), q = grow(adv, mhalf);
-    return {__ffma2_rn(p.re, splat2(0.75f), __fmul2_rn(q.re, splat2(0.25f))),
-            __ffma2_rn(p.im, splat2(0.75f), __fmul2_rn(q.im, splat2(0.25f)))};
-  } else {
-    const C2 p = grow(w0, full), q = grow(adv, e);   // q + (p - q)/3, see rk_update
-    const C2 d = csub(p, q);
-    return {__ffma2_rn(d.re, splat2(1.f / 3.f), q.re), __ffma2_rn(d.im, splat2(1.f / 3.f), q.im)};
-  }
+// Out-of-line parts of a cell quad: rare, and each would otherwise be copied into the kernel
+// with its trigonometric argument reductions (the row kernel waited on instruction fetches).
+// E(dt/2) - 1 where a series of half_factor_m1 does not reach
+static __device__ __noinline__ float2 half_factor_far(float x, float half_th) {
+  const float d = expm1_series(x);
+  float sh, ch;
+  sincos_series(half_th, &sh, &ch);
+  const float g = -2.f * sh * sh, sn = 2.f * sh * ch;
+  return make_float2(d + g + d * g, (1.f + d) * sn);
+}
+// the forcing of k = (kx, ky) and (-kx, ky); -k takes the conjugates
+static __device__ __noinline__ float4 stochastic_pair(const DevParams* P, int n, int p, int c, float dt) {
+  const float kx = (float)c, ky = (float)p, k2 = kx * kx + ky * ky;
+  const float2 f1 = stochastic_term(*P, n, p, c, kx, ky, k2, dt);
+  const float2 f2 = stochastic_term(*P, n, p, (n - c) & (n - 1), -kx, ky, k2, dt);
+  return make_float4(f1.x, f1.y, f2.x, f2.y);
+}
+// the stage update cell by cell where a factor overflows or vanishes: zero modes stay zero
+static __device__ __noinline__ float2 rk_cell(int stage, float2 e, float2 w0, float2 wc, float2 rhs, float dt) {
+  const bool quiet = wc.x == 0.f && wc.y == 0.f && w0.x == 0.f && w0.y == 0.f && rhs.x == 0.f && rhs.y == 0.f;
+  if (quiet) return make_float2(0.f, 0.f);
+  return stage == 0 ? rk_update<0>(e, w0, wc, rhs, dt)
+         : stage == 1 ? rk_update<1>(e, w0, wc, rhs, dt) : rk_update<2>(e, w0, wc, rhs, dt);
 }
 
-// one group's row pair; MODE as spec_rows_tile
-template <int MODE, bool PTR, class TU>
-__device__ __forceinline__ void pair_rows_tile(const SpecArgs& a, int tile, float4* smem) {
+// One group's row pair.  `stage` is the RK stage at run time (one kernel for the step, see
+// pair_cols_tile), -1 packs wcur only; the grid's parameters, step and twiddles come beside
+// the arrays of `a`, its first cell is `base`.
+template <class TU, bool WAIT = false>
+__device__ __forceinline__ void pair_rows_tile(const SpecArgs& a, size_t base, const DevParams* P, float dt, bool forced,
+                                               const float4* ptw, int stage, int tile, float4* smem) {
   constexpr int N = TU::N, V = TU::V, T = TU::T, BAND = TU::BAND, KMAX = TU::KMAX;
-  constexpr int Q = (BAND + T - 1) / T;
   const int t = threadIdx.x % T, g = threadIdx.x / T;
   const int p = min(tile * TU::PPB + g, KMAX);   // the last CTA's spare groups repeat pair KMAX
-  const size_t ra = (size_t)p * N, rb = (size_t)((N - p) & (N - 1)) * N;
+  const size_t ra = base + (size_t)p * N, rb = base + (size_t)((N - p) & (N - 1)) * N;
   float4* const l4 = smem + g * TU::PADDED;
   float2* const l2 = reinterpret_cast<float2*>(smem + TU::PPB * TU::PADDED) + g * TU::PADDED;
-  const GroupSync<T, TU::B_THREADS> sync;
+  const GroupSync<T, TU::THREADS> sync;
   C2 x[V];
   float2 y[V];
-  // every global load of the stage goes out here: Z first, then the quads' state cells
-  if constexpr (MODE >= 0) {
-#pragma unroll
-    for (int m = 0; m < V; ++m) x[m] = pair_of(__ldcs(a.z + ra + t + T * m), __ldcs(a.z + rb + t + T * m));
-  }
-  Quad wq[Q], w0q[Q];
-#pragma unroll
-  for (int q = 0; q < Q; ++q) {
-    const int c = t + T * q, mc = (N - c) & (N - 1);
+  const bool two = stage >= 1;   // w0 is not wcur
+  // state cells (row, column) = (a, c), (a, -c), (b, c), (b, -c) of the next column, the first
+  // loaded ahead of the x-transform
+  float2 nw[4], nw0[4];
+  auto fetch = [&](int c) {
     if (c < BAND) {
-      wq[q] = load_quad(a.wcur, ra, rb, c, mc);
-      if constexpr (MODE >= 1) w0q[q] = load_quad(a.w0, ra, rb, c, mc);
+      const int mc = (N - c) & (N - 1);
+      nw[0] = a.wcur[ra + c], nw[1] = a.wcur[ra + mc], nw[2] = a.wcur[rb + c], nw[3] = a.wcur[rb + mc];
+      if (two) nw0[0] = a.w0[ra + c], nw0[1] = a.w0[ra + mc], nw0[2] = a.w0[rb + c], nw0[3] = a.w0[rb + mc];
     }
-  }
-  const DevParams& P = *a.params;
-  const float dt = MODE >= 0 ? __ldg(a.dt) : 0.f;
-  if constexpr (MODE >= 0) {
-    pair_fft<TU, -1, false, 1>(x, y, l4, l2, t, a.ptw, sync);
+  };
+  fetch(t);
+  const float beta = P->beta, mu = P->mu, nu = P->nu_h;
+  const int hyper = P->hyper_p;
+  const float2 fb = forced ? forcing_k2_bounds(*P) : make_float2(1.f, 0.f);   // empty without forcing
+  const float ky = (float)p;
+  // all of the above is two or more launches old; Z is the launch before
+  if constexpr (WAIT) pdl_wait();
+  if (stage >= 0) {
+#pragma unroll
+    for (int m = 0; m < V; ++m) {
+      const int c = t + T * m;
+      x[m] = pair_of(__ldcs(a.z + ra + c), __ldcs(a.z + rb + c));
+    }
+    lines_fft<TU, -1, true, false, 1>(x, y, l4, l2, t, ptw, sync);
 #pragma unroll
     for (int m = 0; m < V; ++m) {
       const int c = t + T * m;
       if (!slot_empty<TU>(m) && pair_inband<TU>(c))
         l4[TU::pad(c)] = make_float4(x[m].re.x, x[m].re.y, x[m].im.x, x[m].im.y);
     }
-    sync();
   }
-  const float ky = (float)p;
+  sync();
   constexpr float inv_n2 = 1.0f / ((float)N * (float)N);
+#pragma unroll 1
+  for (int c = t; c < BAND; c += T) {
+    const int mc = (N - c) & (N - 1), ic = TU::pad(c), im = TU::pad(mc);
+    const float kx = (float)c;
+    const float k2 = kx * kx + ky * ky;
+    float2 wq[4], w0q[4];
 #pragma unroll
-  for (int q = 0; q < Q; ++q) {
-    const int c = t + T * q, mc = (N - c) & (N - 1);
-    if (c < BAND) {
-      const float kx = (float)c;
-      const float k2 = kx * kx + ky * ky;
-      C2 w = pair_of(wq[q].v[0], wq[q].v[2]), wm = pair_of(wq[q].v[1], wq[q].v[3]);   // columns c, -c
-      if constexpr (MODE >= 0) {
-        const float4 zc = l4[TU::pad(c)], zm = l4[TU::pad(mc)];   // (re a, re b, im a, im b)
-        // right-hand sides at k = (kx, ky) and (-kx, ky); the other two cells hold the conjugates
-        auto minus_nhat = [&](float kxs, float2 zk, float2 zp) {   // zp = Z(-k)
-          const float2 q1 = make_float2(0.5f * (zk.x + zp.x), 0.5f * (zk.y - zp.y));
-          const float2 q2 = make_float2(0.5f * (zk.y + zp.y), -0.5f * (zk.x - zp.x));
-          return make_float2(kxs * q1.y + ky * q2.y, -(kxs * q1.x) - ky * q2.x);
-        };
-        float2 r1 = minus_nhat(kx, make_float2(zc.x, zc.z), make_float2(zm.y, zm.w));
-        float2 r2 = minus_nhat(-kx, make_float2(zm.x, zm.z), make_float2(zc.y, zc.w));
-        if (a.stochastic && k2 > 0.f) {
-          const float2 fb = forcing_k2_bounds(P);
-          if (k2 >= fb.x && k2 <= fb.y) {
-            // the term of -k is the conjugate of that of k
-            const float2 f1 = stochastic_term(P, N, p, c, kx, ky, k2, dt);
-            const float2 f2 = stochastic_term(P, N, p, mc, -kx, ky, k2, dt);
-            r1 = cadd(r1, f1);
-            r2 = cadd(r2, f2);
-          }
-        }
-        C2 r = {make_float2(r1.x, r2.x), make_float2(r1.y, -r2.y)};
-        C2 rm = {make_float2(r2.x, r1.x), make_float2(r2.y, -r1.y)};
-        if constexpr (PTR) {
-          const Quad f = load_quad(a.fptr, ra, rb, c, mc);
-          r = cadd(r, pair_of(f.v[0], f.v[2]));
-          rm = cadd(rm, pair_of(f.v[1], f.v[3]));
-        }
-        const float2 e = half_factor_m1(P, kx, fmaxf(k2, 1.f), dt);
-        const float2 e1 = make_float2(1.f + e.x, e.y);
-        const float nrm = e1.x * e1.x + e1.y * e1.y;
-        C2 w0 = w, w0m = wm;
-        if constexpr (MODE >= 1) {
-          w0 = pair_of(w0q[q].v[0], w0q[q].v[2]);
-          w0m = pair_of(w0q[q].v[1], w0q[q].v[3]);
-        }
-        if (nrm > 1e-30f && nrm < 1e30f) {
-          const float2 full = cmul(e, make_float2(2.f + e.x, e.y));
-          float2 mhalf = make_float2(0.f, 0.f);
-          if constexpr (MODE == 1) {
-            const float rden = __frcp_rn(nrm);
-            const float2 qq = cmul(e, cconj(e1));
-            mhalf = make_float2(-qq.x * rden, -qq.y * rden);
-          }
-          const float2 d2 = splat2(dt);
-          const C2 adv = {__ffma2_rn(r.re, d2, w.re), __ffma2_rn(r.im, d2, w.im)};
-          const C2 advm = {__ffma2_rn(rm.re, d2, wm.re), __ffma2_rn(rm.im, d2, wm.im)};
-          w = rk_pair<MODE>(e, full, mhalf, w0, adv);
-          wm = rk_pair<MODE>(cconj(e), cconj(full), cconj(mhalf), w0m, advm);
-        } else {
-          // a factor that overflows or vanishes: cell by cell, zero modes stay zero
-          auto one = [&](float2 ee, float2 v0, float2 vc, float2 rr) {
-            const bool quiet = vc.x == 0.f && vc.y == 0.f && v0.x == 0.f && v0.y == 0.f && rr.x == 0.f && rr.y == 0.f;
-            return quiet ? make_float2(0.f, 0.f) : rk_update<MODE>(ee, v0, vc, rr, dt);
-          };
-          auto two = [&](float2 ee, C2 v0, C2 vc, C2 rr) {
-            return pair_of(one(ee, make_float2(v0.re.x, v0.im.x), make_float2(vc.re.x, vc.im.x), make_float2(rr.re.x, rr.im.x)),
-                           one(ee, make_float2(v0.re.y, v0.im.y), make_float2(vc.re.y, vc.im.y), make_float2(rr.re.y, rr.im.y)));
-          };
-          w = two(e, w0, w, r);
-          wm = two(cconj(e), w0m, wm, rm);
-        }
-        if (k2 == 0.f) w = wm = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-        a.wout[ra + c] = make_float2(w.re.x, w.im.x);
-        a.wout[ra + mc] = make_float2(wm.re.x, wm.im.x);
-        a.wout[rb + c] = make_float2(w.re.y, w.im.y);
-        a.wout[rb + mc] = make_float2(wm.re.y, wm.im.y);
+    for (int k = 0; k < 4; ++k) {
+      wq[k] = nw[k];
+      w0q[k] = nw0[k];
+    }
+    fetch(c + T);
+    C2 w = pair_of(wq[0], wq[2]), wm = pair_of(wq[1], wq[3]);   // columns c, -c
+    if (stage >= 0) {
+      const float4 zc = l4[ic], zm = l4[im];   // (re a, re b, im a, im b)
+      // right-hand sides at k = (kx, ky) and (-kx, ky); the other two cells hold the conjugates
+      auto minus_nhat = [&](float kxs, float2 zk, float2 zp) {   // zp = Z(-k)
+        const float2 q1 = make_float2(0.5f * (zk.x + zp.x), 0.5f * (zk.y - zp.y));
+        const float2 q2 = make_float2(0.5f * (zk.y + zp.y), -0.5f * (zk.x - zp.x));
+        return make_float2(kxs * q1.y + ky * q2.y, -(kxs * q1.x) - ky * q2.x);
+      };
+      float2 r1 = minus_nhat(kx, make_float2(zc.x, zc.z), make_float2(zm.y, zm.w));
+      float2 r2 = minus_nhat(-kx, make_float2(zm.x, zm.z), make_float2(zc.y, zc.w));
+      if (k2 > 0.f && k2 >= fb.x && k2 <= fb.y) {
+        const float4 f = stochastic_pair(P, N, p, c, dt);
+        r1 = cadd(r1, make_float2(f.x, f.y));
+        r2 = cadd(r2, make_float2(f.z, f.w));
       }
-      // next-stage packs scaled by 1/N^2: w + i u_hat = w (1 -+ ky/k2) on rows +-ky, and the
-      // Hermitian part of v_hat = -i kx w/k2 on row ky
-      const float inv = k2 > 0.f ? __frcp_rn(k2) : 0.f;
-      const float2 fa = make_float2((1.f - ky * inv) * inv_n2, (1.f + ky * inv) * inv_n2);
-      const float fb = 0.5f * (kx * inv * inv_n2);
-      const C2 pc = {__fmul2_rn(w.re, fa), __fmul2_rn(w.im, fa)}, pm = {__fmul2_rn(wm.re, fa), __fmul2_rn(wm.im, fa)};
-      const float2 vc = make_float2((w.im.x - wm.im.y) * fb, -(w.re.x + wm.re.y) * fb);
-      const float2 vm = make_float2(-(wm.im.x - w.im.y) * fb, (wm.re.x + w.re.y) * fb);
-      l4[TU::pad(c)] = make_float4(pc.re.x, pc.re.y, pc.im.x, pc.im.y);
-      l4[TU::pad(mc)] = make_float4(pm.re.x, pm.re.y, pm.im.x, pm.im.y);
-      l2[TU::pad(c)] = vc;
-      l2[TU::pad(mc)] = vm;
+      C2 r = {make_float2(r1.x, r2.x), make_float2(r1.y, -r2.y)};
+      C2 rm = {make_float2(r2.x, r1.x), make_float2(r2.y, -r1.y)};
+      if (a.fptr) {
+        r = cadd(r, pair_of(__ldg(a.fptr + ra + c), __ldg(a.fptr + rb + c)));
+        rm = cadd(rm, pair_of(__ldg(a.fptr + ra + mc), __ldg(a.fptr + rb + mc)));
+      }
+      C2 w0 = w, w0m = wm;
+      if (two) {
+        w0 = pair_of(w0q[0], w0q[2]);
+        w0m = pair_of(w0q[1], w0q[3]);
+      }
+      // E(dt/2) - 1 (half_factor_m1)
+      const float ex = (-mu - nu * powi(k2, hyper)) * (0.5f * dt);
+      const float hth = beta == 0.f ? 0.f : 0.5f * (beta * __fdividef(kx, fmaxf(k2, 1.f)) * (0.5f * dt));
+      float2 e;
+      if (fabsf(ex) < 0.25f && fabsf(hth) <= 0.78539816f) {
+        const float m1 = expm1_series(ex);
+        float sh, ch;
+        sincos_series(hth, &sh, &ch);
+        const float gg = -2.f * sh * sh, sn = 2.f * sh * ch;
+        e = make_float2(m1 + gg + m1 * gg, (1.f + m1) * sn);
+      } else {
+        e = half_factor_far(ex, hth);
+      }
+      const float2 e1 = make_float2(1.f + e.x, e.y);
+      const float nrm = e1.x * e1.x + e1.y * e1.y;
+      if (nrm > 1e-30f && nrm < 1e30f) {
+        // wout = B + cA (A - B), A = E(a dt) w0, B = E(b dt)(wcur + dt rhs): rk_update<stage>
+        const float2 full = cmul(e, make_float2(2.f + e.x, e.y));
+        float2 fA = full, fB = e;
+        float cA = 1.f / 3.f;
+        if (stage == 0) {
+          fB = full;
+          cA = 0.f;
+        } else if (stage == 1) {
+          const float rden = __frcp_rn(nrm);
+          const float2 qq = cmul(e, cconj(e1));
+          fA = e;
+          fB = make_float2(-qq.x * rden, -qq.y * rden);
+          cA = 0.75f;
+        }
+        const float2 d2 = splat2(dt), c2 = splat2(cA);
+        auto blend = [&](C2 v0, C2 vc, C2 rr, float2 ea, float2 eb) {
+          const C2 A = grow(v0, ea), B = grow({__ffma2_rn(rr.re, d2, vc.re), __ffma2_rn(rr.im, d2, vc.im)}, eb);
+          const C2 dd = csub(A, B);
+          return C2{__ffma2_rn(dd.re, c2, B.re), __ffma2_rn(dd.im, c2, B.im)};
+        };
+        w = blend(w0, w, r, fA, fB);
+        wm = blend(w0m, wm, rm, cconj(fA), cconj(fB));
+      } else {
+        auto cell2 = [&](float2 ee, C2 v0, C2 vc, C2 rr) {
+          return pair_of(rk_cell(stage, ee, make_float2(v0.re.x, v0.im.x), make_float2(vc.re.x, vc.im.x), make_float2(rr.re.x, rr.im.x), dt),
+                         rk_cell(stage, ee, make_float2(v0.re.y, v0.im.y), make_float2(vc.re.y, vc.im.y), make_float2(rr.re.y, rr.im.y), dt));
+        };
+        w = cell2(e, w0, w, r);
+        wm = cell2(cconj(e), w0m, wm, rm);
+      }
+      if (k2 == 0.f) w = wm = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+      a.wout[ra + c] = make_float2(w.re.x, w.im.x);
+      a.wout[ra + mc] = make_float2(wm.re.x, wm.im.x);
+      a.wout[rb + c] = make_float2(w.re.y, w.im.y);
+      a.wout[rb + mc] = make_float2(wm.re.y, wm.im.y);
     }
+    // next-stage packs scaled by 1/N^2: w + i u_hat = w (1 -+ ky/k2) on rows +-ky, and the
+    // Hermitian part of v_hat = -i kx w/k2 on row ky
+    const float inv = k2 > 0.f ? __frcp_rn(k2) : 0.f;
+    const float2 fa = make_float2((1.f - ky * inv) * inv_n2, (1.f + ky * inv) * inv_n2);
+    const float hb = 0.5f * (kx * inv * inv_n2);
+    const C2 pc = {__fmul2_rn(w.re, fa), __fmul2_rn(w.im, fa)}, pm = {__fmul2_rn(wm.re, fa), __fmul2_rn(wm.im, fa)};
+    const float2 vc = make_float2((w.im.x - wm.im.y) * hb, -(w.re.x + wm.re.y) * hb);
+    const float2 vm = make_float2(-(wm.im.x - w.im.y) * hb, (wm.re.x + w.re.y) * hb);
+    l4[ic] = make_float4(pc.re.x, pc.re.y, pc.im.x, pc.im.y);
+    l4[im] = make_float4(pm.re.x, pm.re.y, pm.im.x, pm.im.y);
+    l2[ic] = vc;
+    l2[im] = vm;
   }
   sync();
+  // in-band elements of a line, zeros elsewhere
+  auto load_x = [&] {
+#pragma unroll
+    for (int m = 0; m < V; ++m) {
+      const int c = t + T * m;
+      x[m] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+      if (!slot_empty<TU>(m) && pair_inband<TU>(c)) {
+        const float4 q = l4[TU::pad(c)];
+        x[m] = {make_float2(q.x, q.y), make_float2(q.z, q.w)};
+      }
+    }
+  };
+  auto load_y = [&] {
+#pragma unroll
+    for (int m = 0; m < V; ++m) {
+      const int c = t + T * m;
+      y[m] = !slot_empty<TU>(m) && pair_inband<TU>(c) ? l2[TU::pad(c)] : make_float2(0.f, 0.f);
+    }
+  };
+  const size_t bs = TU::BP && !a.full_pb ? (size_t)4 * N : 4, rs = TU::BP && !a.full_pb ? 4 : N;
+  auto pat = [&](int r, int c) { return base + (size_t)r * rs + (size_t)(c >> 2) * bs + (c & 3); };
+  auto store_y = [&] {
+#pragma unroll
+    for (int m = 0; m < V; ++m) {
+      const int c = t + T * m;
+      a.pb[pat(p, c)] = y[m];
+      if (a.full_pb && p > 0) a.pb[rb + c] = cconj(y[m]);
+    }
+  };
+  load_x();
+  load_y();
+  sync();
+  lines_fft<TU, +1, true, true, 1>(x, y, l4, l2, t, ptw, sync);
+  store_y();
 #pragma unroll
   for (int m = 0; m < V; ++m) {
     const int c = t + T * m;
-    x[m] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-    y[m] = make_float2(0.f, 0.f);
-    if (!slot_empty<TU>(m) && pair_inband<TU>(c)) {
-      const float4 q = l4[TU::pad(c)];
-      x[m] = {make_float2(q.x, q.y), make_float2(q.z, q.w)};
-      y[m] = l2[TU::pad(c)];
-    }
-  }
-  sync();
-  pair_fft<TU, +1, true, 1>(x, y, l4, l2, t, a.ptw, sync);
-#pragma unroll
-  for (int m = 0; m < V; ++m) {
-    const int c = t + T * m;
-    a.pa[ra + c] = make_float2(x[m].re.x, x[m].im.x);
-    a.pa[rb + c] = make_float2(x[m].re.y, x[m].im.y);
-    a.pb[ra + c] = y[m];
-    if (a.full_pb && p > 0) a.pb[rb + c] = cconj(y[m]);
+    a.pa[pat(p, c)] = make_float2(x[m].re.x, x[m].im.x);
+    a.pa[pat((N - p) & (N - 1), c)] = make_float2(x[m].re.y, x[m].im.y);
   }
 }
 
-template <int MODE, bool PTR, class TU>
-__global__ void __launch_bounds__(TU::B_THREADS, TU::B_MINB) k_pair_rows(SpecArgs a) {
+// the next dt from the maximum k_pair_cols left, by one thread of the last stage's row kernel
+// (its CTAs do not wait for it; as the column kernel's own last-CTA reduction it took 1.7 us)
+__device__ __forceinline__ void pair_cfl(const SpecArgs& a) {
+  const float m = __uint_as_float(*a.top);
+  a.dt_out[0] = cfl_dt(*a.params, m);
+  a.dt_out[1] = m;
+  *a.top = 0u;
+}
+
+template <class TU>
+__global__ void __launch_bounds__(TU::THREADS, TU::MINB) k_pair_rows(SpecArgs a, int stage) {
   extern __shared__ __align__(16) float4 smem4[];
-  pair_rows_tile<MODE, PTR, TU>(a, blockIdx.x, smem4);
+  pair_rows_tile<TU, true>(a, 0, a.params, stage >= 0 ? __ldg(a.dt) : 0.f, a.stochastic != 0, a.ptw, stage, blockIdx.x,
+                           smem4);
+  if (stage == 2 && a.top && blockIdx.x == 0 && threadIdx.x == 0) pair_cfl(a);
 }
 
 // the row flags of packs written by k_pair_rows: in-band rows
@@ -509,13 +623,20 @@ static __global__ void k_band_flags(int* row_nz, int n) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r < n) row_nz[r] = (r <= n / 3 || r >= n - n / 3) ? 1 : 0;
 }
-// packs written by k_pair_rows made whole: rows outside the band zero, PB(-ky) = conj PB(ky)
+// packs written by k_pair_rows made whole: rows outside the band zero, PB(-ky) = conj PB(ky);
+// a blocked pack ([x/4][ky][4]) is first copied to tmp and comes out in rows
 static __global__ void k_expand_packs(float2* pa, float2* pb, int n, int half_pb) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (size_t)n * n) return;
   const int r = (int)(i / n), c = (int)(i & (n - 1));
   if (r > n / 3 && r < n - n / 3) pa[i] = pb[i] = make_float2(0.f, 0.f);
   else if (half_pb && r > n / 2) pb[i] = cconj(pb[(size_t)(n - r) * n + c]);
+}
+static __global__ void k_unblock_pack(float2* out, const float2* __restrict__ tmp, int n) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= (size_t)n * n) return;
+  const int r = (int)(i / n), c = (int)(i & (n - 1));
+  out[i] = tmp[((size_t)(c >> 2) * n + r) * 4 + (c & 3)];
 }
 
 // whether a (prefix of a) complex n x n spectrum is zero outside the dealias band

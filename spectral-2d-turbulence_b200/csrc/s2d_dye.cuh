@@ -22,6 +22,7 @@
 //     the corrected texel's alpha is 1 whatever the inputs.
 #pragma once
 #include <cuda_fp16.h>
+#include "s2d_async.cuh"
 #include "s2d_device.cuh"
 
 namespace s2d {
@@ -157,18 +158,9 @@ __device__ __forceinline__ float2 texel_pos(int x, int y, float inv_m) {
 }
 __device__ __forceinline__ float2 texel_pos(int x, int y, int m) { return texel_pos(x, y, __frcp_rn((float)m)); }
 
-// BFECC correction of one texel from its source (a, with the 4-texel min/max) and
-// back-advected (b) samples, fade and splat dye (dye.wgsl:81-112); pos() gives the texel
-// centre, formed only when there are splats to place
+// a corrected texel plus the splat dye at its centre pos(), formed only when there are splats
 template <class POS>
-__device__ __forceinline__ uint2 correct_from(const Rgba& a, const Rgba& b, const Rgba& lo, const Rgba& hi,
-                                              const POS& pos, float fade, const DevSplats* __restrict__ S) {
-  auto corr = [&](float x, float y, float l, float u) {
-    return __fmul_rn(fminf(fmaxf(__fsub_rn(__fmul_rn(1.5f, x), __fmul_rn(0.5f, y)), l), u), fade);
-  };
-  float r = corr(a.r, b.r, lo.r, hi.r);
-  float g = corr(a.g, b.g, lo.g, hi.g);
-  float bb = corr(a.b, b.b, lo.b, hi.b);
+__device__ __forceinline__ uint2 splat_texel(float r, float g, float bb, const POS& pos, const DevSplats* __restrict__ S) {
   const int cnt = S->count;
   if (cnt == 0) return pack_texel(r, g, bb, 1.f);
   const float2 p = pos();
@@ -186,6 +178,18 @@ __device__ __forceinline__ uint2 correct_from(const Rgba& a, const Rgba& b, cons
     }
   }
   return pack_texel(r, g, bb, 1.f);
+}
+
+// BFECC correction of one texel from its source (a, with the 4-texel min/max) and
+// back-advected (b) samples, fade and splat dye (dye.wgsl:81-112); pos() gives the texel
+// centre, formed only when there are splats to place
+template <class POS>
+__device__ __forceinline__ uint2 correct_from(const Rgba& a, const Rgba& b, const Rgba& lo, const Rgba& hi,
+                                              const POS& pos, float fade, const DevSplats* __restrict__ S) {
+  auto corr = [&](float x, float y, float l, float u) {
+    return __fmul_rn(fminf(fmaxf(__fsub_rn(__fmul_rn(1.5f, x), __fmul_rn(0.5f, y)), l), u), fade);
+  };
+  return splat_texel(corr(a.r, b.r, lo.r, hi.r), corr(a.g, b.g, lo.g, hi.g), corr(a.b, b.b, lo.b, hi.b), pos, S);
 }
 
 template <class SF, class BF>
@@ -228,15 +232,13 @@ __global__ void k_dye_correct(const float2* __restrict__ vel, const uint2* __res
 // (floor(x + d) is x - 1 or x for |d| < 1) has the bilinear footprint [x - 1, x + 1], so
 // each level extends the region by one texel on each side.
 constexpr int kDyeLo = 1, kDyeHi = 1;
-constexpr int kDyeTileY = 32;
-// Output tile TX x 32 (TX = 64 when the dye is refined over the flow: 103 KB of windows,
-// 2 CTAs of 512 threads per SM, and 20 % / 10 % of recomputed forward / backward halo
-// texels instead of 28 % / 14 % at TX = 32; TX = 32 otherwise, where the velocity window
-// is as large as the dye windows)
-template <int TX> struct DyeGeom {
-  static constexpr int TY = kDyeTileY;
-  static constexpr int THREADS = TX * 8;
-  static constexpr int MINB = TX >= 64 ? 2 : 3;   // resident CTAs per SM (shared memory bound)
+// Output tile TX x TY, NT threads, MINB resident CTAs per SM.  64 x 32 when the dye is refined
+// over the flow (103 KB of windows, 2 CTAs of 512 threads per SM, and 20 % / 10 % of recomputed
+// forward / backward halo texels instead of 28 % / 14 % at 32 x 32); 32 x 32 otherwise, where
+// the velocity window is as large as the dye windows; 32 x 8 for textures whose wide tiles
+// would leave SMs without work (dye_tile).
+template <int TX_, int TY_, int NT_, int MINB_> struct DyeGeom {
+  static constexpr int TX = TX_, TY = TY_, THREADS = NT_, MINB = MINB_;
   static constexpr int H = kDyeLo + kDyeHi;
   static constexpr int W1X = TX + H, W1Y = TY + H;           // backward-pass region
   static constexpr int W2X = TX + 2 * H, W2Y = TY + 2 * H;   // forward-pass region
@@ -256,23 +258,11 @@ template <int TX> struct DyeGeom {
            sizeof(float2) * (W2X * W2Y + TX * TY + vel_x(n, m) * vel_y(n, m));
   }
 };
-// the wide tile for dye grids at least 2x the velocity grid and 64 texels wide
-inline bool dye_wide_tile(int n, int m) { return m >= 64 && m >= 2 * n; }
-
-// 8-byte asynchronous global -> shared copy (no register staging) and its wait
-__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
-               "l"(src)
-               : "memory");
-}
-// 16-byte variant (both addresses 16-byte aligned)
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
-               "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+using DyeWide = DyeGeom<64, 32, 512, 2>;
+using DyeSquare = DyeGeom<32, 32, 256, 3>;
+using DyeSmall = DyeGeom<32, 8, 256, 4>;
+// 0: wide, 1: square, 2: small
+inline int dye_tile(int n, int m) { return m <= 256 ? 2 : m >= 2 * n ? 0 : 1; }
 
 struct Rgb {
   float r, g, b;
@@ -526,7 +516,7 @@ __device__ __forceinline__ uint2 correct_rgb(const Rgb& a, const Rgb& b, const R
 }
 
 // Windows, origins and constants of one CTA of the fused dye kernel.
-template <int TX> struct DyeCta {
+template <class G> struct DyeCta {
   const float2* vel;
   const uint2* src;
   uint2* dst;
@@ -536,6 +526,7 @@ template <int TX> struct DyeCta {
   int n, m, tx0, ty0;
   int sx0, sy0, fx0, fy0, bx0, by0;   // wrapped origins of the source / forward / backward windows
   int vxw, vyw, vwx, vwy;             // velocity window: wrapped origin and extent
+  int vx0, vy0;                       // its origin before wrapping
   float h, fade;
 };
 
@@ -543,10 +534,9 @@ template <int TX> struct DyeCta {
 // moves less than one texel (checked on the velocity window the traces read), so every
 // footprint lies inside its window and the lookups skip the bounds tests and the
 // recomputation from global memory; the arithmetic, and so the bits, are the same.
-template <int TX, bool FAST>
-__device__ __forceinline__ void dye_cta_passes(const DyeCta<TX>& c) {
-  using G = DyeGeom<TX>;
-  constexpr int TY = G::TY, NT = G::THREADS;
+template <class G, bool FAST>
+__device__ __forceinline__ void dye_cta_passes(const DyeCta<G>& c) {
+  constexpr int TX = G::TX, TY = G::TY, NT = G::THREADS;
   constexpr int W1X = G::W1X, W1Y = G::W1Y, W2X = G::W2X, W2Y = G::W2Y, W3X = G::W3X, W3Y = G::W3Y;
   const int tid = threadIdx.x;
   const int n = c.n, m = c.m;
@@ -626,17 +616,139 @@ __device__ __forceinline__ void dye_cta_passes(const DyeCta<TX>& c) {
     c.dst[(size_t)y * m + x] = correct_rgb(a, b, lo, hi, [&] { return texel_pos(x, y, inv_m); }, c.fade, c.S);
   }
 }
+// ---- tiles whose region lies inside the texture, every trace under one texel
+// No position of the tile wraps: p - d + 1 lies in [1, 2), so its fract is x - 1, and cells and
+// texels are window-relative without masks.  floor(g) comes from g + 1.5 2^23 rounded down (the
+// sum's last place is 1), both coordinates in one packed add, and its bits are the index; the
+// three conversions it replaces ran on the quarter-rate pipe.  Every operation rounds as the
+// general form's, so the texels are the same bits.
+constexpr float kFloorMagic = 12582912.f;              // 1.5 * 2^23
+constexpr unsigned kFloorBits = 0x4B400000u;           // its bits
+struct InFoot {
+  float2 f;        // weights
+  unsigned ix, iy; // floor + kFloorBits
+};
+__device__ __forceinline__ InFoot in_foot(float2 p, float scale) {
+  const float2 g = __ffma2_rn(p, make_float2(scale, scale), make_float2(-0.5f, -0.5f));   // p * scale exact
+  const float2 t = __fadd2_rd(g, make_float2(kFloorMagic, kFloorMagic));
+  const float2 b = __fadd2_rn(t, make_float2(-kFloorMagic, -kFloorMagic));
+  return {__ffma2_rn(b, make_float2(-1.f, -1.f), g), __float_as_uint(t.x), __float_as_uint(t.y)};
+}
+// an FP32 or binary16 window: row length w, and the offset that takes in_foot's bits to slots
+template <class T> struct InWin {
+  const T* sm;
+  unsigned w, off;
+  __device__ __forceinline__ InWin(const T* s, int w_, int ox, int oy)
+      : sm(s), w((unsigned)w_), off(0u - (kFloorBits + (unsigned)oy) * (unsigned)w_ - kFloorBits - (unsigned)ox) {}
+  __device__ __forceinline__ const T* at(const InFoot& f) const { return sm + (int)(f.iy * w + f.ix + off); }
+};
+__device__ __forceinline__ float2 in_shift(float2 p, float2 v, float s) {   // fract_shift2
+  const float2 d = __ffma2_rn(v, make_float2(-s, -s), make_float2(0.f, 0.f));
+  return __fadd2_rn(__fadd2_rn(__fadd2_rn(p, d), make_float2(1.f, 1.f)), make_float2(-1.f, -1.f));
+}
+__device__ __forceinline__ float2 in_vel(const InWin<float2>& v, float2 p, float nf) {
+  const InFoot f = in_foot(p, nf);
+  const float2* q = v.at(f);
+  return lerp2v(lerp2v(q[0], q[1], f.f.x), lerp2v(q[v.w], q[v.w + 1], f.f.x), f.f.y);
+}
+// r, g, b of a sample: r, g packed, and the two rows' b packed for the lerp in x
+__device__ __forceinline__ Rgb in_sample(const InWin<uint2>& t, float2 p, float mf) {
+  const InFoot f = in_foot(p, mf);
+  const uint2* q = t.at(f);
+  const Rgb c00 = rgb_of(q[0]), c10 = rgb_of(q[1]), c01 = rgb_of(q[t.w]), c11 = rgb_of(q[t.w + 1]);
+  const float2 rg = lerp2v(lerp2v(make_float2(c00.r, c00.g), make_float2(c10.r, c10.g), f.f.x),
+                           lerp2v(make_float2(c01.r, c01.g), make_float2(c11.r, c11.g), f.f.x), f.f.y);
+  const float2 b = lerp2v(make_float2(c00.b, c01.b), make_float2(c10.b, c11.b), f.f.x);
+  return {rg.x, rg.y, lerp1(b.x, b.y, f.f.y)};
+}
+__device__ __forceinline__ float min4(float a, float b, float c, float d) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(fminf(a, b)), "f"(c), "f"(d));
+  return r;
+}
+__device__ __forceinline__ float max4(float a, float b, float c, float d) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(fmaxf(a, b)), "f"(c), "f"(d));
+  return r;
+}
+
+template <class G> __device__ __forceinline__ void dye_cta_passes_interior(const DyeCta<G>& c) {
+  constexpr int TX = G::TX, TY = G::TY, NT = G::THREADS;
+  constexpr int W1X = G::W1X, W1Y = G::W1Y, W2X = G::W2X, W2Y = G::W2Y, W3X = G::W3X;
+  const int tid = threadIdx.x;
+  const int m = c.m;
+  const float h = c.h, hh = 0.5f * h, nf = (float)c.n, mf = (float)m;
+  const float inv_m = __frcp_rn(mf);
+  // window origins, not wrapped (the velocity window may start below cell 0: its slots hold
+  // the wrapped cells in order)
+  const int vx0 = c.vx0, vy0 = c.vy0;
+  const InWin<float2> V(c.s_vel, c.vwx, vx0, vy0);
+  const InWin<uint2> T(c.s_src, W3X, c.tx0 - 3 * kDyeLo - 1, c.ty0 - 3 * kDyeLo);
+  const InWin<uint2> F(c.s_fwd, W2X, c.tx0 - 2 * kDyeLo, c.ty0 - 2 * kDyeLo);
+  const InWin<uint2> B(c.s_back, W1X, c.tx0 - kDyeLo, c.ty0 - kDyeLo);
+  // centre of region texel (rx, ry): (2^22 + r) / m + (origin + 1/2 - 2^22) / m, all exact; the
+  // first factor's bits are 2 r + those of 2^22
+  auto centre = [&](int rx, int ry, float2 org) {
+    const float2 r = make_float2(__uint_as_float(0x4A800000u + 2u * (unsigned)rx), __uint_as_float(0x4A800000u + 2u * (unsigned)ry));
+    return __ffma2_rn(r, make_float2(inv_m, inv_m), org);
+  };
+  auto origin = [&](int ox, int oy) {
+    return make_float2(((float)ox + 0.5f - 4194304.f) * inv_m, ((float)oy + 0.5f - 4194304.f) * inv_m);
+  };
+  const float2 fo = origin(c.tx0 - 2 * kDyeLo, c.ty0 - 2 * kDyeLo), bo = origin(c.tx0 - kDyeLo, c.ty0 - kDyeLo);
+
+  for (int i = tid; i < W2X * W2Y; i += NT) {
+    const int ry = i / W2X, rx = i - ry * W2X;
+    const float2 p = centre(rx, ry, fo);
+    const float2 v1 = in_vel(V, p, nf);
+    c.s_v1[i] = v1;
+    const float2 sp = in_shift(p, in_vel(V, in_shift(p, v1, hh), nf), h);
+    const int ix = rx - 2 * kDyeLo, iy = ry - 2 * kDyeLo;
+    if ((unsigned)ix < (unsigned)TX && (unsigned)iy < (unsigned)TY) c.s_sp[iy * TX + ix] = sp;
+    c.s_fwd[i] = pack_rgb(in_sample(T, sp, mf));
+  }
+  __syncthreads();
+  for (int i = tid; i < W1X * W1Y; i += NT) {
+    const int ry = i / W1X, rx = i - ry * W1X;
+    const float2 p = centre(rx, ry, bo);
+    const float2 v1 = c.s_v1[(ry + kDyeLo) * W2X + rx + kDyeLo];
+    c.s_back[i] = pack_rgb(in_sample(F, in_shift(p, in_vel(V, in_shift(p, v1, -hh), nf), -h), mf));
+  }
+  __syncthreads();
+  for (int i = tid; i < TX * TY; i += NT) {
+    const int ry = i / TX, rx = i - ry * TX;
+    const InFoot f = in_foot(c.s_sp[i], mf);
+    const uint2 *pa = T.at(f), *pb = B.at(f);
+    const Rgb a00 = rgb_of(pa[0]), a10 = rgb_of(pa[1]), a01 = rgb_of(pa[T.w]), a11 = rgb_of(pa[T.w + 1]);
+    const Rgb b00 = rgb_of(pb[0]), b10 = rgb_of(pb[1]), b01 = rgb_of(pb[B.w]), b11 = rgb_of(pb[B.w + 1]);
+    const float2 arg = lerp2v(lerp2v(make_float2(a00.r, a00.g), make_float2(a10.r, a10.g), f.f.x),
+                              lerp2v(make_float2(a01.r, a01.g), make_float2(a11.r, a11.g), f.f.x), f.f.y);
+    const float2 brg = lerp2v(lerp2v(make_float2(b00.r, b00.g), make_float2(b10.r, b10.g), f.f.x),
+                              lerp2v(make_float2(b01.r, b01.g), make_float2(b11.r, b11.g), f.f.x), f.f.y);
+    const float2 bb = lerp2v(lerp2v(make_float2(a00.b, b00.b), make_float2(a10.b, b10.b), f.f.x),
+                             lerp2v(make_float2(a01.b, b01.b), make_float2(a11.b, b11.b), f.f.x), f.f.y);
+    // 1.5 a - 0.5 b (0.5 b exact, so one multiply-add rounds as the difference), limited, faded
+    const float2 rg = __ffma2_rn(brg, make_float2(-0.5f, -0.5f), __fmul2_rn(arg, make_float2(1.5f, 1.5f)));
+    const float bl = __fmaf_rn(bb.y, -0.5f, __fmul_rn(bb.x, 1.5f));
+    const float r = fminf(fmaxf(rg.x, min4(a00.r, a10.r, a01.r, a11.r)), max4(a00.r, a10.r, a01.r, a11.r));
+    const float g = fminf(fmaxf(rg.y, min4(a00.g, a10.g, a01.g, a11.g)), max4(a00.g, a10.g, a01.g, a11.g));
+    const float b = fminf(fmaxf(bl, min4(a00.b, a10.b, a01.b, a11.b)), max4(a00.b, a10.b, a01.b, a11.b));
+    const float2 rgf = __fmul2_rn(make_float2(r, g), make_float2(c.fade, c.fade));
+    const int x = c.tx0 + rx, y = c.ty0 + ry;
+    c.dst[(size_t)y * m + x] =
+        splat_texel(rgf.x, rgf.y, __fmul_rn(b, c.fade), [&] { return texel_pos(x, y, inv_m); }, c.S);
+  }
+}
 // the context of this CTA from the kernel arguments
-template <int TX>
-__device__ __forceinline__ DyeCta<TX> dye_cta_setup(const float2* __restrict__ vel, const uint2* __restrict__ src,
+template <class G>
+__device__ __forceinline__ DyeCta<G> dye_cta_setup(const float2* __restrict__ vel, const uint2* __restrict__ src,
                                                     uint2* __restrict__ dst, const float* __restrict__ dtbuf,
                                                     const DevParams* __restrict__ params,
                                                     const DevSplats* __restrict__ S, int n, int m) {
-  using G = DyeGeom<TX>;
-  constexpr int TY = G::TY;
+  constexpr int TX = G::TX, TY = G::TY;
   constexpr int W1X = G::W1X, W1Y = G::W1Y, W2X = G::W2X, W2Y = G::W2Y, W3X = G::W3X, W3Y = G::W3Y;
   extern __shared__ __align__(16) uint2 dsm2[];
-  DyeCta<TX> c;
+  DyeCta<G> c;
   c.vel = vel;
   c.src = src;
   c.dst = dst;
@@ -664,6 +776,8 @@ __device__ __forceinline__ DyeCta<TX> dye_cta_setup(const float2* __restrict__ v
   c.by0 = (c.ty0 - kDyeLo) & (m - 1);
   const int vx0 = (int)floorf(((float)(c.tx0 - 2 * kDyeLo - 1) + 0.5f) * (float)n / (float)m - 0.5f) - 1;
   const int vy0 = (int)floorf(((float)(c.ty0 - 2 * kDyeLo - 1) + 0.5f) * (float)n / (float)m - 0.5f) - 1;
+  c.vx0 = vx0;
+  c.vy0 = vy0;
   c.vxw = vx0 & (n - 1);
   c.vyw = vy0 & (n - 1);
   return c;
@@ -672,21 +786,20 @@ __device__ __forceinline__ DyeCta<TX> dye_cta_setup(const float2* __restrict__ v
 // the general passes kept out of line, from the kernel arguments: the rarely taken path
 // with its recomputation chains neither sets the register budget of the fast path nor
 // makes it keep its context in memory
-template <int TX>
+template <class G>
 __device__ __noinline__ void dye_cta_passes_general(const float2* vel, const uint2* src, uint2* dst,
                                                     const float* dtbuf, const DevParams* params,
                                                     const DevSplats* S, int n, int m) {
-  dye_cta_passes<TX, false>(dye_cta_setup<TX>(vel, src, dst, dtbuf, params, S, n, m));
+  dye_cta_passes<G, false>(dye_cta_setup<G>(vel, src, dst, dtbuf, params, S, n, m));
 }
 
-template <int TX>
-__global__ void __launch_bounds__(DyeGeom<TX>::THREADS, DyeGeom<TX>::MINB)
+template <class G>
+__global__ void __launch_bounds__(G::THREADS, G::MINB)
     k_dye_fused(const float2* __restrict__ vel, const uint2* __restrict__ src, uint2* __restrict__ dst,
                 const float* __restrict__ dtbuf, const DevParams* __restrict__ params,
                 const DevSplats* __restrict__ S, int n, int m) {
-  using G = DyeGeom<TX>;
   constexpr int NT = G::THREADS, W3X = G::W3X, W3Y = G::W3Y;
-  const DyeCta<TX> c = dye_cta_setup<TX>(vel, src, dst, dtbuf, params, S, n, m);
+  const DyeCta<G> c = dye_cta_setup<G>(vel, src, dst, dtbuf, params, S, n, m);
   const int tid = threadIdx.x;
 
   // the source window arrives asynchronously while the velocity window loads: one
@@ -713,8 +826,10 @@ __global__ void __launch_bounds__(DyeGeom<TX>::THREADS, DyeGeom<TX>::MINB)
   }
   // this thread's source copies have landed; the barrier below makes every thread's visible
   cp_async_wait_all();
-  if (__syncthreads_or(far ? 1 : 0)) dye_cta_passes_general<TX>(vel, src, dst, dtbuf, params, S, n, m);
-  else dye_cta_passes<TX, true>(c);
+  if (__syncthreads_or(far ? 1 : 0)) dye_cta_passes_general<G>(vel, src, dst, dtbuf, params, S, n, m);
+  else if (blockIdx.x > 0 && blockIdx.y > 0 && blockIdx.x + 1 < gridDim.x && blockIdx.y + 1 < gridDim.y)
+    dye_cta_passes_interior<G>(c);
+  else dye_cta_passes<G, true>(c);
 }
 
 }  // namespace s2d

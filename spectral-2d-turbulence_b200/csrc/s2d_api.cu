@@ -16,7 +16,9 @@
 
 #include "../../include/s2d.h"
 #include "s2d_aux_kernels.cuh"
+#include "s2d_host_checks.h"
 #include "s2d_ops.cuh"
+#include "s2d_readback.h"
 #include "s2d_tc.cuh"
 #include "s2d_tc_cols.cuh"
 #include "s2d_tc_lines.h"
@@ -292,6 +294,7 @@ struct ProfScope {
 static int seed_parts_count(int n) { return (n * n + 255) / 256; }
 
 static void free_solver(s2d_solver* s) {
+  readback_release(s->dev);
   if (s->diag_stream) cudaStreamSynchronize(s->diag_stream);   // its copies read device memory
   for (auto& kv : s->graphs) {
     if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
@@ -651,6 +654,7 @@ extern "C" int s2d_create(int n, int dye_scale, int fft_precision, int device, s
   if (int rc = check_device(device)) return rc;
   DeviceGuard guard(device);
   s2d_solver* s = new s2d_solver();
+  readback_retain(device);
   s->dev = device;
   s->n = n;
   s->m = n * dye_scale;
@@ -1452,6 +1456,7 @@ extern "C" int s2d_seed_band(s2d_solver* s, float kmin, float kmax, float rms, u
 }
 
 static int check_finite(const float* v, size_t count) {
+  if (all_finite(v, count)) return S2D_OK;
   for (size_t i = 0; i < count; ++i)
     if (!std::isfinite(v[i])) return fail(S2D_ERR_NAN, "non-finite value at index " + std::to_string(i));
   return S2D_OK;
@@ -1761,7 +1766,7 @@ extern "C" int s2d_get_buffer(s2d_solver* s, int id, void* host, size_t bytes) {
     return S2D_OK;
   }
   if (bytes > sz) return fail(S2D_ERR_ARG, "requested more bytes than the buffer holds");
-  S2D_CUDA(cudaMemcpyAsync(host, p, bytes, cudaMemcpyDeviceToHost, s->stream));
+  S2D_CUDA(read_back(s->dev, host, p, bytes, s->stream));
   return check_device_error(s);
 }
 
@@ -1856,9 +1861,7 @@ extern "C" int s2d_get_dye(s2d_solver* s, uint16_t* out) {
   S2D_USE(s);
   if (!out) return fail(S2D_ERR_ARG, "out is null");
   DeviceGuard guard(s->dev);
-  S2D_CUDA(cudaMemcpyAsync(out, s->dye[s->dye_parity], (size_t)s->m * s->m * sizeof(ushort4),
-                           cudaMemcpyDeviceToHost, s->stream));
-  S2D_CUDA(cudaStreamSynchronize(s->stream));
+  S2D_CUDA(read_back(s->dev, out, s->dye[s->dye_parity], (size_t)s->m * s->m * sizeof(ushort4), s->stream));
   return S2D_OK;
 }
 

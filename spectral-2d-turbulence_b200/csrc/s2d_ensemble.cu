@@ -18,8 +18,10 @@
 
 #include "../../include/s2d.h"
 #include "s2d_band.cuh"
+#include "s2d_host_checks.h"
 #include "s2d_kernels.cuh"
 #include "s2d_pairs.cuh"
+#include "s2d_readback.h"
 
 using namespace s2d;
 
@@ -429,6 +431,7 @@ static void ens_set_banded(s2d_ensemble* e, bool banded) {
 }
 
 static void ens_free(s2d_ensemble* e) {
+  readback_release(e->dev);
   ens_drop_graphs(e);
   void* ptrs[] = {e->dinst, e->dseeds, e->items, e->ptw, e->pool.s[0], e->pool.s[1], e->pool.s[2],
                   e->pool.pa, e->pool.pb, e->pool.z, e->pool.row_nz, e->tw, e->sums, e->err};
@@ -457,6 +460,7 @@ extern "C" int s2d_ensemble_create(const s2d_instance_desc* descs, int count, in
   cudaGetDevice(&prev);
   cudaSetDevice(device);
   s2d_ensemble* e = new s2d_ensemble();
+  readback_retain(device);
   e->dev = device;
   e->count = count;
   auto bail = [&](cudaError_t err, const char* what) {
@@ -631,8 +635,7 @@ extern "C" int s2d_ensemble_set_state(s2d_ensemble* e, int index, const float* s
   if (index < 0 || index >= e->count || !spectrum) return efail(S2D_ERR_ARG, "bad instance index");
   const EnsInst& I = e->hinst[index];
   const size_t bytes = sizeof(float2) * (size_t)I.n * I.n;
-  for (size_t i = 0; i < bytes / sizeof(float); ++i)
-    if (!std::isfinite(spectrum[i])) return efail(S2D_ERR_NAN, "non-finite value in spectrum");
+  if (!all_finite(spectrum, bytes / sizeof(float))) return efail(S2D_ERR_NAN, "non-finite value in spectrum");
   E_CUDA(cudaMemcpyAsync(e->pool.s[e->phase] + I.off, spectrum, bytes, cudaMemcpyHostToDevice, e->stream));
   E_CUDA(cudaStreamSynchronize(e->stream));
   e->packs_valid = false;
@@ -644,9 +647,13 @@ extern "C" int s2d_ensemble_get_state(s2d_ensemble* e, int index, float* spectru
   E_USE(e);
   if (index < 0 || index >= e->count || !spectrum) return efail(S2D_ERR_ARG, "bad instance index");
   const EnsInst& I = e->hinst[index];
-  E_CUDA(cudaMemcpyAsync(spectrum, e->pool.s[e->phase] + I.off, sizeof(float2) * (size_t)I.n * I.n,
-                         cudaMemcpyDeviceToHost, e->stream));
-  E_CUDA(cudaStreamSynchronize(e->stream));
+  int prev = 0;
+  cudaGetDevice(&prev);
+  if (prev != e->dev) cudaSetDevice(e->dev);
+  const cudaError_t err =
+      read_back(e->dev, spectrum, e->pool.s[e->phase] + I.off, sizeof(float2) * (size_t)I.n * I.n, e->stream);
+  if (prev != e->dev) cudaSetDevice(prev);
+  E_CUDA(err);
   return ens_check_err(e);
 }
 

@@ -639,19 +639,4 @@ static __global__ void k_unblock_pack(float2* out, const float2* __restrict__ tm
   out[i] = tmp[((size_t)(c >> 2) * n + r) * 4 + (c & 3)];
 }
 
-// whether a (prefix of a) complex n x n spectrum is zero outside the dealias band
-inline bool band_limited(const float* w, size_t count, int n) {
-  auto any = [&](size_t lo, size_t hi) {
-    bool some = false;
-    for (size_t i = lo, e = hi < count ? hi : count; i < e; ++i) some |= w[i] != 0.f;
-    return some;
-  };
-  for (int r = 0; r < n; ++r) {
-    const size_t row = (size_t)2 * n * r;
-    const bool in = r <= n / 3 || r >= n - n / 3;
-    if (any(row + (in ? 2 * (size_t)(n / 3 + 1) : 0), row + (in ? 2 * (size_t)(n - n / 3) : 2 * (size_t)n))) return false;
-  }
-  return true;
-}
-
 }  // namespace s2d

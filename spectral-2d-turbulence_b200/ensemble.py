@@ -57,7 +57,7 @@ class Ensemble:
 
     def getState(self, index: int) -> np.ndarray:
         n = self.instances[index]["n"]
-        out = np.zeros((n, n), np.complex64)
+        out = np.empty((n, n), np.complex64)
         L.call("s2d_ensemble_get_state", self._h, int(index), out.ctypes.data_as(C.POINTER(C.c_float)))
         return out
 

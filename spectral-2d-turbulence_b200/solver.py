@@ -399,7 +399,7 @@ class Solver:
     @property
     def currentDye(self) -> np.ndarray:
         """solver.js:610-612: the current dye texture as binary16 bits [m, m, 4]."""
-        out = np.zeros((self.m, self.m, 4), np.uint16)
+        out = np.empty((self.m, self.m, 4), np.uint16)
         L.call("s2d_get_dye", self._use(), out.ctypes.data_as(C.POINTER(C.c_uint16)))
         return out
 
@@ -414,7 +414,7 @@ class Solver:
             out = np.zeros(4, np.float32)
             L.call("s2d_get_buffer", self._use(), bid, out.ctypes.data, out.nbytes)
             return out
-        out = np.zeros((self.n, self.n), np.complex64)
+        out = np.empty((self.n, self.n), np.complex64)
         L.call("s2d_get_buffer", self._use(), bid, out.ctypes.data, out.nbytes)
         return out
 

@@ -1,0 +1,85 @@
+"""Fields read into pageable memory: direct, staged by one thread and by several; odd lengths;
+destinations that are not pageable; several host threads at once; staging made, given back with
+the last object and made again."""
+import ctypes as C
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _spectrum(n, seed):
+    rng = np.random.default_rng(seed)
+    return (rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))).astype(np.complex64)
+
+
+def _read(pkg, s, out, count):
+    lib = pkg.lib()
+    p = C.c_void_p(out.ctypes.data)
+    assert lib.s2d_get_buffer(s._h, 0, p, count) == 0
+
+
+@pytest.mark.parametrize("n", [64, 128, 256, 512, 1024, 2048])
+def test_fields_come_back_whole(pkg, n):
+    w = _spectrum(n, n)
+    s = pkg.Solver.create(n=n, dyeScale=1)
+    try:
+        s.setBuffer("state0", w)
+        assert np.array_equal(s.getBuffer("state0"), w)
+        bits = np.random.default_rng(1).integers(0, 2 ** 16, (n, n, 4), dtype=np.uint16)
+        s.setDye(bits)
+        assert np.array_equal(s.currentDye, bits)
+        flat = w.reshape(-1).view(np.uint8)
+        for count in {8, flat.size // 2 + 8, flat.size - 8, max(8, flat.size // 3 // 8 * 8)}:
+            out = np.full(flat.size + 16, 0xA5, np.uint8)[3:]      # unaligned, with a guard behind
+            _read(pkg, s, out, count)
+            assert np.array_equal(out[:count], flat[:count]) and np.all(out[count:] == 0xA5)
+    finally:
+        s.destroy()
+
+
+def test_pinned_destination(pkg):
+    import torch
+    n = 512
+    w = _spectrum(n, 2)
+    s = pkg.Solver.create(n=n, dyeScale=1)
+    try:
+        s.setBuffer("state0", w)
+        out = torch.empty(w.nbytes, dtype=torch.uint8, pin_memory=True).numpy()
+        _read(pkg, s, out, w.nbytes)
+        assert np.array_equal(out, w.reshape(-1).view(np.uint8))
+    finally:
+        s.destroy()
+
+
+def test_ensemble_and_solvers_from_several_threads(pkg):
+    fails = []
+
+    def work(k):
+        try:
+            for r in range(3):
+                n = (256, 512, 1024)[(k + r) % 3]
+                w = _spectrum(n, 10 * k + r)
+                if k % 2:
+                    e = pkg.Ensemble([{"n": n, "dt": 1e-3}])
+                    e.setState(0, w)
+                    got = [e.getState(0) for _ in range(4)]
+                    e.destroy()
+                else:
+                    s = pkg.Solver.create(n=n, dyeScale=1)
+                    s.setBuffer("state0", w)
+                    got = [s.getBuffer("state0") for _ in range(4)]
+                    s.destroy()
+                if not all(np.array_equal(g, w) for g in got):
+                    fails.append((k, r))
+        except Exception as ex:          # reported by the assert below
+            fails.append(repr(ex))
+
+    team = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in team:
+        t.start()
+    for t in team:
+        t.join()
+    assert not fails

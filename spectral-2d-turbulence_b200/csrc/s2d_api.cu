@@ -192,6 +192,8 @@ struct s2d_solver {
   // store other states, which the pair kernels do not take
   bool banded = true;
   float4* ptw = nullptr;              // pass-ordered twiddles of the pair kernels
+  // the whole step in one launch (small grids), or null
+  void (*step_run)(const PhysArgs&, const SpecArgs&, float2* const (&)[3], cudaStream_t) = nullptr;
   uchar4* image = nullptr;            // headless render target, grown on demand
   size_t image_px = 0;
   ushort4* dye[3] = {nullptr, nullptr, nullptr};
@@ -622,12 +624,16 @@ static void mark_packs(s2d_solver* s) {
   s->packs_pairs = pair_rows(s);
   s->packs_half = s->packs_pairs && pair_cols(s);
 }
+// what the pair row kernel takes beside the row stage's arguments
+static void pair_row_args(s2d_solver* s, SpecArgs* a) {
+  a->ptw = s->ptw + s->ops->ptw_rows;
+  a->top = pair_cols(s) ? s->ticket + 1 : nullptr;
+  a->dt_out = dt_slot(s, s->slot ^ 1);
+  a->full_pb = pair_cols(s) ? 0 : 1;
+}
 // the row stage with the solver's chosen variant
 static void run_spec(s2d_solver* s, int mode, bool ptr, SpecArgs a) {
-  a.ptw = s->ptw + s->ops->ptw_rows;
-  a.top = pair_cols(s) ? s->ticket + 1 : nullptr;
-  a.dt_out = dt_slot(s, s->slot ^ 1);
-  a.full_pb = pair_cols(s) ? 0 : 1;
+  pair_row_args(s, &a);
   if (tc_rows(s)) {
     if (s->fft_precision == S2D_FFT_TC_BF16) tc_rows_launch<tc::PrecBF16>(mode, ptr, a, s->tctab, s->stream);
     else tc_rows_launch<tc::PrecF16>(mode, ptr, a, s->tctab, s->stream);
@@ -714,6 +720,7 @@ extern "C" int s2d_create(int n, int dye_scale, int fft_precision, int device, s
   TRY(cudaMallocHost(&s->h_upload, kUploadSlotBytes * kUploadSlots), "pinned upload ring");
   for (cudaEvent_t& ev : s->upload_ev) TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "event");
   TRY(set_all_attrs(*ops), "kernel attributes");
+  if (fft_precision == S2D_FFT_FP32) TRY(ops->step_attrs(&s->step_run), "kernel attributes");
   switch (dye_tile(n, s->m)) {
     case 0: TRY(set_smem(k_dye_fused<DyeWide>, DyeWide::smem(n, s->m)), "dye kernel attributes"); break;
     case 1: TRY(set_smem(k_dye_fused<DyeSquare>, DyeSquare::smem(n, s->m)), "dye kernel attributes"); break;
@@ -1094,19 +1101,16 @@ extern "C" int s2d_encode_step(s2d_solver* s) {
     return enqueue_unfused_step(s, ptr);
   }
   const int p = s->phase;
-  for (int st = 0; st < 3; ++st) {
-    {
-      ProfScope ps(s, S2D_PROF_PHYS_COLS);
-      PhysArgs pa = phys_args(s, st == 2 ? 1 : 0);
-      if (st == 0 && s->latch_pending) {
-        pa.latch = s->dparams;
-        pa.counter = s->step_counter;
-        s->latch_pending = false;
-      }
-      enqueue_phys_cols(s, st == 2 ? 2 : 1, pa);
-      S2D_LAUNCHED();
+  auto cols_args = [&](int st) {
+    PhysArgs a = phys_args(s, st == 2 ? 1 : 0);
+    if (st == 0 && s->latch_pending) {
+      a.latch = s->dparams;
+      a.counter = s->step_counter;
+      s->latch_pending = false;
     }
-    ProfScope ps(s, S2D_PROF_SPEC_ROWS);
+    return a;
+  };
+  auto rows_args = [&](int st) {
     SpecArgs a{};
     a.z = s->physZ;
     a.w0 = s->state[p];
@@ -1121,8 +1125,26 @@ extern "C" int s2d_encode_step(s2d_solver* s) {
     a.stochastic = s->hp.force_amp > 0.f ? 1 : 0;
     a.err = s->err;
     a.row_nz = s->row_nz;
-    run_spec(s, st, ptr, a);
+    return a;
+  };
+  if (s->step_run && pair_cols(s) && !s->profiling) {
+    // one launch (profiling times the stages apart)
+    SpecArgs b = rows_args(0);
+    pair_row_args(s, &b);
+    float2* const ring[3] = {s->state[p], s->state[(p + 1) % 3], s->state[(p + 2) % 3]};
+    s->step_run(cols_args(0), b, ring, s->stream);
     S2D_LAUNCHED();
+  } else {
+    for (int st = 0; st < 3; ++st) {
+      {
+        ProfScope ps(s, S2D_PROF_PHYS_COLS);
+        enqueue_phys_cols(s, st == 2 ? 2 : 1, cols_args(st));
+        S2D_LAUNCHED();
+      }
+      ProfScope ps(s, S2D_PROF_SPEC_ROWS);
+      run_spec(s, st, ptr, rows_args(st));
+      S2D_LAUNCHED();
+    }
   }
   s->reduced_valid = true;
   mark_packs(s);

@@ -6,6 +6,7 @@
 // and row variants.
 #pragma once
 #include <cuda_runtime.h>
+#include <type_traits>
 #include "s2d_kernels.cuh"
 #include "s2d_pairs.cuh"
 
@@ -44,6 +45,8 @@ struct NOps {
   void (*fft_cols)(int sign, float2* data, const float2* tw, cudaStream_t st);
   // pass-ordered twiddles of the pair kernels: entries, and where the rows' table starts
   int ptw_size, ptw_rows;
+  // the whole step in one launch, where the size has it (PairImpl::step_attrs)
+  cudaError_t (*step_attrs)(void (**)(const PhysArgs&, const SpecArgs&, float2* const (&)[3], cudaStream_t));
   bool blocked_packs;   // the pair kernels keep the packs in blocks of four columns
   void (*make_ptw)(float4* out, const float2* tw, cudaStream_t st);
   int n_phys = 0, n_spec = 0;
@@ -131,6 +134,48 @@ template <int N> struct PairImpl {
   }
   static PhysVariant phys() { return PhysVariant{"column pairs", &phys_attrs, &phys_run, true}; }
   static SpecVariant spec() { return SpecVariant{"row pairs", &spec_attrs, &spec_run, true}; }
+  // the whole step as one cluster (small grids): nullptr where the stages are launched apart or
+  // the device cannot hold the cluster
+  using S = typename PairStepShape<N>::S;
+  using StepFn = void (*)(const PhysArgs&, const SpecArgs&, float2* const (&)[3], cudaStream_t);
+  static cudaLaunchConfig_t step_config(cudaLaunchAttribute (&attr)[2], cudaStream_t st) {
+    cudaLaunchConfig_t cfg{};
+    if constexpr (!std::is_void<S>::value) {
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim = {S::CTAS, 1, 1};
+      attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[1].val.programmaticStreamSerializationAllowed = 1;
+      cfg.gridDim = dim3(S::CTAS);
+      cfg.blockDim = dim3(S::THREADS);
+      cfg.dynamicSmemBytes = S::SMEM;
+      cfg.stream = st;
+      cfg.attrs = attr;
+      cfg.numAttrs = 2;
+    }
+    return cfg;
+  }
+  static void step_run(const PhysArgs& a, const SpecArgs& b, float2* const (&s)[3], cudaStream_t st) {
+    if constexpr (!std::is_void<S>::value) {
+      cudaLaunchAttribute attr[2]{};
+      const cudaLaunchConfig_t cfg = step_config(attr, st);
+      cudaLaunchKernelEx(&cfg, k_pair_step<S>, a, b, s[0], s[1], s[2]);
+    }
+  }
+  static cudaError_t step_attrs(StepFn* fn) {
+    *fn = nullptr;
+    if constexpr (!std::is_void<S>::value) {
+      cudaError_t e = set_smem(k_pair_step<S>, S::SMEM);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k_pair_step<S>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      if (e != cudaSuccess) return e;
+      cudaLaunchAttribute attr[2]{};
+      cudaLaunchConfig_t cfg = step_config(attr, nullptr);
+      cfg.numAttrs = 1;
+      int fit = 0;
+      if (cudaOccupancyMaxActiveClusters(&fit, k_pair_step<S>, &cfg) == cudaSuccess && fit > 0) *fn = &step_run;
+      cudaGetLastError();
+    }
+    return cudaSuccess;
+  }
   // pass-ordered twiddles: the columns' table, then the rows'
   static constexpr int CTW = PassTw<N, C::V>::SIZE, RTW = PassTw<N, R::V>::SIZE;
   static void make_ptw(float4* out, const float2* tw, cudaStream_t st) {
@@ -182,6 +227,7 @@ template <int N> struct OpsImpl {
     o.ptw_rows = PT::CTW;
     o.make_ptw = &PT::make_ptw;
     o.blocked_packs = PT::C::BP;
+    o.step_attrs = &PT::step_attrs;
     o.phys[o.n_phys++] = PT::phys();
     o.spec[o.n_spec++] = PT::spec();
     o.phys[o.n_phys++] = PhysImpl<N, TU>::make("V=16");

@@ -173,6 +173,10 @@ template <> struct PairShape<512> { using C = PairCols<512, 8, 2, 4>; using R = 
 template <> struct PairShape<1024> { using C = PairCols<1024, 16, 4, 1>; using R = PairRows<1024, 8, 128, 3>; };
 template <> struct PairShape<2048> { using C = PairCols<2048, 16, 4, 1>; using R = PairRows<2048, 16, 128, 3>; };
 template <> struct PairShape<4096> { using C = PairCols<4096, 16, 2, 1, true>; using R = PairRows<4096, 16, 256, 2, true>; };
+template <int N> struct PairStepShape { using S = void; };
+template <> struct PairStepShape<32>;
+template <> struct PairStepShape<64>;
+template <> struct PairStepShape<128>;
 template <class TU> __device__ __forceinline__ bool pair_inband(int i) { return i <= TU::KMAX || i >= TU::N - TU::KMAX; }
 // whether register slot m (indices T m .. T m + T - 1) holds no in-band index
 template <class TU> __host__ __device__ constexpr bool slot_empty(int m) {
@@ -198,8 +202,8 @@ __device__ __forceinline__ void lines_fft(C2 (&x)[TU::V], float2 (&y)[TU::V], fl
   sfor<PL::P>([&](auto pc) {
     constexpr int p = decltype(pc)::value;
     constexpr int R = PL::radix(p), B = V / R, NS = PL::ns(p);
-    C2 v[V];
-    float2 w[V];
+    [[maybe_unused]] C2 v[V];
+    [[maybe_unused]] float2 w[V];
     if constexpr (p == 0) {
 #pragma unroll
       for (int b = 0; b < B; ++b)
@@ -305,7 +309,7 @@ __device__ __forceinline__ float pair_cols_tile(const PhysArgs& a, size_t base, 
       y[m] = make_float2(0.f, 0.f);
       if (!slot_empty<TU>(m) && pair_inband<TU>(row)) {
         const bool up = row < N / 2;
-        const float4 q = __ldg(reinterpret_cast<const float4*>(a.pb + at(up ? row : N - row)));
+        const float4 q = *reinterpret_cast<const float4*>(a.pb + at(up ? row : N - row));
         // V(x) + i V(x+1), conjugated spectra for -ky; row 0 is real
         if (row == 0) y[m] = make_float2(q.x, q.z);
         else y[m] = up ? make_float2(q.x - q.w, q.y + q.z) : make_float2(q.x + q.w, q.z - q.y);
@@ -616,6 +620,58 @@ __global__ void __launch_bounds__(TU::THREADS, TU::MINB) k_pair_rows(SpecArgs a,
   pair_rows_tile<TU, true>(a, 0, a.params, stage >= 0 ? __ldg(a.dt) : 0.f, a.stochastic != 0, a.ptw, stage, blockIdx.x,
                            smem4);
   if (stage == 2 && a.top && blockIdx.x == 0 && threadIdx.x == 0) pair_cfl(a);
+}
+
+// ------------------------------------------------------------------ a whole step in one launch
+// Up to 256^2 a stage kernel is launch and latency (3.4 us each at 64^2 for 0.3 us of work), so
+// one thread-block cluster runs the six passes: the packs and Z go through L2 as between
+// launches, and the cluster barrier orders them.
+template <class C_, class R_, int CTAS_> struct PairStep {
+  using C = C_;
+  using R = R_;
+  static constexpr int CTAS = CTAS_, THREADS = C::THREADS;
+  static constexpr size_t SMEM = C::SMEM > R::SMEM ? C::SMEM : R::SMEM;
+  static_assert(C::THREADS == R::THREADS && C::GRID % CTAS == 0, "one block shape");
+};
+template <> struct PairStepShape<32> { using S = PairStep<PairCols<32, 4, 16, 1>, PairRows<32, 4, 128, 1>, 1>; };
+template <> struct PairStepShape<64> { using S = PairStep<PairCols<64, 4, 4, 1>, PairRows<64, 4, 64, 1>, 8>; };
+template <> struct PairStepShape<128> { using S = PairStep<PairCols<128, 4, 4, 1>, PairRows<128, 4, 128, 1>, 16>; };
+template <int CTAS> __device__ __forceinline__ void cluster_barrier() {
+  if constexpr (CTAS == 1) {
+    __syncthreads();
+  } else {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+}
+template <class S>
+__global__ void __launch_bounds__(S::THREADS, 1) k_pair_step(PhysArgs pa, SpecArgs sa, float2* s0, float2* s1, float2* s2) {
+  using C = typename S::C;
+  using R = typename S::R;
+  extern __shared__ __align__(16) float4 smem4[];
+  pdl_wait();
+  phys_latch(pa);
+  const float dt = __ldg(sa.dt);
+  float speed = 0.f;
+#pragma unroll 1
+  for (int stage = 0; stage < 3; ++stage) {
+    for (int tile = blockIdx.x; tile < C::GRID; tile += S::CTAS) {
+      speed = fmaxf(speed, pair_cols_tile<C>(pa, 0, pa.ptw, stage == 2 ? 2 : 1, tile, smem4));
+      __syncthreads();
+    }
+    if (stage == 2) cols_speed_max<S::THREADS>(sa.top, speed);
+    cluster_barrier<S::CTAS>();
+    // the state ring of stage `stage` (k_pair_rows' arguments, launch by launch)
+    sa.w0 = s0;
+    sa.wcur = stage == 0 ? s0 : stage == 1 ? s1 : s2;
+    sa.wout = stage == 1 ? s2 : s1;
+    for (int tile = blockIdx.x; tile < R::GRID; tile += S::CTAS) {
+      pair_rows_tile<R>(sa, 0, sa.params, dt, sa.stochastic != 0, sa.ptw, stage, tile, smem4);
+      __syncthreads();
+    }
+    if (stage == 2 && blockIdx.x == 0 && threadIdx.x == 0) pair_cfl(sa);
+    if (stage < 2) cluster_barrier<S::CTAS>();
+  }
 }
 
 // the row flags of packs written by k_pair_rows: in-band rows

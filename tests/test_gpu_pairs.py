@@ -140,3 +140,21 @@ def test_ensemble_states(pkg, banded):
             assert banded or np.array_equal(a, b)
     finally:
         e.destroy()
+
+
+@pytest.mark.parametrize("n", [32, 64, 128])
+@pytest.mark.parametrize("splat", [False, True])
+def test_the_step_in_one_launch_matches_its_stages(pkg, n, splat):
+    """The small grids' one-launch step against the same step launched stage by stage (as the
+    profiler times it): state ring, velocity, dt and packs."""
+    outs = []
+    for apart in (False, True):
+        s = pkg.Solver.create(n=n, dyeScale=1)
+        try:
+            s.profile(apart)
+            outs.append(_stepped(s, n, (0, 0), steps=4, splat=splat))
+            outs[-1]["ring"] = np.stack([s.getBuffer(f"state{i}") for i in range(3)])
+        finally:
+            s.destroy()
+    for key in outs[0]:
+        assert rel_l2(outs[0][key], outs[1][key]) <= TOL, key

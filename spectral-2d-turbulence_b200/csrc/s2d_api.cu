@@ -118,14 +118,14 @@ static int check_device(int dev) {
 struct GraphKey {
   int phase, slot, parity;
   unsigned flags;
-  int ptr, prof, banded;
+  int ptr, prof, banded, steps;
   bool operator<(const GraphKey& o) const {
-    return std::tie(phase, slot, parity, flags, ptr, prof, banded) <
-           std::tie(o.phase, o.slot, o.parity, o.flags, o.ptr, o.prof, o.banded);
+    return std::tie(phase, slot, parity, flags, ptr, prof, banded, steps) <
+           std::tie(o.phase, o.slot, o.parity, o.flags, o.ptr, o.prof, o.banded, o.steps);
   }
 };
 
-// a captured substep; when profiling, it carries event-record nodes around its kernels
+// captured substeps; when profiling, it carries event-record nodes around its kernels
 struct GraphEntry {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -145,6 +145,7 @@ static size_t diag_block_offset(int nbins, int n, int b) { return (size_t)b * di
 static size_t diag_dt_offset(int nbins, int n) { return 2 * diag_block_stride(nbins, n); }
 static size_t diag_alloc_bytes(int nbins, int n) { return diag_dt_offset(nbins, n) + 4 * sizeof(float); }
 
+constexpr int kGraphSteps = 6;   // substeps of a long run's graph (phases, dt slots and dye textures realign)
 constexpr int kUploadSlots = 8;
 constexpr size_t kUploadSlotBytes = 512;
 // the parameter and splat blocks sit back to back in one device allocation, so that a
@@ -164,6 +165,7 @@ struct s2d_solver {
   cudaStream_t diag_stream = nullptr;
   cudaEvent_t diag_ready = nullptr;     // main-stream point the diagnostics stream waits for
   cudaEvent_t diag_done = nullptr;      // the last spectra launch has finished
+  cudaEvent_t join_event = nullptr;     // orders the dye branch while substeps are captured
   bool diag_outstanding = false;        // diag_done not yet waited for by the main stream
   int diag_age = 0;                     // steps enqueued since the outstanding spectra launch
   int in_step = 0;                      // inside a step call (its inner entry points do not order)
@@ -220,6 +222,9 @@ struct s2d_solver {
   double sim_time = 0.0;
   bool primed = false, packs_valid = false, reduced_valid = false, disposed = false;
   int read_state = 0;  // 0 idle, 1 copied
+  // While s2d_step_graph captures several substeps, the dye of a small texture goes on a branch
+  // (diag_stream lends its capture) that joins before the next velocity is written.
+  bool fork_dye = false, dye_forked = false;
   bool latch_pending = false;   // S2D_STEP_RELATCH: the next step's first column kernel latches
   int phys_choice = 0, spec_choice = 0;   // stage-kernel shapes in use (ops->phys / ops->spec)
   std::map<GraphKey, GraphEntry> graphs;
@@ -320,7 +325,7 @@ static void free_solver(s2d_solver* s) {
   void* host_ptrs[] = {s->h_base, s->h_upload};
   for (void* p : host_ptrs)
     if (p) cudaFreeHost(p);
-  for (cudaEvent_t ev : {s->diag_event, s->diag_ready, s->diag_done})
+  for (cudaEvent_t ev : {s->diag_event, s->diag_ready, s->diag_done, s->join_event})
     if (ev) cudaEventDestroy(ev);
   for (cudaEvent_t ev : s->upload_ev)
     if (ev) cudaEventDestroy(ev);
@@ -688,6 +693,7 @@ extern "C" int s2d_create(int n, int dye_scale, int fft_precision, int device, s
   TRY(cudaEventCreateWithFlags(&s->diag_event, cudaEventDisableTiming), "event");
   TRY(cudaEventCreateWithFlags(&s->diag_ready, cudaEventDisableTiming), "event");
   TRY(cudaEventCreateWithFlags(&s->diag_done, cudaEventDisableTiming), "event");
+  TRY(cudaEventCreateWithFlags(&s->join_event, cudaEventDisableTiming), "event");
   for (int i = 0; i < 3; ++i) TRY(cudaMalloc(&s->state[i], cbytes), "state");
   TRY(cudaMalloc(&s->packA, cbytes), "packA");
   TRY(cudaMalloc(&s->packB, cbytes), "packB");
@@ -1015,6 +1021,15 @@ static void enqueue_phys_cols(s2d_solver* s, int mode, const PhysArgs& a) {
 
 extern "C" int s2d_encode_reduce(s2d_solver* s);
 
+// the main stream (being captured) waits for the dye branch
+static int join_dye(s2d_solver* s) {
+  if (!s->dye_forked) return S2D_OK;
+  s->dye_forked = false;
+  S2D_CUDA(cudaEventRecord(s->join_event, s->diag_stream));
+  S2D_CUDA(cudaStreamWaitEvent(s->stream, s->join_event, 0));
+  return S2D_OK;
+}
+
 // Tensor-core solvers at the sizes without fused tensor-core stage kernels (N != 1024) run
 // the reference's per-stage order (solver.js:488-521): velocity pack, two inverse 2D
 // transforms, products, forward transform, assemble, RK3 update -- with every 2D transform
@@ -1128,6 +1143,7 @@ extern "C" int s2d_encode_step(s2d_solver* s) {
     return a;
   };
   if (s->step_run && pair_cols(s) && !s->profiling) {
+    if (int rc = join_dye(s)) return rc;
     // one launch (profiling times the stages apart)
     SpecArgs b = rows_args(0);
     pair_row_args(s, &b);
@@ -1137,6 +1153,8 @@ extern "C" int s2d_encode_step(s2d_solver* s) {
   } else {
     for (int st = 0; st < 3; ++st) {
       {
+        if (st == 2)
+          if (int rc = join_dye(s)) return rc;
         ProfScope ps(s, S2D_PROF_PHYS_COLS);
         enqueue_phys_cols(s, st == 2 ? 2 : 1, cols_args(st));
         S2D_LAUNCHED();
@@ -1157,7 +1175,8 @@ static uint2* tex(s2d_solver* s, int i) { return reinterpret_cast<uint2*>(s->dye
 
 template <class G> static void launch_dye(s2d_solver* s) {
   const int p = s->dye_parity, m = s->m;
-  k_dye_fused<G><<<dim3(m / G::TX, m / G::TY), G::THREADS, G::smem(s->n, m), s->stream>>>(
+  const cudaStream_t st = s->dye_forked ? s->diag_stream : s->stream;
+  k_dye_fused<G><<<dim3(m / G::TX, m / G::TY), G::THREADS, G::smem(s->n, m), st>>>(
       s->vel, tex(s, p), tex(s, 1 - p), dt_slot(s, s->slot), s->dparams, s->dsplats, s->n, m);
 }
 
@@ -1168,6 +1187,11 @@ extern "C" int s2d_encode_dye(s2d_solver* s) {
   DeviceGuard guard(s->dev);
   const int p = s->dye_parity, m = s->m;
   ProfScope ps(s, S2D_PROF_DYE);
+  if (s->fork_dye) {
+    S2D_CUDA(cudaEventRecord(s->join_event, s->stream));
+    S2D_CUDA(cudaStreamWaitEvent(s->diag_stream, s->join_event, 0));
+    s->dye_forked = true;
+  }
   switch (dye_tile(s->n, m)) {
     case 0: launch_dye<DyeWide>(s); break;
     case 1: launch_dye<DyeSquare>(s); break;
@@ -1270,11 +1294,17 @@ extern "C" int s2d_step_graph(s2d_solver* s, int substeps, unsigned flags) {
     if (int rc = enqueue_pack_prime(s)) return rc;
   if (flags & S2D_STEP_RELATCH)
     if (int rc = sync_step_counter(s)) return rc;
-  for (int i = 0; i < substeps; ++i) {
-    const GraphKey key{s->phase, s->slot, s->dye_parity, flags, s->hs.count > 0 ? 1 : 0, s->profiling ? 1 : 0, s->banded ? 1 : 0};
+  for (int i = 0; i < substeps;) {
+    // Six substeps return phase, dt slot and dye texture to where they were, so one graph of six
+    // serves a long run: a sixth of the launches, and within it the dye of a small texture runs
+    // beside the next substep up to its velocity.  Beyond 1024^2 texels the dye fills the SMs
+    // and gains nothing there (1024^2 grid, 2048^2 dye: 134.8 us either way; 256^2 and 512^2
+    // dye: 35.8 -> 27.6 us; 512^2 and 1024^2 dye: 59.7 -> 48.8).
+    const int count = !s->profiling && substeps - i >= kGraphSteps ? kGraphSteps : 1;
+    const GraphKey key{s->phase, s->slot, s->dye_parity, flags, s->hs.count > 0 ? 1 : 0, s->profiling ? 1 : 0, s->banded ? 1 : 0, count};
     auto it = s->graphs.find(key);
     if (it == s->graphs.end()) {
-      // capture one substep from the current host state, then restore it
+      // capture the substeps from the current host state, then restore it
       const int phase = s->phase, slot = s->slot, parity = s->dye_parity;
       const uint32_t si = s->step_index;
       const bool rv = s->reduced_valid;
@@ -1282,10 +1312,16 @@ extern "C" int s2d_step_graph(s2d_solver* s, int substeps, unsigned flags) {
       cudaGraphExec_t ge = nullptr;
       const size_t ev_before = s->prof_events.size();
       S2D_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-      int rc = (flags & S2D_STEP_RELATCH) ? enqueue_relatch(s) : S2D_OK;
-      if (!rc) rc = s2d_encode_step(s);
-      if (!rc && (flags & S2D_STEP_DYE)) rc = s2d_encode_dye(s);
-      if (!rc && (flags & S2D_STEP_REDUCE)) rc = s2d_encode_reduce(s);
+      s->fork_dye = count > 1 && s->m <= 1024;
+      int rc = S2D_OK;
+      for (int k = 0; k < count && !rc; ++k) {
+        if (flags & S2D_STEP_RELATCH) rc = enqueue_relatch(s);
+        if (!rc) rc = s2d_encode_step(s);
+        if (!rc && (flags & S2D_STEP_DYE)) rc = s2d_encode_dye(s);
+        if (!rc && (flags & S2D_STEP_REDUCE)) rc = s2d_encode_reduce(s);
+      }
+      if (!rc) rc = join_dye(s);
+      s->fork_dye = s->dye_forked = false;
       cudaError_t e = cudaStreamEndCapture(s->stream, &g);
       if (rc) {
         if (g) cudaGraphDestroy(g);
@@ -1322,18 +1358,20 @@ extern "C" int s2d_step_graph(s2d_solver* s, int substeps, unsigned flags) {
         }
       }
     }
-    // advance the host mirror exactly as the captured substep did
-    s->phase = (s->phase + 1) % 3;
-    s->step_index += 1;
-    if (tc_unfused(s)) s->packs_valid = true;
-    else mark_packs(s);
-    s->reduced_valid = true;
-    if (flags & S2D_STEP_DYE) s->dye_parity ^= 1;
-    if (flags & S2D_STEP_REDUCE) {
-      s->slot ^= 1;
-      s->reduced_valid = false;
+    // advance the host mirror exactly as the captured substeps did
+    for (int k = 0; k < count; ++k, ++i) {
+      s->phase = (s->phase + 1) % 3;
+      s->step_index += 1;
+      if (tc_unfused(s)) s->packs_valid = true;
+      else mark_packs(s);
+      s->reduced_valid = true;
+      if (flags & S2D_STEP_DYE) s->dye_parity ^= 1;
+      if (flags & S2D_STEP_REDUCE) {
+        s->slot ^= 1;
+        s->reduced_valid = false;
+      }
+      ++s->diag_age;
     }
-    ++s->diag_age;
   }
   return S2D_OK;
 }

@@ -193,7 +193,7 @@ struct s2d_solver {
   // every cell of the state ring outside the dealias band is zero (seeds, steps); a caller may
   // store other states, which the pair kernels do not take
   bool banded = true;
-  float4* ptw = nullptr;              // pass-ordered twiddles of the pair kernels
+  float2* ptw = nullptr;              // pass-ordered twiddles of the pair kernels
   // the whole step in one launch (small grids), or null
   void (*step_run)(const PhysArgs&, const SpecArgs&, float2* const (&)[3], cudaStream_t) = nullptr;
   uchar4* image = nullptr;            // headless render target, grown on demand
@@ -702,7 +702,7 @@ extern "C" int s2d_create(int n, int dye_scale, int fft_precision, int device, s
   TRY(cudaMalloc(&s->force, cbytes), "force");
   TRY(cudaMalloc(&s->vel, cbytes), "vel");
   TRY(cudaMalloc(&s->tw, sizeof(float2) * n), "twiddles");
-  TRY(cudaMalloc(&s->ptw, sizeof(float4) * ops->ptw_size), "twiddles");
+  TRY(cudaMalloc(&s->ptw, sizeof(float2) * ops->ptw_size), "twiddles");
   // column-kernel grids are at most n CTAs in every registered shape
   const int nparts = std::max(std::max(n, 256), seed_parts_count(n));
   TRY(cudaMalloc(&s->partials, sizeof(float) * nparts), "partials");

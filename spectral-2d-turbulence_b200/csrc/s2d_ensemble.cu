@@ -50,7 +50,7 @@ struct EnsInst {
   long long off;         // first cell in the pooled arrays
   long long roff;        // first row in the pooled row flags
   const float2* tw;      // twiddle table of this n
-  const float4* ptw;     // pass-ordered twiddles of this n (pair kernels)
+  const float2* ptw;     // pass-ordered twiddles of this n (pair kernels)
 };
 
 constexpr int kEnsAThreads = 256;
@@ -375,12 +375,12 @@ EnsTiles tiles_of(int n) {
   return n == 64 ? tiles_of<64>() : n == 128 ? tiles_of<128>() : n == 256 ? tiles_of<256>()
          : n == 512 ? tiles_of<512>() : tiles_of<1024>();
 }
-template <int N> cudaError_t ens_make_ptw(float4* out, const float2* tw, cudaStream_t st) {
+template <int N> cudaError_t ens_make_ptw(float2* out, const float2* tw, cudaStream_t st) {
   static_assert(PassTw<N, EnsCols<N>::V>::SIZE <= N && EnsCols<N>::V == EnsRows<N>::V, "one table below n entries");
-  k_pass_twiddles<N, EnsCols<N>::V><<<(N + 255) / 256, 256, 0, st>>>(out, tw);
+  k_pass_twiddles<N, EnsCols<N>::V, false><<<(N + 255) / 256, 256, 0, st>>>(out, tw);
   return cudaGetLastError();
 }
-cudaError_t ens_make_ptw(int n, float4* out, const float2* tw, cudaStream_t st) {
+cudaError_t ens_make_ptw(int n, float2* out, const float2* tw, cudaStream_t st) {
   return n == 64 ? ens_make_ptw<64>(out, tw, st) : n == 128 ? ens_make_ptw<128>(out, tw, st)
          : n == 256 ? ens_make_ptw<256>(out, tw, st) : n == 512 ? ens_make_ptw<512>(out, tw, st)
                                                                : ens_make_ptw<1024>(out, tw, st);
@@ -403,7 +403,7 @@ struct s2d_ensemble {
   bool banded = true;
   Pools pool{};
   float2* tw = nullptr;
-  float4* ptw = nullptr;
+  float2* ptw = nullptr;
   double* sums = nullptr;    // 2 * count
   int* err = nullptr;        // device error word (bounded waits that gave up)
   long long cells = 0;
@@ -488,7 +488,7 @@ extern "C" int s2d_ensemble_create(const s2d_instance_desc* descs, int count, in
     TRY(cudaGetLastError(), "twiddle kernel");
   }
   // SIZE of every pass-ordered table is below n
-  TRY(cudaMalloc(&e->ptw, sizeof(float4) * tw_len), "twiddles");
+  TRY(cudaMalloc(&e->ptw, sizeof(float2) * tw_len), "twiddles");
   for (auto& kv : tw_off)
     TRY(ens_make_ptw(kv.first, e->ptw + kv.second, e->tw + kv.second, e->stream), "twiddle kernel");
   // instances and work lists (largest grids first for balance)

@@ -89,7 +89,7 @@ struct PhysArgs {
   DevParams* latch;     // non-null: latch step_index from *counter (and advance it) first
   uint32_t* counter;
   const int* row_nz;    // non-null: row ky of PA/PB is all zero (and need not be read) where 0
-  const float4* ptw;    // pass-ordered twiddles of the pair kernels (s2d_pairs.cuh)
+  const float2* ptw;    // pass-ordered twiddles of the pair kernels (s2d_pairs.cuh)
 };
 
 // the per-substep stepIndex latch (S2D_STEP_RELATCH): params.step_index = counter++,
@@ -119,7 +119,7 @@ struct SpecArgs {
   int* err;             // device error word (bounded waits that gave up)
   int* row_nz;          // non-null: per row, 1 if the written PA/PB row holds a nonzero value;
                         // a CTA whose rows are all zero then skips its transforms and stores
-  const float4* ptw;    // pass-ordered twiddles of the pair kernels (s2d_pairs.cuh)
+  const float2* ptw;    // pass-ordered twiddles of the pair kernels (s2d_pairs.cuh)
   unsigned* top;        // pair kernel, last stage: max |u|+|v| (bits) left by k_pair_cols, or null
   float* dt_out;        // ... and the dt slot it goes to: [dt, speed]
   int full_pb;          // pair kernel: also write the rows ky < 0 of PB (readers other than k_pair_cols)

@@ -48,7 +48,7 @@ struct NOps {
   // the whole step in one launch, where the size has it (PairImpl::step_attrs)
   cudaError_t (*step_attrs)(void (**)(const PhysArgs&, const SpecArgs&, float2* const (&)[3], cudaStream_t));
   bool blocked_packs;   // the pair kernels keep the packs in blocks of four columns
-  void (*make_ptw)(float4* out, const float2* tw, cudaStream_t st);
+  void (*make_ptw)(float2* out, const float2* tw, cudaStream_t st);
   int n_phys = 0, n_spec = 0;
   PhysVariant phys[kMaxVariants];
   SpecVariant spec[kMaxVariants];
@@ -177,10 +177,12 @@ template <int N> struct PairImpl {
     return cudaSuccess;
   }
   // pass-ordered twiddles: the columns' table, then the rows'
-  static constexpr int CTW = PassTw<N, C::V>::SIZE, RTW = PassTw<N, R::V>::SIZE;
-  static void make_ptw(float4* out, const float2* tw, cudaStream_t st) {
-    k_pass_twiddles<N, C::V><<<(CTW + 255) / 256, 256, 0, st>>>(out, tw);
-    k_pass_twiddles<N, R::V><<<(RTW + 255) / 256, 256, 0, st>>>(out + CTW, tw);
+  // (float2 units; 16-byte aligned)
+  static constexpr int CTW = (PassTw<N, C::V>::SIZE + 1) & ~1, RTW = PassTw<N, R::V>::SIZE * (R::WIDE_TW ? 2 : 1);
+  static void make_ptw(float2* out, const float2* tw, cudaStream_t st) {
+    static_assert(!C::WIDE_TW, "the columns' table comes first");
+    k_pass_twiddles<N, C::V, false><<<(N + 255) / 256, 256, 0, st>>>(out, tw);
+    k_pass_twiddles<N, R::V, R::WIDE_TW><<<(N + 255) / 256, 256, 0, st>>>(out + CTW, tw);
   }
 };
 

@@ -99,9 +99,11 @@ template <int SIGN, class E> struct DftE<4, SIGN, E> {
 };
 
 // ------------------------------------------------------------------ pass-ordered twiddles
-// Entry [r-1][jm] of pass p (p >= 1) is W_N^{jm r N/(NS R)} = c - i s as (c, c, s, s): lanes
-// of a warp read consecutive entries (the plain table's stride would touch a line per lane),
-// and both components arrive as packed operands.
+// Entry [r-1][jm] of pass p (p >= 1) is W_N^{jm r N/(NS R)} = c - i s as (c, s): lanes of a warp
+// read consecutive entries (the plain table's stride would touch a line per lane).  A shape
+// with WIDE_TW has (c, c, s, s) instead, packed operands as they are: the row kernel at 1024^2,
+// where registers are to spare, gains (10.0 against 11.0 us); the others lose more to the
+// doubled loads (2048^2 step 198 against 186 us, 4096^2 798 / 760, 256 x 256^2 593 / 581).
 template <int N, int V> struct PassTw {
   using PL = LinePlan<N, V>;
   __host__ __device__ static constexpr int offset(int p) {
@@ -111,7 +113,7 @@ template <int N, int V> struct PassTw {
   }
   static constexpr int SIZE = offset(PL::P);
 };
-template <int N, int V> __global__ void k_pass_twiddles(float4* out, const float2* __restrict__ tw) {
+template <int N, int V, bool WIDE> __global__ void k_pass_twiddles(float2* out, const float2* __restrict__ tw) {
   using PL = LinePlan<N, V>;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   int o = 0;
@@ -120,7 +122,8 @@ template <int N, int V> __global__ void k_pass_twiddles(float4* out, const float
     if (i >= o && i < o + len) {
       const int q = (i - o) / ns + 1, jm = (i - o) % ns;
       const float2 w = tw[jm * q * (N / (ns * r))];   // (cos, -sin)
-      out[i] = make_float4(w.x, w.x, -w.y, -w.y);
+      if (WIDE) reinterpret_cast<float4*>(out)[i] = make_float4(w.x, w.x, -w.y, -w.y);
+      else out[i] = make_float2(w.x, -w.y);
     }
     o += len;
   }
@@ -141,12 +144,15 @@ template <int N_, int V_, bool BP_ = false> struct PairLine {
   static constexpr int PADDED = N + T;
 };
 template <int N_, int V_, int GP_, int MINB_, bool BP_ = false> struct PairCols : PairLine<N_, V_, BP_> {
+  static constexpr bool WIDE_TW = false;
   using L = PairLine<N_, V_, BP_>;
   static constexpr int GP = GP_, THREADS = GP * L::T, GRID = N_ / 2 / GP, MINB = MINB_;
   static constexpr size_t SMEM = (size_t)L::PADDED * GP * (sizeof(float4) + sizeof(float2));
   static_assert((N_ / 2) % GP == 0 && (!BP_ || GP >= 2), "whole lines and blocks");
 };
-template <int N_, int V_, int THREADS_, int MINB_, bool BP_ = false> struct PairRows : PairLine<N_, V_, BP_> {
+template <int N_, int V_, int THREADS_, int MINB_, bool BP_ = false, bool WIDE_TW_ = false>
+struct PairRows : PairLine<N_, V_, BP_> {
+  static constexpr bool WIDE_TW = WIDE_TW_;
   using L = PairLine<N_, V_, BP_>;
   static constexpr int THREADS = THREADS_, PPB = THREADS / L::T, GRID = (L::BAND + PPB - 1) / PPB, MINB = MINB_;
   static constexpr size_t SMEM = (size_t)L::PADDED * PPB * (sizeof(float4) + sizeof(float2));
@@ -170,7 +176,7 @@ template <> struct PairShape<64> { using C = PairCols<64, 4, 2, 16>; using R = P
 template <> struct PairShape<128> { using C = PairCols<128, 4, 1, 16>; using R = PairRows<128, 4, 32, 16>; };
 template <> struct PairShape<256> { using C = PairCols<256, 4, 1, 8>; using R = PairRows<256, 4, 64, 8>; };
 template <> struct PairShape<512> { using C = PairCols<512, 8, 2, 4>; using R = PairRows<512, 8, 64, 8>; };
-template <> struct PairShape<1024> { using C = PairCols<1024, 16, 4, 1>; using R = PairRows<1024, 8, 128, 3>; };
+template <> struct PairShape<1024> { using C = PairCols<1024, 16, 4, 1>; using R = PairRows<1024, 8, 128, 3, false, true>; };
 template <> struct PairShape<2048> { using C = PairCols<2048, 16, 4, 1>; using R = PairRows<2048, 16, 128, 3>; };
 template <> struct PairShape<4096> { using C = PairCols<4096, 16, 2, 1, true>; using R = PairRows<4096, 16, 256, 2, true>; };
 template <int N> struct PairStepShape { using S = void; };
@@ -196,7 +202,7 @@ template <int T, int NTHREADS> struct GroupSync {
 // Element i of the pair is at l4[pad(i) * ST], of the single line at l2[pad(i) * ST].
 template <class TU, int SIGN, bool HASX, bool HASY, int ST, class Sync>
 __device__ __forceinline__ void lines_fft(C2 (&x)[TU::V], float2 (&y)[TU::V], float4* l4, float2* l2, int t,
-                                          const float4* __restrict__ tw, const Sync& sync) {
+                                          const float2* __restrict__ tw, const Sync& sync) {
   using PL = typename TU::PL;
   constexpr int N = TU::N, V = TU::V, T = TU::T;
   sfor<PL::P>([&](auto pc) {
@@ -229,10 +235,17 @@ __device__ __forceinline__ void lines_fft(C2 (&x)[TU::V], float2 (&y)[TU::V], fl
       for (int b = 0; b < B; ++b)
 #pragma unroll
         for (int r = 1; r < R; ++r) {
-          const float4 q = __ldg(tw + PassTw<N, V>::offset(p) + (r - 1) * NS + ((t + T * b) & (NS - 1)));
-          const float2 c = make_float2(q.x, q.y), s = make_float2(q.z, q.w);
+          const int e = PassTw<N, V>::offset(p) + (r - 1) * NS + ((t + T * b) & (NS - 1));
+          float2 c, s;
+          if constexpr (TU::WIDE_TW) {
+            const float4 q = __ldg(reinterpret_cast<const float4*>(tw) + e);
+            c = make_float2(q.x, q.y), s = make_float2(q.z, q.w);
+          } else {
+            const float2 q = __ldg(tw + e);
+            c = splat2(q.x), s = splat2(q.y);
+          }
           if constexpr (HASX) v[b * R + r] = cmul_cs(v[b * R + r], c, SIGN > 0 ? s : neg2(s));
-          if constexpr (HASY) w[b * R + r] = cmul(w[b * R + r], make_float2(q.x, SIGN > 0 ? q.z : -q.z));
+          if constexpr (HASY) w[b * R + r] = cmul(w[b * R + r], make_float2(c.x, SIGN > 0 ? s.x : -s.x));
         }
     }
 #pragma unroll
@@ -275,7 +288,7 @@ __device__ __forceinline__ void lines_fft(C2 (&x)[TU::V], float2 (&y)[TU::V], fl
 // its twiddles.  One column pair per group; groups interleave over lanes (two pairs are one 32-byte sector per row).  Returns
 // this thread's max |u|+|v| (mode != 1).
 template <class TU>
-__device__ __forceinline__ float pair_cols_tile(const PhysArgs& a, size_t base, const float4* ptw, int mode, int tile,
+__device__ __forceinline__ float pair_cols_tile(const PhysArgs& a, size_t base, const float2* ptw, int mode, int tile,
                                                 float4* smem) {
   constexpr int N = TU::N, V = TU::V, T = TU::T, GP = TU::GP;
   const int g = threadIdx.x % GP, t = threadIdx.x / GP;
@@ -414,7 +427,7 @@ static __device__ __noinline__ float2 rk_cell(int stage, float2 e, float2 w0, fl
 // the arrays of `a`, its first cell is `base`.
 template <class TU, bool WAIT = false>
 __device__ __forceinline__ void pair_rows_tile(const SpecArgs& a, size_t base, const DevParams* P, float dt, bool forced,
-                                               const float4* ptw, int stage, int tile, float4* smem) {
+                                               const float2* ptw, int stage, int tile, float4* smem) {
   constexpr int N = TU::N, V = TU::V, T = TU::T, BAND = TU::BAND, KMAX = TU::KMAX;
   const int t = threadIdx.x % T, g = threadIdx.x / T;
   const int p = min(tile * TU::PPB + g, KMAX);   // the last CTA's spare groups repeat pair KMAX
@@ -439,6 +452,8 @@ __device__ __forceinline__ void pair_rows_tile(const SpecArgs& a, size_t base, c
   const float beta = P->beta, mu = P->mu, nu = P->nu_h;
   const int hyper = P->hyper_p;
   const float2 fb = forced ? forcing_k2_bounds(*P) : make_float2(1.f, 0.f);   // empty without forcing
+  // Z-hat, then the packs, lie in natural order without padding: every access of theirs is a
+  // run of consecutive slots, upwards or (-kx) downwards, at any alignment
   const float ky = (float)p;
   // all of the above is two or more launches old; Z is the launch before
   if constexpr (WAIT) pdl_wait();
@@ -453,14 +468,14 @@ __device__ __forceinline__ void pair_rows_tile(const SpecArgs& a, size_t base, c
     for (int m = 0; m < V; ++m) {
       const int c = t + T * m;
       if (!slot_empty<TU>(m) && pair_inband<TU>(c))
-        l4[TU::pad(c)] = make_float4(x[m].re.x, x[m].re.y, x[m].im.x, x[m].im.y);
+        l4[c] = make_float4(x[m].re.x, x[m].re.y, x[m].im.x, x[m].im.y);
     }
   }
   sync();
   constexpr float inv_n2 = 1.0f / ((float)N * (float)N);
 #pragma unroll 1
   for (int c = t; c < BAND; c += T) {
-    const int mc = (N - c) & (N - 1), ic = TU::pad(c), im = TU::pad(mc);
+    const int mc = (N - c) & (N - 1);
     const float kx = (float)c;
     const float k2 = kx * kx + ky * ky;
     float2 wq[4], w0q[4];
@@ -472,7 +487,7 @@ __device__ __forceinline__ void pair_rows_tile(const SpecArgs& a, size_t base, c
     fetch(c + T);
     C2 w = pair_of(wq[0], wq[2]), wm = pair_of(wq[1], wq[3]);   // columns c, -c
     if (stage >= 0) {
-      const float4 zc = l4[ic], zm = l4[im];   // (re a, re b, im a, im b)
+      const float4 zc = l4[c], zm = l4[mc];   // (re a, re b, im a, im b)
       // right-hand sides at k = (kx, ky) and (-kx, ky); the other two cells hold the conjugates
       auto minus_nhat = [&](float kxs, float2 zk, float2 zp) {   // zp = Z(-k)
         const float2 q1 = make_float2(0.5f * (zk.x + zp.x), 0.5f * (zk.y - zp.y));
@@ -557,10 +572,10 @@ __device__ __forceinline__ void pair_rows_tile(const SpecArgs& a, size_t base, c
     const C2 pc = {__fmul2_rn(w.re, fa), __fmul2_rn(w.im, fa)}, pm = {__fmul2_rn(wm.re, fa), __fmul2_rn(wm.im, fa)};
     const float2 vc = make_float2((w.im.x - wm.im.y) * hb, -(w.re.x + wm.re.y) * hb);
     const float2 vm = make_float2(-(wm.im.x - w.im.y) * hb, (wm.re.x + w.re.y) * hb);
-    l4[ic] = make_float4(pc.re.x, pc.re.y, pc.im.x, pc.im.y);
-    l4[im] = make_float4(pm.re.x, pm.re.y, pm.im.x, pm.im.y);
-    l2[ic] = vc;
-    l2[im] = vm;
+    l4[c] = make_float4(pc.re.x, pc.re.y, pc.im.x, pc.im.y);
+    l4[mc] = make_float4(pm.re.x, pm.re.y, pm.im.x, pm.im.y);
+    l2[c] = vc;
+    l2[mc] = vm;
   }
   sync();
   // in-band elements of a line, zeros elsewhere
@@ -570,7 +585,7 @@ __device__ __forceinline__ void pair_rows_tile(const SpecArgs& a, size_t base, c
       const int c = t + T * m;
       x[m] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
       if (!slot_empty<TU>(m) && pair_inband<TU>(c)) {
-        const float4 q = l4[TU::pad(c)];
+        const float4 q = l4[c];
         x[m] = {make_float2(q.x, q.y), make_float2(q.z, q.w)};
       }
     }
@@ -579,7 +594,7 @@ __device__ __forceinline__ void pair_rows_tile(const SpecArgs& a, size_t base, c
 #pragma unroll
     for (int m = 0; m < V; ++m) {
       const int c = t + T * m;
-      y[m] = !slot_empty<TU>(m) && pair_inband<TU>(c) ? l2[TU::pad(c)] : make_float2(0.f, 0.f);
+      y[m] = !slot_empty<TU>(m) && pair_inband<TU>(c) ? l2[c] : make_float2(0.f, 0.f);
     }
   };
   const size_t bs = TU::BP && !a.full_pb ? (size_t)4 * N : 4, rs = TU::BP && !a.full_pb ? 4 : N;

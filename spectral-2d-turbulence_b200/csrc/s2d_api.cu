@@ -589,10 +589,8 @@ template <class P> static void tc_fft2_launch(float2* buf, int sign, const char*
   }
 }
 template <class P> static void tc_cols_launch(int mode, const PhysArgs& a, const char* tab, int* err, cudaStream_t st) {
-  const dim3 g(tc::kC2Grid), b(tc::kC2Threads);
-  if (mode == 0) tc::k_phys_cols_tc2<0, P><<<g, b, tc::kC2Smem, st>>>(a, tab, err);
-  else if (mode == 1) tc::k_phys_cols_tc2<1, P><<<g, b, tc::kC2Smem, st>>>(a, tab, err);
-  else tc::k_phys_cols_tc2<2, P><<<g, b, tc::kC2Smem, st>>>(a, tab, err);
+  launch_pdl(mode == 0 ? tc::k_phys_cols_tc2<0, P> : mode == 1 ? tc::k_phys_cols_tc2<1, P> : tc::k_phys_cols_tc2<2, P>,
+             tc::kC2Grid, tc::kC2Threads, tc::kC2Smem, st, a, tab, err);
 }
 // the row stage on the tensor cores: mode -1 = prime (pack wcur only), 0..2 = RK stage
 template <class P> static void tc_rows_launch(int mode, bool ptr, const SpecArgs& a, const char* tab, cudaStream_t st) {

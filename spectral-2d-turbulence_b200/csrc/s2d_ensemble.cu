@@ -254,28 +254,13 @@ struct EnsWork {
   const int2* items;
   int nitems, grid;
 };
-// pair kernels with programmatic stream serialisation (pdl_wait)
-template <class... P, class... A>
-void ens_launch_pair(void (*kernel)(P...), int threads, size_t smem, const EnsWork& w, cudaStream_t st, A... args) {
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(w.grid);
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, args...);
-}
 void ens_launch_phys(int v, const EnsWork& w, cudaStream_t st, const EnsInst* inst, Pools pool) {
   if (v == 0) {
     PhysArgs a{};
     a.pa = pool.pa;
     a.pb = pool.pb;
     a.z = pool.z;
-    ens_launch_pair(k_ens_pair_cols, kEnsPairThreads, kEnsPairSmem, w, st, inst, w.items, w.nitems, a);
+    launch_pdl(k_ens_pair_cols, w.grid, kEnsPairThreads, kEnsPairSmem, st, inst, w.items, w.nitems, a);
   }
   else k_ens_phys<2><<<w.grid, kEnsAThreads, kEnsASmem, st>>>(inst, w.items, w.nitems, pool);
 }
@@ -298,7 +283,7 @@ void ens_launch_spec(int mode, int v, const EnsWork& w, cudaStream_t st, const E
     a.pa = pool.pa;
     a.pb = pool.pb;
     a.full_pb = full_pb;
-    ens_launch_pair(k_ens_pair_rows, kEnsPairThreads, kEnsPairSmem, w, st, inst, w.items, w.nitems, a, mode);
+    launch_pdl(k_ens_pair_rows, w.grid, kEnsPairThreads, kEnsPairSmem, st, inst, w.items, w.nitems, a, mode);
   } else if (mode < 0) ens_launch_spec_m<-1>(v, w, st, inst, pool, phase, err);
   else if (mode == 0) ens_launch_spec_m<0>(v, w, st, inst, pool, phase, err);
   else if (mode == 1) ens_launch_spec_m<1>(v, w, st, inst, pool, phase, err);

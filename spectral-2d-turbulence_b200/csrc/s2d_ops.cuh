@@ -105,32 +105,17 @@ template <int N, class TU> struct SpecImpl {
 };
 
 // ---------------------------------------------------------------- pair-kernel variants
-// launched with programmatic stream serialisation (pdl_wait)
-template <class A> inline void launch_pdl(void (*kernel)(A, int), int grid, int threads, size_t smem, cudaStream_t st,
-                                          const A& a, int mode) {
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, a, mode);
-}
 template <int N> struct PairImpl {
   using C = typename PairShape<N>::C;
   using R = typename PairShape<N>::R;
   static_assert(C::BP == R::BP, "one pack layout");
   static cudaError_t phys_attrs() { return set_smem(k_pair_cols<C>, C::SMEM); }
   static void phys_run(int mode, const PhysArgs& a, cudaStream_t st) {
-    launch_pdl<PhysArgs>(k_pair_cols<C>, C::GRID, C::THREADS, C::SMEM, st, a, mode);
+    launch_pdl(k_pair_cols<C>, C::GRID, C::THREADS, C::SMEM, st, a, mode);
   }
   static cudaError_t spec_attrs() { return set_smem(k_pair_rows<R>, R::SMEM); }
   static void spec_run(int mode, bool, const SpecArgs& a, cudaStream_t st) {
-    launch_pdl<SpecArgs>(k_pair_rows<R>, R::GRID, R::THREADS, R::SMEM, st, a, mode);
+    launch_pdl(k_pair_rows<R>, R::GRID, R::THREADS, R::SMEM, st, a, mode);
   }
   static PhysVariant phys() { return PhysVariant{"column pairs", &phys_attrs, &phys_run, true}; }
   static SpecVariant spec() { return SpecVariant{"row pairs", &spec_attrs, &spec_run, true}; }

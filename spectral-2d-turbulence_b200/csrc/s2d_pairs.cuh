@@ -148,7 +148,7 @@ template <int N_, int V_, int GP_, int MINB_, bool BP_ = false> struct PairCols 
   using L = PairLine<N_, V_, BP_>;
   static constexpr int GP = GP_, THREADS = GP * L::T, GRID = N_ / 2 / GP, MINB = MINB_;
   static constexpr size_t SMEM = (size_t)L::PADDED * GP * (sizeof(float4) + sizeof(float2));
-  static_assert((N_ / 2) % GP == 0 && (!BP_ || GP >= 2), "whole lines and blocks");
+  static_assert((N_ / 2) % GP == 0 && (!BP_ || GP == 2), "whole lines, one block of four columns");
 };
 template <int N_, int V_, int THREADS_, int MINB_, bool BP_ = false, bool WIDE_TW_ = false>
 struct PairRows : PairLine<N_, V_, BP_> {
@@ -360,13 +360,9 @@ __device__ __forceinline__ float pair_cols_tile(const PhysArgs& a, size_t base, 
   return speed;
 }
 
-// Programmatic dependent launch: a stage kernel may start while the one before it drains.
-// pdl_wait returns once that kernel has finished (and its writes are visible); every kernel
-// lets its successor start only after its own wait, so whatever ran two or more launches
-// back is complete when a kernel starts -- its prologue may read that, and nothing newer.
-__device__ __forceinline__ void pdl_wait() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+// bytes (a multiple of 16, from a 16-byte boundary) from global memory towards L2
+__device__ __forceinline__ void l2_prefetch(const void* p, unsigned bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
 // CTA maximum of |u|+|v| into *top (bits of a non-negative float order as integers); the row
@@ -387,6 +383,19 @@ __global__ void __launch_bounds__(TU::THREADS, TU::MINB) k_pair_cols(PhysArgs a,
   extern __shared__ __align__(16) float4 smem4[];
   pdl_wait();
   phys_latch(a);
+  if constexpr (TU::BP) {
+    // blocked packs of a column CTA are three contiguous pieces: the CTA that follows on an SM
+    // (148 SMs) finds its own on their way from HBM (4096^2: 121 -> 109 us; the row kernel's
+    // rows gained nothing, 126 -> 130 us)
+    const int next = blockIdx.x + 148 * TU::MINB;
+    if (threadIdx.x == 0 && next < TU::GRID) {
+      constexpr int W = 2 * TU::GP;   // columns
+      const size_t b = (size_t)next * TU::N * W;
+      l2_prefetch(a.pa + b, TU::BAND * W * sizeof(float2));
+      l2_prefetch(a.pa + b + (size_t)(TU::N - TU::KMAX) * W, TU::KMAX * W * sizeof(float2));
+      l2_prefetch(a.pb + b, TU::BAND * W * sizeof(float2));
+    }
+  }
   const float speed = pair_cols_tile<TU>(a, 0, a.ptw, mode, blockIdx.x, smem4);
   if (mode == 2) cols_speed_max<TU::THREADS>(a.ticket + 1, speed);
   else if (mode == 0) cols_speed_finalize<TU::THREADS>(a, speed);

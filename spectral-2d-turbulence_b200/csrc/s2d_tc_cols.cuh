@@ -173,8 +173,6 @@ __global__ void __launch_bounds__(kC2Threads, 2) k_phys_cols_tc2(PhysArgs a, con
   char* op = sm + kC2OffOp + wg * kC2Op;
   const uint32_t op_s = smem_u32(op), b_s = smem_u32(sm + kC2OffB);
   const int x0 = blockIdx.x * kC2Cols + 2 * wg;
-  phys_latch(a);
-
   // ---- CTA set-up: TMEM (64 columns per WG), barriers, table copies, row-flag bitmask
   if (warp == 0) {
     tmem_alloc(tslot, 64 * kC2Wg);
@@ -187,6 +185,9 @@ __global__ void __launch_bounds__(kC2Threads, 2) k_phys_cols_tc2(PhysArgs a, con
     mbar_arrive_expect_tx(setup, 2 * kBBytes + kTcTwBytes);
     bulk_g2s(sm + kC2OffB, tab + kTabFwd, 2 * kBBytes + kTcTwBytes, setup);   // DFT planes + twiddles
   }
+  // the set-up needs nothing of the launch before; all below does
+  pdl_wait();
+  phys_latch(a);
   if (a.row_nz) {
 #pragma unroll
     for (int i = 0; i < N / kC2Threads; ++i) {

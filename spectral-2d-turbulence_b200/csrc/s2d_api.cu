@@ -1097,9 +1097,16 @@ extern "C" int s2d_encode_prime(s2d_solver* s) {
   return S2D_OK;
 }
 
+static int diag_order_step(s2d_solver* s, int substeps);
+
 extern "C" int s2d_encode_step(s2d_solver* s) {
-  S2D_USE(s);
+  S2D_USE_NOORDER(s);
   DeviceGuard guard(s->dev);
+  if (!s->in_step) {
+    // a step of its own is ordered, and counted, as one substep
+    if (int rc = diag_order_step(s, 1)) return rc;
+    ++s->diag_age;
+  }
   if (!s->packs_valid && !tc_unfused(s))
     if (int rc = enqueue_pack_prime(s)) return rc;
   const bool ptr = s->hs.count > 0;
@@ -1181,7 +1188,7 @@ template <class G> static void launch_dye(s2d_solver* s) {
 // encodeDye (solver.js:523-536) as one fused launch: forward, backward and
 // corrected passes of a tile computed from on-chip halos (s2d_dye.cuh)
 extern "C" int s2d_encode_dye(s2d_solver* s) {
-  S2D_USE(s);
+  S2D_USE_NOORDER(s);   // touches nothing the spectra read or write
   DeviceGuard guard(s->dev);
   const int p = s->dye_parity, m = s->m;
   ProfScope ps(s, S2D_PROF_DYE);
@@ -1220,7 +1227,7 @@ extern "C" int s2d_encode_dye_passes(s2d_solver* s) {
 }
 
 extern "C" int s2d_encode_reduce(s2d_solver* s) {
-  S2D_USE(s);
+  S2D_USE_NOORDER(s);   // touches nothing the spectra read or write
   DeviceGuard guard(s->dev);
   if (!s->reduced_valid) {
     // velocity came from a stage hook: the reference's two-level reduction

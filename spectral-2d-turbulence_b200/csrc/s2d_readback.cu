@@ -53,13 +53,13 @@ struct Staging {
     if (ready) cudaEventDestroy(ready);
   }
 
-  // thread t of `threads`: chunks t, t + threads, ...
-  cudaError_t share(int t, int threads, char* dst, const char* src, size_t bytes) {
+  // thread t of `threads`: chunks t, t + threads, ... (chunk <= kSlot)
+  cudaError_t share(int t, int threads, size_t chunk, char* dst, const char* src, size_t bytes) {
     char* const slot[2] = {pinned + 2 * t * kSlot, pinned + (2 * t + 1) * kSlot};
-    const size_t chunks = (bytes + kSlot - 1) / kSlot;
+    const size_t chunks = (bytes + chunk - 1) / chunk;
     auto fill = [&](size_t c, int b) {
-      const size_t lo = c * kSlot;
-      const cudaError_t e = cudaMemcpyAsync(slot[b], src + lo, std::min(kSlot, bytes - lo), cudaMemcpyDeviceToHost, stream[t]);
+      const size_t lo = c * chunk;
+      const cudaError_t e = cudaMemcpyAsync(slot[b], src + lo, std::min(chunk, bytes - lo), cudaMemcpyDeviceToHost, stream[t]);
       return e == cudaSuccess ? cudaEventRecord(filled[2 * t + b], stream[t]) : e;
     };
     cudaError_t e = cudaStreamWaitEvent(stream[t], ready, 0);
@@ -68,7 +68,7 @@ struct Staging {
     for (size_t c = t; e == cudaSuccess && c < chunks; c += threads, b ^= 1) {
       if (c + threads < chunks) e = fill(c + threads, b ^ 1);
       if (e == cudaSuccess) e = cudaEventSynchronize(filled[2 * t + b]);
-      if (e == cudaSuccess) std::memcpy(dst + c * kSlot, slot[b], std::min(kSlot, bytes - c * kSlot));
+      if (e == cudaSuccess) std::memcpy(dst + c * chunk, slot[b], std::min(chunk, bytes - c * chunk));
     }
     if (e != cudaSuccess) cudaStreamSynchronize(stream[t]);   // no transfer into a slot outlives the read
     return e;
@@ -124,6 +124,8 @@ cudaError_t read_back(int dev, void* dst, const void* src, size_t bytes, cudaStr
   if (e != cudaSuccess) return e;
   const int cores = std::max(1, (int)std::thread::hardware_concurrency());
   int threads = (int)std::min<size_t>(std::min(kThreads, cores), std::max<size_t>(1, bytes / kPerThread));
+  // four chunks a thread at least, so that a short read overlaps its transfer with its copies
+  const size_t chunk = std::min(kSlot, std::max(size_t(64) << 10, bytes / (4 * threads) & ~size_t(4095)));
   char* const d = static_cast<char*>(dst);
   const char* const p = static_cast<const char*>(src);
   cudaError_t err[kThreads] = {};
@@ -131,7 +133,7 @@ cudaError_t read_back(int dev, void* dst, const void* src, size_t bytes, cudaStr
   int started = 1;
   auto run = [&](int t) {
     cudaError_t r = t ? cudaSetDevice(dev) : cudaSuccess;
-    if (r == cudaSuccess) r = s->share(t, threads, d, p, bytes);
+    if (r == cudaSuccess) r = s->share(t, threads, chunk, d, p, bytes);
     err[t] = r;
   };
   for (; started < threads; ++started) {

@@ -362,7 +362,7 @@ EnsTiles tiles_of(int n) {
 }
 template <int N> cudaError_t ens_make_ptw(float2* out, const float2* tw, cudaStream_t st) {
   static_assert(PassTw<N, EnsCols<N>::V>::SIZE <= N && EnsCols<N>::V == EnsRows<N>::V, "one table below n entries");
-  k_pass_twiddles<N, EnsCols<N>::V, false><<<(N + 255) / 256, 256, 0, st>>>(out, tw);
+  k_pass_twiddles<N, EnsCols<N>::V><<<(N + 255) / 256, 256, 0, st>>>(out, tw);
   return cudaGetLastError();
 }
 cudaError_t ens_make_ptw(int n, float2* out, const float2* tw, cudaStream_t st) {

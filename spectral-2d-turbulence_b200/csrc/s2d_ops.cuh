@@ -162,12 +162,10 @@ template <int N> struct PairImpl {
     return cudaSuccess;
   }
   // pass-ordered twiddles: the columns' table, then the rows'
-  // (float2 units; 16-byte aligned)
-  static constexpr int CTW = (PassTw<N, C::V>::SIZE + 1) & ~1, RTW = PassTw<N, R::V>::SIZE * (R::WIDE_TW ? 2 : 1);
+  static constexpr int CTW = PassTw<N, C::V>::SIZE, RTW = PassTw<N, R::V>::SIZE;
   static void make_ptw(float2* out, const float2* tw, cudaStream_t st) {
-    static_assert(!C::WIDE_TW, "the columns' table comes first");
-    k_pass_twiddles<N, C::V, false><<<(N + 255) / 256, 256, 0, st>>>(out, tw);
-    k_pass_twiddles<N, R::V, R::WIDE_TW><<<(N + 255) / 256, 256, 0, st>>>(out + CTW, tw);
+    k_pass_twiddles<N, C::V><<<(CTW + 255) / 256, 256, 0, st>>>(out, tw);
+    k_pass_twiddles<N, R::V><<<(RTW + 255) / 256, 256, 0, st>>>(out + CTW, tw);
   }
 };
 

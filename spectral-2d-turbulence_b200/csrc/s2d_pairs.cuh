@@ -100,10 +100,9 @@ template <int SIGN, class E> struct DftE<4, SIGN, E> {
 
 // ------------------------------------------------------------------ pass-ordered twiddles
 // Entry [r-1][jm] of pass p (p >= 1) is W_N^{jm r N/(NS R)} = c - i s as (c, s): lanes of a warp
-// read consecutive entries (the plain table's stride would touch a line per lane).  A shape
-// with WIDE_TW has (c, c, s, s) instead, packed operands as they are: the row kernel at 1024^2,
-// where registers are to spare, gains (10.0 against 11.0 us); the others lose more to the
-// doubled loads (2048^2 step 198 against 186 us, 4096^2 798 / 760, 256 x 256^2 593 / 581).
+// read consecutive entries (the plain table's stride would touch a line per lane).  As packed
+// operands (c, c, s, s) the table costs twice the loads: 2048^2 step 198 against 186 us, 4096^2
+// 798 / 760, 256 x 256^2 ensemble 593 / 581.
 template <int N, int V> struct PassTw {
   using PL = LinePlan<N, V>;
   __host__ __device__ static constexpr int offset(int p) {
@@ -113,7 +112,7 @@ template <int N, int V> struct PassTw {
   }
   static constexpr int SIZE = offset(PL::P);
 };
-template <int N, int V, bool WIDE> __global__ void k_pass_twiddles(float2* out, const float2* __restrict__ tw) {
+template <int N, int V> __global__ void k_pass_twiddles(float2* out, const float2* __restrict__ tw) {
   using PL = LinePlan<N, V>;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   int o = 0;
@@ -122,8 +121,7 @@ template <int N, int V, bool WIDE> __global__ void k_pass_twiddles(float2* out, 
     if (i >= o && i < o + len) {
       const int q = (i - o) / ns + 1, jm = (i - o) % ns;
       const float2 w = tw[jm * q * (N / (ns * r))];   // (cos, -sin)
-      if (WIDE) reinterpret_cast<float4*>(out)[i] = make_float4(w.x, w.x, -w.y, -w.y);
-      else out[i] = make_float2(w.x, -w.y);
+      out[i] = make_float2(w.x, -w.y);
     }
     o += len;
   }
@@ -144,39 +142,43 @@ template <int N_, int V_, bool BP_ = false> struct PairLine {
   static constexpr int PADDED = N + T;
 };
 template <int N_, int V_, int GP_, int MINB_, bool BP_ = false> struct PairCols : PairLine<N_, V_, BP_> {
-  static constexpr bool WIDE_TW = false;
   using L = PairLine<N_, V_, BP_>;
   static constexpr int GP = GP_, THREADS = GP * L::T, GRID = N_ / 2 / GP, MINB = MINB_;
   static constexpr size_t SMEM = (size_t)L::PADDED * GP * (sizeof(float4) + sizeof(float2));
   static_assert((N_ / 2) % GP == 0 && (!BP_ || GP == 2), "whole lines, one block of four columns");
 };
-template <int N_, int V_, int THREADS_, int MINB_, bool BP_ = false, bool WIDE_TW_ = false>
+template <int N_, int V_, int THREADS_, int MINB_, bool BP_ = false, bool SPLIT_ = false>
 struct PairRows : PairLine<N_, V_, BP_> {
-  static constexpr bool WIDE_TW = WIDE_TW_;
   using L = PairLine<N_, V_, BP_>;
-  static constexpr int THREADS = THREADS_, PPB = THREADS / L::T, GRID = (L::BAND + PPB - 1) / PPB, MINB = MINB_;
+  // SPLIT_: a CTA is one row pair with 2 T threads; the second half does the single line's
+  // transform and half of the cells
+  static constexpr bool SPLIT = SPLIT_;
+  static constexpr int TP = SPLIT ? 2 * L::T : L::T;   // threads of a row pair
+  static constexpr int THREADS = THREADS_, PPB = THREADS / TP, GRID = (L::BAND + PPB - 1) / PPB, MINB = MINB_;
   static constexpr size_t SMEM = (size_t)L::PADDED * PPB * (sizeof(float4) + sizeof(float2));
-  static_assert(THREADS % L::T == 0, "whole lines");
+  static_assert(SPLIT ? THREADS == TP && L::T >= 32 : THREADS % L::T == 0, "whole lines");
 };
 // The shapes in use, each the fastest of those timed in turn on a B200 (us per launch, graph
-// replayed, columns / rows of stage 1):
-//   64     V=4  1.7 /  3.7     V=8  1.8 /  5.1
-//   256    V=4  2.6 /  4.1     V=8  2.6 /  5.4
-//   512    V=8  3.3 /  5.7     V=4  4.3 /  6.0    V=16  5.3 / 10
-//   1024   columns V=16, 8 columns a CTA 7.4 (4 columns 8.1, V=8 9.3); rows V=8, 3 CTAs/SM 10.0
-//          (4 CTAs/SM 11.9, V=16 11, V=4 15)
-//   2048   V=16 34 / 29 (4 row CTAs/SM 32.5)    V=8 43 / 33
-//   4096   V=16 in blocks 129 / 134, in rows 189 / 125    V=8 183 / 173
+// replayed without forcing, columns / rows of stage 1; "split": SPLIT_):
+//   64     V=4  1.7 / 2.9
+//   256    V=4, 4 columns a CTA, split 2.6 / 2.7     rows not split 3.2, V=8 split 3.7
+//   512    V=8, split 3.4 / 4.5                      rows not split 4.9, V=4 split 5.3
+//   1024   columns V=16, 8 columns a CTA 7.2 (4 columns 8.1, V=8 9.3); rows V=16, split, 3 CTAs/SM
+//          8.7 (V=8 9.5, V=8 split 9.2; 2 or 4 CTAs/SM 13.1, 9.8)
+//   2048   V=16 33 / 28 (rows split 28, 4 CTAs/SM 32)    V=8 43 / 33
+//   4096   V=16 in blocks 109 / 129, in rows 189 / 125   V=8 183 / 173
 // Small grids want more threads per line (the chain of a thread's cells sets the time), large
-// ones fewer, longer passes (shared-memory traffic does).  Blocked packs pay where a column's
-// rows lie 32 KB apart (4096); at 2048 the row kernel loses what the column kernel gains.
+// ones fewer, longer passes (shared-memory traffic does).  Splitting a row pair shortens the
+// chain by a third of the cells and the single line, and pays while SMs have room.  Blocked packs
+// pay where a column's rows lie 32 KB apart (4096); at 2048 the row kernel loses what the
+// column kernel gains.
 template <int N> struct PairShape;
 template <> struct PairShape<32> { using C = PairCols<32, 4, 4, 16>; using R = PairRows<32, 4, 32, 16>; };
 template <> struct PairShape<64> { using C = PairCols<64, 4, 2, 16>; using R = PairRows<64, 4, 32, 16>; };
-template <> struct PairShape<128> { using C = PairCols<128, 4, 1, 16>; using R = PairRows<128, 4, 32, 16>; };
-template <> struct PairShape<256> { using C = PairCols<256, 4, 1, 8>; using R = PairRows<256, 4, 64, 8>; };
-template <> struct PairShape<512> { using C = PairCols<512, 8, 2, 4>; using R = PairRows<512, 8, 64, 8>; };
-template <> struct PairShape<1024> { using C = PairCols<1024, 16, 4, 1>; using R = PairRows<1024, 8, 128, 3, false, true>; };
+template <> struct PairShape<128> { using C = PairCols<128, 4, 1, 16>; using R = PairRows<128, 4, 64, 8, false, true>; };
+template <> struct PairShape<256> { using C = PairCols<256, 4, 2, 4>; using R = PairRows<256, 4, 128, 4, false, true>; };
+template <> struct PairShape<512> { using C = PairCols<512, 8, 2, 4>; using R = PairRows<512, 8, 128, 4, false, true>; };
+template <> struct PairShape<1024> { using C = PairCols<1024, 16, 4, 1>; using R = PairRows<1024, 16, 128, 3, false, true>; };
 template <> struct PairShape<2048> { using C = PairCols<2048, 16, 4, 1>; using R = PairRows<2048, 16, 128, 3>; };
 template <> struct PairShape<4096> { using C = PairCols<4096, 16, 2, 1, true>; using R = PairRows<4096, 16, 256, 2, true>; };
 template <int N> struct PairStepShape { using S = void; };
@@ -235,17 +237,10 @@ __device__ __forceinline__ void lines_fft(C2 (&x)[TU::V], float2 (&y)[TU::V], fl
       for (int b = 0; b < B; ++b)
 #pragma unroll
         for (int r = 1; r < R; ++r) {
-          const int e = PassTw<N, V>::offset(p) + (r - 1) * NS + ((t + T * b) & (NS - 1));
-          float2 c, s;
-          if constexpr (TU::WIDE_TW) {
-            const float4 q = __ldg(reinterpret_cast<const float4*>(tw) + e);
-            c = make_float2(q.x, q.y), s = make_float2(q.z, q.w);
-          } else {
-            const float2 q = __ldg(tw + e);
-            c = splat2(q.x), s = splat2(q.y);
-          }
+          const float2 q = __ldg(tw + PassTw<N, V>::offset(p) + (r - 1) * NS + ((t + T * b) & (NS - 1)));
+          const float2 c = splat2(q.x), s = splat2(q.y);
           if constexpr (HASX) v[b * R + r] = cmul_cs(v[b * R + r], c, SIGN > 0 ? s : neg2(s));
-          if constexpr (HASY) w[b * R + r] = cmul(w[b * R + r], make_float2(c.x, SIGN > 0 ? s.x : -s.x));
+          if constexpr (HASY) w[b * R + r] = cmul(w[b * R + r], make_float2(q.x, SIGN > 0 ? q.y : -q.y));
         }
     }
 #pragma unroll
@@ -438,12 +433,16 @@ template <class TU, bool WAIT = false>
 __device__ __forceinline__ void pair_rows_tile(const SpecArgs& a, size_t base, const DevParams* P, float dt, bool forced,
                                                const float2* ptw, int stage, int tile, float4* smem) {
   constexpr int N = TU::N, V = TU::V, T = TU::T, BAND = TU::BAND, KMAX = TU::KMAX;
-  const int t = threadIdx.x % T, g = threadIdx.x / T;
+  const int t = threadIdx.x % T, g = threadIdx.x / TU::TP;
+  // cells from column t0 on; with SPLIT the threads of the single line come second
+  const int t0 = threadIdx.x % TU::TP;
+  const bool has_x = !TU::SPLIT || t0 < T, has_y = !TU::SPLIT || t0 >= T;
   const int p = min(tile * TU::PPB + g, KMAX);   // the last CTA's spare groups repeat pair KMAX
   const size_t ra = base + (size_t)p * N, rb = base + (size_t)((N - p) & (N - 1)) * N;
   float4* const l4 = smem + g * TU::PADDED;
   float2* const l2 = reinterpret_cast<float2*>(smem + TU::PPB * TU::PADDED) + g * TU::PADDED;
-  const GroupSync<T, TU::THREADS> sync;
+  const GroupSync<T, TU::THREADS> sync;          // the threads of a line
+  const GroupSync<TU::TP, TU::THREADS> psync;    // ... of the pair
   C2 x[V];
   float2 y[V];
   const bool two = stage >= 1;   // w0 is not wcur
@@ -457,7 +456,7 @@ __device__ __forceinline__ void pair_rows_tile(const SpecArgs& a, size_t base, c
       if (two) nw0[0] = a.w0[ra + c], nw0[1] = a.w0[ra + mc], nw0[2] = a.w0[rb + c], nw0[3] = a.w0[rb + mc];
     }
   };
-  fetch(t);
+  fetch(t0);
   const float beta = P->beta, mu = P->mu, nu = P->nu_h;
   const int hyper = P->hyper_p;
   const float2 fb = forced ? forcing_k2_bounds(*P) : make_float2(1.f, 0.f);   // empty without forcing
@@ -466,7 +465,7 @@ __device__ __forceinline__ void pair_rows_tile(const SpecArgs& a, size_t base, c
   const float ky = (float)p;
   // all of the above is two or more launches old; Z is the launch before
   if constexpr (WAIT) pdl_wait();
-  if (stage >= 0) {
+  if (stage >= 0 && has_x) {
 #pragma unroll
     for (int m = 0; m < V; ++m) {
       const int c = t + T * m;
@@ -480,10 +479,10 @@ __device__ __forceinline__ void pair_rows_tile(const SpecArgs& a, size_t base, c
         l4[c] = make_float4(x[m].re.x, x[m].re.y, x[m].im.x, x[m].im.y);
     }
   }
-  sync();
+  psync();
   constexpr float inv_n2 = 1.0f / ((float)N * (float)N);
 #pragma unroll 1
-  for (int c = t; c < BAND; c += T) {
+  for (int c = t0; c < BAND; c += TU::TP) {
     const int mc = (N - c) & (N - 1);
     const float kx = (float)c;
     const float k2 = kx * kx + ky * ky;
@@ -493,7 +492,7 @@ __device__ __forceinline__ void pair_rows_tile(const SpecArgs& a, size_t base, c
       wq[k] = nw[k];
       w0q[k] = nw0[k];
     }
-    fetch(c + T);
+    fetch(c + TU::TP);
     C2 w = pair_of(wq[0], wq[2]), wm = pair_of(wq[1], wq[3]);   // columns c, -c
     if (stage >= 0) {
       const float4 zc = l4[c], zm = l4[mc];   // (re a, re b, im a, im b)
@@ -586,7 +585,7 @@ __device__ __forceinline__ void pair_rows_tile(const SpecArgs& a, size_t base, c
     l2[c] = vc;
     l2[mc] = vm;
   }
-  sync();
+  psync();
   // in-band elements of a line, zeros elsewhere
   auto load_x = [&] {
 #pragma unroll
@@ -616,11 +615,24 @@ __device__ __forceinline__ void pair_rows_tile(const SpecArgs& a, size_t base, c
       if (a.full_pb && p > 0) a.pb[rb + c] = cconj(y[m]);
     }
   };
-  load_x();
-  load_y();
-  sync();
-  lines_fft<TU, +1, true, true, 1>(x, y, l4, l2, t, ptw, sync);
-  store_y();
+  if constexpr (TU::SPLIT) {
+    if (has_y) {
+      load_y();
+      sync();
+      lines_fft<TU, +1, false, true, 1>(x, y, l4, l2, t, ptw, sync);
+      store_y();
+      return;
+    }
+    load_x();
+    sync();
+    lines_fft<TU, +1, true, false, 1>(x, y, l4, l2, t, ptw, sync);
+  } else {
+    load_x();
+    load_y();
+    sync();
+    lines_fft<TU, +1, true, true, 1>(x, y, l4, l2, t, ptw, sync);
+    store_y();
+  }
 #pragma unroll
   for (int m = 0; m < V; ++m) {
     const int c = t + T * m;

@@ -224,7 +224,7 @@ struct s2d_solver {
   int read_state = 0;  // 0 idle, 1 copied
   // While s2d_step_graph captures several substeps, the dye of a small texture goes on a branch
   // (diag_stream lends its capture) that joins before the next velocity is written.
-  bool fork_dye = false, dye_forked = false;
+  bool substep_graph = false, fork_dye = false, dye_forked = false;
   bool latch_pending = false;   // S2D_STEP_RELATCH: the next step's first column kernel latches
   int phys_choice = 0, spec_choice = 0;   // stage-kernel shapes in use (ops->phys / ops->spec)
   std::map<GraphKey, GraphEntry> graphs;
@@ -1182,7 +1182,7 @@ template <class G> static void launch_dye(s2d_solver* s) {
   const int p = s->dye_parity, m = s->m;
   const cudaStream_t st = s->dye_forked ? s->diag_stream : s->stream;
   k_dye_fused<G><<<dim3(m / G::TX, m / G::TY), G::THREADS, G::smem(s->n, m), st>>>(
-      s->vel, tex(s, p), tex(s, 1 - p), dt_slot(s, s->slot), s->dparams, s->dsplats, s->n, m);
+      s->vel, tex(s, p), tex(s, 1 - p), dt_slot(s, s->slot), s->dparams, s->dsplats, s->n, m, s->substep_graph ? 1 : 0);
 }
 
 // encodeDye (solver.js:523-536) as one fused launch: forward, backward and
@@ -1317,6 +1317,7 @@ extern "C" int s2d_step_graph(s2d_solver* s, int substeps, unsigned flags) {
       cudaGraphExec_t ge = nullptr;
       const size_t ev_before = s->prof_events.size();
       S2D_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
+      s->substep_graph = count > 1;
       s->fork_dye = count > 1 && s->m <= 1024;
       int rc = S2D_OK;
       for (int k = 0; k < count && !rc; ++k) {
@@ -1326,7 +1327,7 @@ extern "C" int s2d_step_graph(s2d_solver* s, int substeps, unsigned flags) {
         if (!rc && (flags & S2D_STEP_REDUCE)) rc = s2d_encode_reduce(s);
       }
       if (!rc) rc = join_dye(s);
-      s->fork_dye = s->dye_forked = false;
+      s->substep_graph = s->fork_dye = s->dye_forked = false;
       cudaError_t e = cudaStreamEndCapture(s->stream, &g);
       if (rc) {
         if (g) cudaGraphDestroy(g);

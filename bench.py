@@ -424,7 +424,7 @@ def run_ours(args):
     dom_ms, dom_n = prof[dom]
     avg_launch_s = dom_ms / 1e3 / max(dom_n, 1)
     achieved = ab[dom] / avg_launch_s / 1e9
-    kernel_names = {"phys_cols": "k_phys_cols", "spec_rows": "k_spec_rows", "dye": "k_dye_fused"}
+    kernel_names = {"phys_cols": "k_pair_cols", "spec_rows": "k_pair_rows", "dye": "k_dye_fused"}
     traffic = committed_traffic(kernel_names[dom].split()[0])
     step_ms = ms / args.steps if world == 1 else ms / args.steps
     roofline = {"bound": "hbm", "kernel": kernel_names[dom], "achieved": achieved, "peak": hbm, "unit": "GB/s",
@@ -500,8 +500,8 @@ def run_ours(args):
             "roofline": roofline,
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                     "steps": e2e_steps, "diagnostics_finite": bool(finite)},
-            # per timed step: 3 k_phys_cols + 3 k_spec_rows + k_dye_fused (the CFL reduction
-            # and the stepIndex latch are fused into k_phys_cols)
+            # per timed step: 3 k_pair_cols + 3 k_pair_rows + k_dye_fused (the CFL reduction
+            # and the stepIndex latch are fused into them)
             "gpu_launches": args.steps * 7,
             "clocks": clk,
             "cpu_baseline": cpu,
@@ -659,10 +659,10 @@ def run_ensemble(pkg, torch, world, rank, dev, args, groups=ENSEMBLE_256, seed=1
            "achieved_gbs": gbs, "hbm_peak_gbs": hbm, "frac_of_hbm": gbs / hbm, "finite": ok, "autotune": tune,
            "note": "232 N^2 algorithmic bytes per instance-step; per-instance nu, beta, drag; graph-replayed"}
     # the DRAM bytes the kernels actually move (ncu, committed under profiles/; recorded
-    # for the 256 x 256^2 ensemble): the stage kernels skip out-of-band pack rows, so
-    # they move fewer bytes than the algorithmic count, and this fraction is the one
+    # for the 256 x 256^2 ensemble): the stage kernels move the band's half of the packs
+    # only, fewer bytes than the algorithmic count, and this fraction is the one
     # that says how close to the bandwidth bound they run
-    spec_b, phys_b = committed_traffic("k_ens_spec"), committed_traffic("k_ens_phys")
+    spec_b, phys_b = committed_traffic("k_ens_pair_rows"), committed_traffic("k_ens_pair_cols")
     if spec_b and phys_b and tuple(groups) == ENSEMBLE_256:
         moved = 3 * (spec_b + phys_b)
         out["dram_traffic"] = {"bytes_per_ensemble_step": moved, "gbs": moved * ens_steps_per_s / 1e9,

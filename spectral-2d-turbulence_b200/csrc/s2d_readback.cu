@@ -25,17 +25,24 @@ constexpr size_t kSlot = size_t(1) << 20;
 // a second thread pays from two slots' worth of bytes on (its start takes ~20 us); below
 // kDirect a plain copy takes no longer than the staged one
 constexpr size_t kPerThread = 2 * kSlot, kDirect = size_t(256) << 10;
+// making the slots and giving them back takes 4-6 ms, as long as some 16 MB of plain copies: a
+// program that reads less than that from its solvers never pays for them (512^2 solver read
+// once: 5-10 ms against 1.1 ms)
+constexpr size_t kMakeFrom = size_t(16) << 20;
 
 struct Staging {
   int refs = 0;
   std::mutex busy;   // one read at a time; a read that finds it taken copies directly
   bool tried = false;
+  size_t read = 0;   // bytes asked for so far
   char* pinned = nullptr;
   cudaStream_t stream[kThreads] = {};
   cudaEvent_t filled[2 * kThreads] = {}, ready = nullptr;
 
-  bool make() {   // on first use, by the holder of `busy`
+  bool make(size_t bytes) {   // once it pays, by the holder of `busy`
     if (tried) return pinned != nullptr;
+    if (read < kMakeFrom) read += bytes;
+    if (read < kMakeFrom) return false;
     tried = true;
     bool ok = cudaEventCreateWithFlags(&ready, cudaEventDisableTiming) == cudaSuccess;
     for (cudaStream_t& s : stream) ok = ok && cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess;
@@ -119,7 +126,7 @@ cudaError_t read_back(int dev, void* dst, const void* src, size_t bytes, cudaStr
   }
   std::unique_lock<std::mutex> busy;
   if (s) busy = std::unique_lock<std::mutex>(s->busy, std::try_to_lock);
-  if (!s || !busy.owns_lock() || !s->make()) return read_direct(dst, src, bytes, stream);
+  if (!s || !busy.owns_lock() || !s->make(bytes)) return read_direct(dst, src, bytes, stream);
   cudaError_t e = cudaEventRecord(s->ready, stream);
   if (e != cudaSuccess) return e;
   const int cores = std::max(1, (int)std::thread::hardware_concurrency());

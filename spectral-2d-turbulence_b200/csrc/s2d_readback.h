@@ -6,7 +6,7 @@
 namespace s2d {
 
 // Every solver and ensemble holds one reference to its device's staging for its lifetime; the
-// staging is made by the first large read and given back with the last reference.
+// staging is made once its holders have read 16 MB and given back with the last reference.
 void readback_retain(int dev);
 void readback_release(int dev);
 

@@ -40,6 +40,24 @@ def test_fields_come_back_whole(pkg, n):
         s.destroy()
 
 
+@pytest.mark.parametrize("n", [256, 512, 1024, 2048])
+def test_reads_before_and_after_the_slots_are_made(pkg, n):
+    """Reads up to 16 MB in all copy plainly, those that follow go through the pinned slots."""
+    w = _spectrum(n, n + 1)
+    flat = w.reshape(-1).view(np.uint8)
+    s = pkg.Solver.create(n=n, dyeScale=1)
+    try:
+        s.setBuffer("state0", w)
+        for r in range((16 << 20) // flat.size + 2):
+            assert np.array_equal(s.getBuffer("state0"), w)
+        for count in {flat.size // 2 + 8, flat.size - 8, flat.size // 3 // 8 * 8}:
+            out = np.full(flat.size + 16, 0xA5, np.uint8)[3:]
+            _read(pkg, s, out, count)
+            assert np.array_equal(out[:count], flat[:count]) and np.all(out[count:] == 0xA5)
+    finally:
+        s.destroy()
+
+
 def test_pinned_destination(pkg):
     import torch
     n = 512

@@ -9,7 +9,9 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <mutex>
+#include <new>
 #include <string>
 #include <tuple>
 #include <vector>
@@ -967,18 +969,41 @@ static int enqueue_pack_prime(s2d_solver* s) {
 
 // make the rows the row kernel skipped (flagged all zero) explicit zeros, before anything
 // other than the fused stage kernels reads or writes the packs
+// blocked packs to rows through host memory, where the device has no room for a second copy
+static int unblock_packs_on_host(s2d_solver* s) {
+  const size_t n = s->n, cells = n * n;
+  std::unique_ptr<float2[]> in(new (std::nothrow) float2[2 * cells]);
+  if (!in) return fail(S2D_ERR_CUDA, "out of memory for the packs");
+  float2* out = in.get() + cells;
+  for (float2* p : {s->packA, s->packB}) {
+    S2D_CUDA(cudaMemcpyAsync(in.get(), p, cells * sizeof(float2), cudaMemcpyDeviceToHost, s->stream));
+    S2D_CUDA(cudaStreamSynchronize(s->stream));
+    for (size_t b = 0; b < n / 4; ++b)
+      for (size_t r = 0; r < n; ++r) std::memcpy(out + r * n + 4 * b, in.get() + (b * n + r) * 4, 4 * sizeof(float2));
+    S2D_CUDA(cudaMemcpyAsync(p, out, cells * sizeof(float2), cudaMemcpyHostToDevice, s->stream));
+    S2D_CUDA(cudaStreamSynchronize(s->stream));
+  }
+  return S2D_OK;
+}
+
 static int materialize_packs(s2d_solver* s) {
   if (!s->packs_flagged) return S2D_OK;
   if (s->packs_half && s->ops->blocked_packs) {
     const size_t cbytes = (size_t)s->n * s->n * sizeof(float2);
     float2* tmp = nullptr;
-    S2D_CUDA(cudaMallocAsync(&tmp, cbytes, s->stream));
-    for (float2* p : {s->packA, s->packB}) {
-      S2D_CUDA(cudaMemcpyAsync(tmp, p, cbytes, cudaMemcpyDeviceToDevice, s->stream));
-      k_unblock_pack<<<cells_grid(s->n), 256, 0, s->stream>>>(p, tmp, s->n);
-      S2D_LAUNCHED();
+    const cudaError_t got = cudaMallocAsync(&tmp, cbytes, s->stream);
+    if (got == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      if (int rc = unblock_packs_on_host(s)) return rc;
+    } else {
+      S2D_CUDA(got);
+      for (float2* p : {s->packA, s->packB}) {
+        S2D_CUDA(cudaMemcpyAsync(tmp, p, cbytes, cudaMemcpyDeviceToDevice, s->stream));
+        k_unblock_pack<<<cells_grid(s->n), 256, 0, s->stream>>>(p, tmp, s->n);
+        S2D_LAUNCHED();
+      }
+      S2D_CUDA(cudaFreeAsync(tmp, s->stream));
     }
-    S2D_CUDA(cudaFreeAsync(tmp, s->stream));
   }
   if (s->packs_pairs)
     k_expand_packs<<<cells_grid(s->n), 256, 0, s->stream>>>(s->packA, s->packB, s->n, s->packs_half ? 1 : 0);
@@ -1304,7 +1329,7 @@ extern "C" int s2d_step_graph(s2d_solver* s, int substeps, unsigned flags) {
     // serves a long run: a sixth of the launches, and within it the dye of a small texture runs
     // beside the next substep up to its velocity.  Beyond 1024^2 texels the dye fills the SMs
     // and gains nothing there (1024^2 grid, 2048^2 dye: 134.8 us either way; 256^2 and 512^2
-    // dye: 35.8 -> 27.6 us; 512^2 and 1024^2 dye: 59.7 -> 48.8).
+    // dye: 29.8 -> 23.0 us, single launches 33.8; 512^2 and 1024^2 dye: 52.7 -> 49.2, 56.4).
     const int count = !s->profiling && substeps - i >= kGraphSteps ? kGraphSteps : 1;
     const GraphKey key{s->phase, s->slot, s->dye_parity, flags, s->hs.count > 0 ? 1 : 0, s->profiling ? 1 : 0, s->banded ? 1 : 0, count};
     auto it = s->graphs.find(key);

@@ -206,7 +206,8 @@ int s2d_reset_scenario(s2d_solver* s, int kind, double param, int dye_pattern);
 /* ---------------------------------------------------------------- autotuner */
 /* No counterpart in the reference (its kernels have one fixed shape).  Each grid
  * size registers up to S2D_TUNE_MAX launch shapes of the column and the row stage
- * kernels (values per thread / radix of the line passes, resident CTAs per SM);
+ * kernels (index 0: the pair kernels, for dealiased states; from 1 on, values per thread /
+ * radix of the line passes and resident CTAs per SM of the kernels that take any state);
  * s2d_autotune times them on this solver's own state (`steps` RK3 steps each, the
  * state saved and restored around every trial), keeps the fastest column shape and
  * then the fastest row shape with it, drops captured step graphs, and remembers the
@@ -250,7 +251,9 @@ int s2d_encode_reduce(s2d_solver* s);                                    /* solv
 /* `substeps` repetitions of encodeStep (+ encodeDye, + encodeReduce per flags),
  * priming first when needed: the body of main.js:409-419. */
 int s2d_step(s2d_solver* s, int substeps, unsigned flags);
-/* As s2d_step, replayed from a captured CUDA graph of one substep. */
+/* As s2d_step, replayed from captured CUDA graphs: one of six substeps for every six of a run
+ * (the state ring, the dt slots and the dye textures are then back where they were), one of a
+ * single substep for the rest; the same results bit for bit. */
 int s2d_step_graph(s2d_solver* s, int substeps, unsigned flags);
 
 /* ---------------------------------------------------------------- diagnostics */
@@ -368,7 +371,8 @@ int s2d_ensemble_energy(s2d_ensemble* e, double* energy, double* enstrophy);
 /* The autotuner for an ensemble (no reference counterpart): times the registered
  * resident-CTA shapes of the persistent column and row kernels over `steps` RK3 steps
  * of this ensemble (its state saved and restored bit for bit), keeps the fastest, and
- * drops captured step graphs.  The shapes differ in register allocation only. */
+ * drops captured step graphs.  Index 0 is the pair kernel, for dealiased states; the others
+ * differ from one another in register allocation only. */
 int s2d_ensemble_autotune(s2d_ensemble* e, int steps, s2d_tune_report* report);
 int s2d_ensemble_tune_variant_name(s2d_ensemble* e, int kind, int index, char* out, int cap);
 /* Pin the column / row launch shapes (indices as in the report above; drops captured

@@ -831,7 +831,7 @@ __global__ void __launch_bounds__(G::THREADS, G::MINB)
     dye_cta_passes_interior<G>(c);
   else dye_cta_passes<G, true>(c);
   // the next step's column kernel may be launched as the last tiles end (it waits for this kernel
-  // before it reads).  Inside a graph of substeps that saves 6 us of 139 at a 2048^2 dye; between
+  // before it reads).  Inside a graph of substeps that saves 5 us of 139 at a 2048^2 dye; between
   // single launches it costs 3, so the caller says which
   if (trigger) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }

@@ -3,7 +3,8 @@
 // Every pass of the fused RK3 stage (physical columns, spectral row pairs) is ONE
 // persistent launch over a work list of (instance, tile) items that mixes grid
 // sizes 64..1024; each CTA loops over items, dispatching on the instance's N to
-// the same tile functions the single-instance kernels use.  All instances share
+// the same tile functions the single-instance kernels use (the pairs of s2d_pairs.cuh while
+// every state is dealiased, otherwise those of s2d_kernels.cuh).  All instances share
 // pooled buffers (state ring, packs, product spectra) addressed by per-instance
 // offsets, and carry their own viscosity, beta, drag, forcing and dt.  A whole
 // RK3 step (6 launches) is captured into a CUDA graph and replayed.
@@ -78,9 +79,13 @@ constexpr size_t kEnsBBarOff =
 constexpr size_t kEnsBSmem = kEnsBBarOff + 16;
 
 // Pair kernels (dealiased states): 128 threads at every size, so 128 / T row pairs or column
-// pairs per item -- a 128-thread CTA synchronises at most four warps.  The row kernel runs three
-// CTAs per SM at 168 registers: at four and 128 it spills (256 x 256^2: 593 against 645 us per
-// step; two CTAs 678), and the column kernel four (three 628).
+// pairs per item -- a 128-thread CTA synchronises at most four warps (256 threads in the column
+// kernel: 610 us per step of 256 x 256^2 against 593).  The row kernel runs three CTAs per SM at
+// 168 registers, since at four and 128 it spills (645; two CTAs 678, five 818), and the column
+// kernel four (three 628).  Bound by the L1 path (columns: 72 % of its wavefronts, rows 52 %) and
+// the waits for pooled state that is larger than L2: rows 115 us and columns 85 cold, 299 and
+// 178 MB, where k_ens_spec and k_ens_phys take 259 and 94.  Per step, with twiddles as (c, s):
+// 256 x 256^2 1098 -> 581 us, 64 x 128^2 + 128 x 256^2 + 16 x 512^2 1006 -> 555.
 constexpr int kEnsPairThreads = 128, kEnsColsMinb = 4, kEnsRowsMinb = 3;
 template <int N> using EnsCols = PairCols<N, 8, kEnsPairThreads / (N / 8), kEnsColsMinb>;
 template <int N> using EnsRows = PairRows<N, 8, kEnsPairThreads, kEnsRowsMinb>;

@@ -1,6 +1,8 @@
 // s2d_kernels.cuh -- sm_100a kernels of the integrating-factor RK3 step.
 //
-// Fused step (one RK stage = two kernels, both whole-line FFTs in shared memory):
+// Fused step (one RK stage = two kernels, both whole-line FFTs in shared memory).  These two take
+// any state, also one with cells outside the 2/3 band; the states that have none step through the
+// pair kernels of s2d_pairs.cuh, unless a caller pins a shape of these:
 //
 //   k_phys_cols  "physical columns": for a tile of GA columns x, read the
 //                x-transformed packs PA(ky,x) = FFT_x^-1(w + i u_hat),
@@ -32,7 +34,7 @@ namespace s2d {
 // rows its RK update reads by bulk copy (PF_), and whether it runs the two inverse
 // x-transforms of the next packs as one two-line transform (PAIR_: half the
 // barrier-separated passes, twice the registers).  Tune<N> is the default shape; the
-// autotuner picks among the variants each size registers (s2d_ops.cuh).
+// autotuner picks among the variants each size registers (s2d_ops.cuh, after the pair shape).
 template <int N_, int V_ = 16, int AMB_ = 0, int BMB_ = 0, bool PF_ = false, bool PAIR_ = false> struct Tune {
   static constexpr int N = N_;
   static constexpr int V = V_;

@@ -1,9 +1,9 @@
 // s2d_ops.cuh -- per-grid-size launch tables for the templated kernels.
 //
-// Each grid size registers one or more launch shapes (Tune<N, V, minBlocks>) of the two
-// stage kernels; index 0 is the default shape Tune<N>.  The autotuner (s2d_autotune)
-// times the registered shapes on the solver's own state and keeps the fastest column
-// and row variants.
+// Each grid size registers its launch shapes of the two stage kernels: index 0, the default,
+// is the pair kernel (s2d_pairs.cuh), index 1 the shape Tune<N> of the kernels that take any
+// state (s2d_kernels.cuh), the rest further shapes of those.  The autotuner (s2d_autotune)
+// times them on the solver's own state and keeps the fastest column and row variants.
 #pragma once
 #include <cuda_runtime.h>
 #include <type_traits>

@@ -8,8 +8,9 @@
 //   k_pair_rows  rows ky and -ky of one pair per group of T = N/V threads.  A thread owns the
 //                four cells (+-kx, +-ky) of each of its columns: they share |k|^2, 1/|k|^2,
 //                the integrating factor (conjugated for -kx), the forcing envelope, and two
-//                of the four Hermitian unpacks and forcing phases.  Its state cells are
-//                loaded before the x-transform of Z and wait in registers.
+//                of the four Hermitian unpacks and forcing phases.  Its cells are a rolled
+//                loop with the state one column ahead, the first column's ahead of the
+//                x-transform and of the launch dependency.
 //   k_pair_cols  columns x and x+1.  v is real, so its x-transformed spectrum obeys
 //                PB(-ky, x) = conj PB(ky, x): only the rows ky >= 0 are stored, and the two
 //                columns' v come out of ONE complex y-transform of V(x) + i V(x+1).
@@ -18,6 +19,14 @@
 // PB); per column pair 3 inverse and 2 forward lines (4 and 2).  PB holds the Hermitian part
 // of v_hat, whose inverse transform is the real part the stage reads, so a state that is not
 // exactly Hermitian steps as before.
+//
+// Bound (1024^2, cold launches under a profiler): latency.  Columns 11.9 us, 8.5 MB read, issue
+// slots 32 % busy, 8 warps per SM (one CTA of 256 threads on each of 128 SMs: its registers are
+// its lines); rows 14.1 us, 13.4 MB read, 34 %, 9 warps, waiting at the barriers of the
+// transforms and for Z and the state.  The kernels of s2d_kernels.cuh take 13.9 and 23.3 us there, with
+// 4.5 and 8.3 M warp instructions against 2.5 and 3.4 M.  An RK3 step, graph-replayed with
+// forcing, against those kernels (us): 64^2 17 / 55.8, 256^2 20.6 / 56, 512^2 28.4 / 63,
+// 1024^2 52 / 98, 2048^2 186 / 418, 4096^2 730 / 2023.
 //
 // States with cells outside the band, set by a caller, take the kernels of s2d_kernels.cuh.
 #pragma once
@@ -373,6 +382,10 @@ template <int NTHREADS> __device__ __forceinline__ void cols_speed_max(unsigned*
   if (threadIdx.x == 0) atomicMax(top, m);
 }
 
+// Bound by latency up to 1024^2 (one wave; see the head of this file), beyond that by shared
+// memory's wavefronts and, at 4096^2, HBM.  The stage is a run-time argument, as in the row
+// kernel: three copies of the code fetched anew by each launch cost more than the tests.
+// 1024^2 7.2 us a launch (k_phys_cols 14), 2048^2 33, 4096^2 109.
 template <class TU>
 __global__ void __launch_bounds__(TU::THREADS, TU::MINB) k_pair_cols(PhysArgs a, int mode) {
   extern __shared__ __align__(16) float4 smem4[];
@@ -650,6 +663,10 @@ __device__ __forceinline__ void pair_cfl(const SpecArgs& a) {
   *a.top = 0u;
 }
 
+// Bound by latency: the barriers of two transforms and a chain of cells per thread (1024^2
+// 8.7 us a launch where k_spec_rows takes 23; 2048^2 28, 4096^2 129).  The cell loop is rolled,
+// with its rare parts out of line, since unrolled it waited on instruction fetches (64^2 5.2 us
+// against 3.7; at 1024^2 3.8 such stalls per issue, now 0.6).
 template <class TU>
 __global__ void __launch_bounds__(TU::THREADS, TU::MINB) k_pair_rows(SpecArgs a, int stage) {
   extern __shared__ __align__(16) float4 smem4[];
@@ -659,9 +676,11 @@ __global__ void __launch_bounds__(TU::THREADS, TU::MINB) k_pair_rows(SpecArgs a,
 }
 
 // ------------------------------------------------------------------ a whole step in one launch
-// Up to 256^2 a stage kernel is launch and latency (3.4 us each at 64^2 for 0.3 us of work), so
+// Up to 128^2 a stage kernel is launch and latency (3.4 us each at 64^2 for 0.3 us of work), so
 // one thread-block cluster runs the six passes: the packs and Z go through L2 as between
-// launches, and the cluster barrier orders them.
+// launches, and the cluster barrier orders them.  64^2 20.6 -> 17 us a step, 128^2 22.7 -> 20
+// (and one host launch of 3 us instead of six); at 256^2 sixteen CTAs have too much to do: 43
+// against 25.
 template <class C_, class R_, int CTAS_> struct PairStep {
   using C = C_;
   using R = R_;

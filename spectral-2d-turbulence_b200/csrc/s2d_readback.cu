@@ -145,7 +145,12 @@ cudaError_t read_back(int dev, void* dst, const void* src, size_t bytes, cudaStr
   };
   for (; started < threads; ++started) {
     try {
-      team[started] = std::thread(run, started);
+      team[started] = std::thread([&run, t = started] {
+        // what a capture on another thread forbids is for the caller's thread, in its mode, to meet
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        run(t);
+      });
     } catch (const std::system_error&) {
       break;
     }

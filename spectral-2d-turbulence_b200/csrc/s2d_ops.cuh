@@ -115,7 +115,10 @@ template <int N> struct PairImpl {
   }
   static cudaError_t spec_attrs() { return set_smem(k_pair_rows<R>, R::SMEM); }
   static void spec_run(int mode, bool, const SpecArgs& a, cudaStream_t st) {
-    launch_pdl(k_pair_rows<R>, R::GRID, R::THREADS, R::SMEM, st, a, mode);
+    // a prime may follow right behind the kernel that writes its state, which the kernel reads
+    // ahead of its dependency: only a stage has a column kernel in between
+    if (mode < 0) k_pair_rows<R><<<R::GRID, R::THREADS, R::SMEM, st>>>(a, mode);
+    else launch_pdl(k_pair_rows<R>, R::GRID, R::THREADS, R::SMEM, st, a, mode);
   }
   static PhysVariant phys() { return PhysVariant{"column pairs", &phys_attrs, &phys_run, true}; }
   static SpecVariant spec() { return SpecVariant{"row pairs", &spec_attrs, &spec_run, true}; }

@@ -192,6 +192,7 @@ struct s2d_solver {
   bool packs_flagged = false;         // PA/PB rows flagged zero were left unwritten
   bool packs_pairs = false;           // ... by the pair kernel (rows outside the band)
   bool packs_half = false;            // ... which also left the rows ky < 0 of PB unwritten
+  int packs_blocked = 0;              // bit 0: PA, bit 1: PB lies in blocks of four columns (NOps::blocked_packs)
   // every cell of the state ring outside the dealias band is zero (seeds, steps); a caller may
   // store other states, which the pair kernels do not take
   bool banded = true;
@@ -628,6 +629,7 @@ static void mark_packs(s2d_solver* s) {
   s->packs_flagged = true;
   s->packs_pairs = pair_rows(s);
   s->packs_half = s->packs_pairs && pair_cols(s);
+  s->packs_blocked = s->packs_half && s->ops->blocked_packs ? 3 : 0;
 }
 // what the pair row kernel takes beside the row stage's arguments
 static void pair_row_args(s2d_solver* s, SpecArgs* a) {
@@ -967,44 +969,58 @@ static int enqueue_pack_prime(s2d_solver* s) {
   return S2D_OK;
 }
 
-// make the rows the row kernel skipped (flagged all zero) explicit zeros, before anything
-// other than the fused stage kernels reads or writes the packs
-// blocked packs to rows through host memory, where the device has no room for a second copy
-static int unblock_packs_on_host(s2d_solver* s) {
+// a blocked pack to rows through host memory, where the device has no room for a second copy
+static int unblock_pack_on_host(s2d_solver* s, float2* p) {
   const size_t n = s->n, cells = n * n;
   std::unique_ptr<float2[]> in(new (std::nothrow) float2[2 * cells]);
   if (!in) return fail(S2D_ERR_CUDA, "out of memory for the packs");
   float2* out = in.get() + cells;
-  for (float2* p : {s->packA, s->packB}) {
-    S2D_CUDA(cudaMemcpyAsync(in.get(), p, cells * sizeof(float2), cudaMemcpyDeviceToHost, s->stream));
-    S2D_CUDA(cudaStreamSynchronize(s->stream));
-    for (size_t b = 0; b < n / 4; ++b)
-      for (size_t r = 0; r < n; ++r) std::memcpy(out + r * n + 4 * b, in.get() + (b * n + r) * 4, 4 * sizeof(float2));
-    S2D_CUDA(cudaMemcpyAsync(p, out, cells * sizeof(float2), cudaMemcpyHostToDevice, s->stream));
-    S2D_CUDA(cudaStreamSynchronize(s->stream));
-  }
+  S2D_CUDA(cudaMemcpyAsync(in.get(), p, cells * sizeof(float2), cudaMemcpyDeviceToHost, s->stream));
+  S2D_CUDA(cudaStreamSynchronize(s->stream));
+  for (size_t b = 0; b < n / 4; ++b)
+    for (size_t r = 0; r < n; ++r) std::memcpy(out + r * n + 4 * b, in.get() + (b * n + r) * 4, 4 * sizeof(float2));
+  S2D_CUDA(cudaMemcpyAsync(p, out, cells * sizeof(float2), cudaMemcpyHostToDevice, s->stream));
+  S2D_CUDA(cudaStreamSynchronize(s->stream));
   return S2D_OK;
 }
 
+// Blocked packs to rows, in place.  The pair columns read blocks, so the packs no longer serve the
+// next step (it makes them again from the state); a pack is marked as its rewrite is enqueued, so
+// that a call after a failed one goes on with the other.
+static int unblock_packs(s2d_solver* s) {
+  if (!s->packs_blocked) return S2D_OK;
+  s->packs_valid = false;
+  const size_t cbytes = (size_t)s->n * s->n * sizeof(float2);
+  float2* tmp = nullptr;
+  const cudaError_t got = cudaMallocAsync(&tmp, cbytes, s->stream);
+  if (got == cudaErrorMemoryAllocation) cudaGetLastError();
+  else S2D_CUDA(got);
+  auto one = [&](int bit, float2* p) -> int {
+    if (!(s->packs_blocked & bit)) return S2D_OK;
+    if (tmp) {
+      S2D_CUDA(cudaMemcpyAsync(tmp, p, cbytes, cudaMemcpyDeviceToDevice, s->stream));
+      k_unblock_pack<<<cells_grid(s->n), 256, 0, s->stream>>>(p, tmp, s->n);
+      S2D_LAUNCHED();
+    } else if (int rc = unblock_pack_on_host(s, p)) {
+      return rc;
+    }
+    s->packs_blocked &= ~bit;
+    return S2D_OK;
+  };
+  int rc = one(1, s->packA);
+  if (!rc) rc = one(2, s->packB);
+  if (tmp) {
+    const cudaError_t e = cudaFreeAsync(tmp, s->stream);
+    if (!rc) S2D_CUDA(e);
+  }
+  return rc;
+}
+
+// make the rows the row kernel skipped (flagged all zero) explicit zeros, before anything
+// other than the fused stage kernels reads or writes the packs
 static int materialize_packs(s2d_solver* s) {
   if (!s->packs_flagged) return S2D_OK;
-  if (s->packs_half && s->ops->blocked_packs) {
-    const size_t cbytes = (size_t)s->n * s->n * sizeof(float2);
-    float2* tmp = nullptr;
-    const cudaError_t got = cudaMallocAsync(&tmp, cbytes, s->stream);
-    if (got == cudaErrorMemoryAllocation) {
-      cudaGetLastError();
-      if (int rc = unblock_packs_on_host(s)) return rc;
-    } else {
-      S2D_CUDA(got);
-      for (float2* p : {s->packA, s->packB}) {
-        S2D_CUDA(cudaMemcpyAsync(tmp, p, cbytes, cudaMemcpyDeviceToDevice, s->stream));
-        k_unblock_pack<<<cells_grid(s->n), 256, 0, s->stream>>>(p, tmp, s->n);
-        S2D_LAUNCHED();
-      }
-      S2D_CUDA(cudaFreeAsync(tmp, s->stream));
-    }
-  }
+  if (int rc = unblock_packs(s)) return rc;
   if (s->packs_pairs)
     k_expand_packs<<<cells_grid(s->n), 256, 0, s->stream>>>(s->packA, s->packB, s->n, s->packs_half ? 1 : 0);
   else

@@ -1,0 +1,54 @@
+"""What the library's host code enqueues, and in which order, on a runtime without a GPU."""
+import pytest
+
+import host_runtime
+
+
+@pytest.fixture(scope="module")
+def library(tmp_path_factory):
+    return host_runtime.build(tmp_path_factory.mktemp("host"))
+
+
+START = """
+import numpy as np
+def solver(n, scale=1, fft="fp32"):
+    s = pkg.Solver.create(n=n, dyeScale=scale, fft=fft)
+    s.configure({"beta": 0.0, "drag": 0.0, "viscosity": 1.0, "hyperP": 2, "forceAmp": 0.0, "forceK": 20.0,
+                 "forceWidth": 2.0, "cfl": 0.5, "dtMin": 1e-6, "dtMax": 1e-3, "dyeFade": 1.0})
+    s.reset({"k0": 6, "amplitude": 3, "seed": 5, "dyePattern": "none"})
+    return s
+def kernels(rec):
+    return [op[2][0] for op in rec.ops if op[0] == "kernel"]
+"""
+
+
+def test_a_pack_is_unblocked_once(library):
+    """4096^2, no room on the device and the second pack's transfer fails: the first pack, already in
+    rows, is not rewritten by the read that follows, and the next step makes the packs again."""
+    host_runtime.run(library, START + """
+s = solver(4096)
+s.step(1, dye=False)
+def read(name):
+    try:
+        s.getBuffer(name)
+        return True
+    except pkg.S2DError:
+        return False
+pkg.host.host_fail(b"cudaMallocAsync", 0, 2)
+pkg.host.host_fail(b"upload", 1, 1)
+pkg.host.host_forget()
+assert not read("packA")
+ups = [op[2][0] for op in Record(pkg.host).ops if op[0] == "upload"]
+assert len(ups) == 1
+pkg.host.host_fail(b"cudaMallocAsync", 0, 2)
+pkg.host.host_forget()
+assert read("packA")
+again = [op[2][0] for op in Record(pkg.host).ops if op[0] == "upload"]
+assert len(again) == 1 and again != ups, (ups, again)
+pkg.host.host_forget()
+s.encodeStep()
+names = kernels(Record(pkg.host))
+assert sum("k_pair_rows" in k for k in names) == 4, names    # three stages, and the packs before them
+s.encodeStep()
+assert sum("k_pair_rows" in k for k in kernels(Record(pkg.host))) == 7
+""")

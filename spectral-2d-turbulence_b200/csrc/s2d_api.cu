@@ -1082,6 +1082,7 @@ static int enqueue_unfused_velocity(s2d_solver* s, int idx) {
   S2D_LAUNCHED();
   if (int rc = enqueue_fft2(s, s->packA, +1)) return rc;
   if (int rc = enqueue_fft2(s, s->packB, +1)) return rc;
+  if (int rc = join_dye(s)) return rc;   // every stage writes the velocity
   k_nl_pack<<<g, 256, 0, s->stream>>>(s->packA, s->packB, s->physZ, s->vel, s->n);
   S2D_LAUNCHED();
   return S2D_OK;

@@ -52,3 +52,26 @@ assert sum("k_pair_rows" in k for k in names) == 4, names    # three stages, and
 s.encodeStep()
 assert sum("k_pair_rows" in k for k in kernels(Record(pkg.host))) == 7
 """)
+
+
+@pytest.mark.parametrize("n,scale,fft", [(256, 1, "tc-f16"), (256, 2, "tc-bf16"), (512, 2, "tc-f16"), (1024, 1, "tc-f16"),
+                                         (64, 2, "fp32"), (256, 2, "fp32"), (512, 2, "fp32"), (1024, 2, "fp32")])
+def test_the_dye_branch_joins_before_the_next_velocity(library, n, scale, fft):
+    """Graphs of six substeps: every dye kernel is ordered behind the kernel that writes its velocity
+    and ahead of the next one that does, whichever kernels a solver steps with."""
+    host_runtime.run(library, START + f"""
+s = solver({n}, {scale}, {fft!r})
+s.step(1)
+pkg.host.host_forget()
+s.step(6, graph=True)
+rec = Record(pkg.host)
+dye = rec.find("kernel", "k_dye_fused")
+one, columns = rec.find("kernel", "k_pair_step"), rec.find("kernel", "cols")
+writers = rec.find("kernel", "k_nl_pack") or one or columns[2::3]
+assert len(dye) == 6 and len(writers) in (6, 18), (dye, writers)
+for d in dye:
+    for w in writers:
+        assert rec.ordered(d, w), (d, w, rec.ops[d], rec.ops[w])
+last = rec.find("graph")[-1]
+assert max(dye) < last
+""")

@@ -135,9 +135,9 @@ struct GraphEntry {
 };
 
 // One diagnostics block: FP64 bins + energy + enstrophy [nbins + 2], u32 fixed-point bins
-// + totals [nbins + 2], zonal mean [n].
+// + totals [nbins + 2], zonal mean [n], then the [dt, speed] that go with it.
 static size_t diag_block_bytes(int nbins, int n) {
-  return (sizeof(double) + sizeof(uint32_t)) * (size_t)(nbins + 2) + sizeof(float) * (size_t)n;
+  return (sizeof(double) + sizeof(uint32_t)) * (size_t)(nbins + 2) + sizeof(float) * (size_t)(n + 2);
 }
 // Two blocks, used in turn, then the two dt slots: [block 0][block 1][dt slots], each part
 // 16-byte aligned.  Each diagnostics call fills one block and clears the sums of the other
@@ -206,7 +206,7 @@ struct s2d_solver {
   double* h_diag = nullptr;
   uint32_t* h_fixed = nullptr;      // inside h_diag's allocation
   float* h_zonal = nullptr;         // inside h_diag's allocation
-  float* h_dt = nullptr;            // inside h_base: [dt, speed] of the slot current at the copy
+  float* h_dt = nullptr;            // inside h_diag's allocation: [dt, speed] of the slot current at the copy
   double* h_base = nullptr;         // the pinned allocation (h_diag etc. point at the copied block)
   cudaEvent_t diag_event = nullptr;
   // pinned upload ring for the per-step parameter and splat blocks: slot i is rewritten
@@ -249,6 +249,7 @@ static void set_host_diag_block(s2d_solver* s, int b) {
   s->h_diag = reinterpret_cast<double*>(reinterpret_cast<char*>(s->h_base) + diag_block_offset(s->nbins, s->n, b));
   s->h_fixed = reinterpret_cast<uint32_t*>(s->h_diag + s->nbins + 2);
   s->h_zonal = reinterpret_cast<float*>(s->h_fixed + s->nbins + 2);
+  s->h_dt = s->h_zonal + s->n;
 }
 
 // Row-stage variants of a solver: the registered FP32 shapes, plus (last index) the row
@@ -723,7 +724,6 @@ extern "C" int s2d_create(int n, int dye_scale, int fft_precision, int device, s
   for (int i = 0; i < 3; ++i) TRY(cudaMalloc(&s->dye[i], dbytes), "dye");
   TRY(cudaMallocHost(&s->h_base, diag_alloc_bytes(s->nbins, n)), "pinned diag");
   std::memset(s->h_base, 0, diag_alloc_bytes(s->nbins, n));
-  s->h_dt = reinterpret_cast<float*>(reinterpret_cast<char*>(s->h_base) + diag_dt_offset(s->nbins, n));   // [dt, speed]
   set_host_diag_block(s, 0);
   TRY(cudaMallocHost(&s->h_upload, kUploadSlotBytes * kUploadSlots), "pinned upload ring");
   for (cudaEvent_t& ev : s->upload_ev) TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "event");
@@ -1462,20 +1462,22 @@ extern "C" int s2d_copy_diagnostics(s2d_solver* s) {
   S2D_USE_NOORDER(s);
   if (s->read_state != 0) return S2D_OK;    // solver.js:561-563
   DeviceGuard guard(s->dev);
-  // on the diagnostics stream, behind the spectra and the main stream's work so far (on the
-  // main stream while a caller captures it): the block last filled, and the [dt, speed]
-  // slot current now
+  const int b = s->diag_last;
+  // the [dt, speed] slot current now joins the block on the main stream, where the second step
+  // from here rewrites it: the copy below runs whenever the copy engine gets to it
+  k_diag_dt<<<1, 32, 0, s->stream>>>(dt_slot(s, s->slot), diag_zonal(s, b) + s->n);
+  S2D_LAUNCHED();
+  // the block on the diagnostics stream, behind the spectra and the main stream's work so far (on
+  // the main stream while a caller captures it)
   const bool side = !stream_capturing(s->stream);
   if (side) {
     S2D_CUDA(cudaEventRecord(s->diag_ready, s->stream));
     S2D_CUDA(cudaStreamWaitEvent(s->diag_stream, s->diag_ready, 0));
   }
   const cudaStream_t st = side ? s->diag_stream : s->stream;
-  const int b = s->diag_last;
   const size_t off = diag_block_offset(s->nbins, s->n, b);
   S2D_CUDA(cudaMemcpyAsync(reinterpret_cast<char*>(s->h_base) + off, reinterpret_cast<char*>(s->diag) + off,
                            diag_block_bytes(s->nbins, s->n), cudaMemcpyDeviceToHost, st));
-  S2D_CUDA(cudaMemcpyAsync(s->h_dt, dt_slot(s, s->slot), 2 * sizeof(float), cudaMemcpyDeviceToHost, st));
   set_host_diag_block(s, b);
   S2D_CUDA(cudaEventRecord(s->diag_event, st));
   s->read_state = 1;

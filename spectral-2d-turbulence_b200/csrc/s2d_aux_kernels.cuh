@@ -242,6 +242,11 @@ __global__ void __launch_bounds__(256) k_diag_zonal(const float2* __restrict__ v
   if (lane == 0) zonal[row] = (float)(acc / n);
 }
 
+// [dt, speed] of a slot beside the diagnostics of the same moment
+__global__ void k_diag_dt(const float* slot, float* out) {
+  if (threadIdx.x < 2) out[threadIdx.x] = slot[threadIdx.x];
+}
+
 // Both spectra in one pass over the state: the FP64 radial spectrum, energy and
 // enstrophy (spectral2d.py:92-104) and the reference's u32 fixed-point bins,
 // truncating, in the dealias band (spectrum.wgsl:19-39).

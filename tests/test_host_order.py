@@ -75,3 +75,30 @@ for d in dye:
 last = rec.find("graph")[-1]
 assert max(dye) < last
 """)
+
+
+@pytest.mark.parametrize("calls", ["s.encodeStep(); s.encodeReduce()", "s.encodeReduce()", "s.step(1, dye=False)",
+                                   "s.step(1, dye=False, graph=True)"])
+def test_the_copied_time_step_is_not_one_that_a_later_step_writes(library, calls):
+    """copyDiagnostics, then steps and reductions that write both dt slots: whatever reads a slot on
+    another stream is ordered ahead of them."""
+    host_runtime.run(library, START + f"""
+pkg.host.host_forget()
+s = solver(64)
+slots = [int(op[2][0]) for op in Record(pkg.host).ops if op[0] == "set" and int(op[2][1]) == 16]
+assert len(slots) == 1
+s.step(2, dye=False)
+pkg.host.host_forget()
+s.encodeDiagnostics(); s.copyDiagnostics()
+for _ in range(3):
+    {calls}
+rec = Record(pkg.host)
+copies = rec.find("download")
+assert copies
+reads = [i for i in copies if int(rec.ops[i][2][1]) < slots[0] + 16 and int(rec.ops[i][2][1]) + int(rec.ops[i][2][2]) > slots[0]]
+writers = [i for i in rec.find("kernel") + rec.find("graph") if i > copies[-1]]
+assert writers
+for r in reads:
+    for w in writers:
+        assert rec.ordered(r, w), (rec.ops[r], rec.ops[w])
+""")

@@ -117,13 +117,14 @@ static int check_device(int dev) {
 }
 
 // ------------------------------------------------------------------ solver object
+// what a captured substep's launches depend on beside device memory
 struct GraphKey {
   int phase, slot, parity;
   unsigned flags;
-  int ptr, prof, banded, steps;
+  int ptr, stochastic, prof, banded, steps;
   bool operator<(const GraphKey& o) const {
-    return std::tie(phase, slot, parity, flags, ptr, prof, banded, steps) <
-           std::tie(o.phase, o.slot, o.parity, o.flags, o.ptr, o.prof, o.banded, o.steps);
+    return std::tie(phase, slot, parity, flags, ptr, stochastic, prof, banded, steps) <
+           std::tie(o.phase, o.slot, o.parity, o.flags, o.ptr, o.stochastic, o.prof, o.banded, o.steps);
   }
 };
 
@@ -611,6 +612,7 @@ template <class P> static void tc_rows_launch(int mode, bool ptr, const SpecArgs
     else tc::k_spec_rows_tc2<2, true, P><<<g, b, sm, st>>>(a, tab);
   }
 }
+static int stochastic(const s2d_solver* s) { return s->hp.force_amp > 0.f ? 1 : 0; }
 static float* dt_slot(s2d_solver* s, int slot) { return s->dtbuf + 2 * slot; }
 static bool is_tc(const s2d_solver* s) { return s->fft_precision != S2D_FFT_FP32; }
 // The stage kernels of the next launch: the chosen shapes, except that the pair kernels need a
@@ -1184,7 +1186,7 @@ extern "C" int s2d_encode_step(s2d_solver* s) {
     a.dt = dt_slot(s, s->slot);
     a.params = s->dparams;
     a.tw = s->tw;
-    a.stochastic = s->hp.force_amp > 0.f ? 1 : 0;
+    a.stochastic = stochastic(s);
     a.err = s->err;
     a.row_nz = s->row_nz;
     return a;
@@ -1348,7 +1350,8 @@ extern "C" int s2d_step_graph(s2d_solver* s, int substeps, unsigned flags) {
     // and gains nothing there (1024^2 grid, 2048^2 dye: 134.8 us either way; 256^2 and 512^2
     // dye: 29.8 -> 23.0 us, single launches 33.8; 512^2 and 1024^2 dye: 52.7 -> 49.2, 56.4).
     const int count = !s->profiling && substeps - i >= kGraphSteps ? kGraphSteps : 1;
-    const GraphKey key{s->phase, s->slot, s->dye_parity, flags, s->hs.count > 0 ? 1 : 0, s->profiling ? 1 : 0, s->banded ? 1 : 0, count};
+    const GraphKey key{s->phase, s->slot, s->dye_parity, flags, s->hs.count > 0 ? 1 : 0, stochastic(s),
+                       s->profiling ? 1 : 0, s->banded ? 1 : 0, count};
     auto it = s->graphs.find(key);
     if (it == s->graphs.end()) {
       // capture the substeps from the current host state, then restore it

@@ -145,7 +145,10 @@ int s2d_set_phase(s2d_solver* s, int phase, int dye_parity);
 int s2d_set_sim_time(s2d_solver* s, double t);
 /* CUDA stream the solver enqueues on (cudaStream_t as void*), created at the highest
  * stream priority.  The diagnostics spectra and readback copies run on a second,
- * lowest-priority stream of the solver (see s2d_encode_diagnostics). */
+ * lowest-priority stream of the solver (see s2d_encode_diagnostics).
+ * Steps (or primes, or rk3 stages) that a caller captures from this stream into a graph of its
+ * own may be replayed on any state, so they, and from then on all steps of the solver, take the
+ * kernels for any state (see the autotuner), not the pair kernels.  An ensemble does the same. */
 int s2d_get_stream(s2d_solver* s, void** stream);
 /* Waits for both streams and reports a bounded device-side wait that gave up. */
 int s2d_synchronize(s2d_solver* s);

@@ -197,6 +197,9 @@ struct s2d_solver {
   // every cell of the state ring outside the dealias band is zero (seeds, steps); a caller may
   // store other states, which the pair kernels do not take
   bool banded = true;
+  // a caller has captured steps into a graph of its own, which it may replay on any state: the
+  // solver then keeps to the kernels (and packs) that take any state (note_capture)
+  bool caller_steps = false, own_capture = false;
   float2* ptw = nullptr;              // pass-ordered twiddles of the pair kernels
   // the whole step in one launch (small grids), or null
   void (*step_run)(const PhysArgs&, const SpecArgs&, float2* const (&)[3], cudaStream_t) = nullptr;
@@ -615,17 +618,26 @@ template <class P> static void tc_rows_launch(int mode, bool ptr, const SpecArgs
 static int stochastic(const s2d_solver* s) { return s->hp.force_amp > 0.f ? 1 : 0; }
 static float* dt_slot(s2d_solver* s, int slot) { return s->dtbuf + 2 * slot; }
 static bool is_tc(const s2d_solver* s) { return s->fft_precision != S2D_FFT_FP32; }
+// whether every state that the next launches may meet is dealiased
+static bool dealiased(const s2d_solver* s) { return s->banded && !s->caller_steps; }
 // The stage kernels of the next launch: the chosen shapes, except that the pair kernels need a
 // dealiased state, and the pair column kernel also rows written by the pair row kernel (it
 // reads PB's rows ky >= 0 as the Hermitian half they then are).
 static int spec_shape(const s2d_solver* s) {
-  return s->ops->spec[s->spec_choice].pairs && !s->banded ? kAnyState : s->spec_choice;
+  return s->ops->spec[s->spec_choice].pairs && !dealiased(s) ? kAnyState : s->spec_choice;
 }
 static bool pair_rows(const s2d_solver* s) { return !tc_rows(s) && s->ops->spec[spec_shape(s)].pairs; }
 static int phys_shape(const s2d_solver* s) {
   return s->ops->phys[s->phys_choice].pairs && !pair_rows(s) ? kAnyState : s->phys_choice;
 }
 static bool pair_cols(const s2d_solver* s) { return !is_tc(s) && s->ops->phys[phys_shape(s)].pairs; }
+// whether the packs are those of state[phase], laid out for the next column launch
+static bool packs_fit(const s2d_solver* s) { return s->packs_valid && s->packs_half == pair_cols(s); }
+// Steps and state updates in a caller's capture: the graph outlives what is known of the state now,
+// and its replays leave packs behind that later calls go on from.
+static void note_capture(s2d_solver* s) {
+  if (!s->own_capture && !s->caller_steps && stream_capturing(s->stream)) s->caller_steps = true;
+}
 // the packs are now those a row-stage launch writes
 static void mark_packs(s2d_solver* s) {
   s->packs_valid = true;
@@ -1123,6 +1135,7 @@ static int enqueue_unfused_step(s2d_solver* s, bool ptr) {
 extern "C" int s2d_encode_prime(s2d_solver* s) {
   S2D_USE(s);
   DeviceGuard guard(s->dev);
+  note_capture(s);
   if (tc_unfused(s)) {
     if (int rc = materialize_packs(s)) return rc;
     if (int rc = enqueue_unfused_velocity(s, s->phase)) return rc;
@@ -1151,7 +1164,8 @@ extern "C" int s2d_encode_step(s2d_solver* s) {
     if (int rc = diag_order_step(s, 1)) return rc;
     ++s->diag_age;
   }
-  if (!s->packs_valid && !tc_unfused(s))
+  note_capture(s);
+  if (!packs_fit(s) && !tc_unfused(s))
     if (int rc = enqueue_pack_prime(s)) return rc;
   const bool ptr = s->hs.count > 0;
   if (ptr) {
@@ -1339,7 +1353,7 @@ extern "C" int s2d_step_graph(s2d_solver* s, int substeps, unsigned flags) {
   InStep in_step(s);
   if (!s->primed)
     if (int rc = s2d_encode_prime(s)) return rc;
-  if (!s->packs_valid && !tc_unfused(s))
+  if (!packs_fit(s) && !tc_unfused(s))
     if (int rc = enqueue_pack_prime(s)) return rc;
   if (flags & S2D_STEP_RELATCH)
     if (int rc = sync_step_counter(s)) return rc;
@@ -1351,7 +1365,7 @@ extern "C" int s2d_step_graph(s2d_solver* s, int substeps, unsigned flags) {
     // dye: 29.8 -> 23.0 us, single launches 33.8; 512^2 and 1024^2 dye: 52.7 -> 49.2, 56.4).
     const int count = !s->profiling && substeps - i >= kGraphSteps ? kGraphSteps : 1;
     const GraphKey key{s->phase, s->slot, s->dye_parity, flags, s->hs.count > 0 ? 1 : 0, stochastic(s),
-                       s->profiling ? 1 : 0, s->banded ? 1 : 0, count};
+                       s->profiling ? 1 : 0, dealiased(s) ? 1 : 0, count};
     auto it = s->graphs.find(key);
     if (it == s->graphs.end()) {
       // capture the substeps from the current host state, then restore it
@@ -1362,6 +1376,7 @@ extern "C" int s2d_step_graph(s2d_solver* s, int substeps, unsigned flags) {
       cudaGraphExec_t ge = nullptr;
       const size_t ev_before = s->prof_events.size();
       S2D_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
+      s->own_capture = true;
       s->substep_graph = count > 1;
       s->fork_dye = count > 1 && s->m <= 1024;
       int rc = S2D_OK;
@@ -1372,7 +1387,7 @@ extern "C" int s2d_step_graph(s2d_solver* s, int substeps, unsigned flags) {
         if (!rc && (flags & S2D_STEP_REDUCE)) rc = s2d_encode_reduce(s);
       }
       if (!rc) rc = join_dye(s);
-      s->substep_graph = s->fork_dye = s->dye_forked = false;
+      s->own_capture = s->substep_graph = s->fork_dye = s->dye_forked = false;
       cudaError_t e = cudaStreamEndCapture(s->stream, &g);
       if (rc) {
         if (g) cudaGraphDestroy(g);
@@ -1965,6 +1980,7 @@ extern "C" int s2d_rk3_stage(s2d_solver* s, int stage) {
   else if (stage == 1) k_rk3<1><<<g, 256, 0, s->stream>>>(w0, wc, wo, s->rhs, dt, s->dparams, s->n);
   else k_rk3<2><<<g, 256, 0, s->stream>>>(w0, wc, wo, s->rhs, dt, s->dparams, s->n);
   S2D_LAUNCHED();
+  note_capture(s);
   s->packs_valid = false;
   s->banded = false;   // rhs is the caller's
   return S2D_OK;

@@ -391,6 +391,9 @@ struct s2d_ensemble {
   // every state is zero outside its dealias band (seeds, steps); a caller may store others,
   // which the pair kernels do not take
   bool banded = true;
+  // a caller has captured steps into a graph of its own, which it may replay on any state: the
+  // ensemble then keeps to the kernels (and packs) that take any state
+  bool caller_steps = false;
   Pools pool{};
   float2* tw = nullptr;
   float2* ptw = nullptr;
@@ -398,13 +401,14 @@ struct s2d_ensemble {
   int* err = nullptr;        // device error word (bounded waits that gave up)
   long long cells = 0;
   int phase = 0;
-  bool packs_valid = false;
-  std::map<int, std::pair<cudaGraph_t, cudaGraphExec_t>> graphs;   // by starting phase
+  bool packs_valid = false, packs_half = false;   // half: PB's rows ky < 0 unwritten, for the pair columns
+  std::map<std::pair<int, bool>, std::pair<cudaGraph_t, cudaGraphExec_t>> graphs;   // by starting phase, kind of state
 };
 
 // the shapes of the next launches: pair kernels only on dealiased states, and pair columns
 // only after pair rows (which leave PB's rows ky < 0 unwritten for them)
-static int ens_sv(const s2d_ensemble* e) { return e->sv == 0 && !e->banded ? kEnsAnyState : e->sv; }
+static bool ens_dealiased(const s2d_ensemble* e) { return e->banded && !e->caller_steps; }
+static int ens_sv(const s2d_ensemble* e) { return e->sv == 0 && !ens_dealiased(e) ? kEnsAnyState : e->sv; }
 static int ens_pv(const s2d_ensemble* e) { return e->pv == 0 && ens_sv(e) != 0 ? kEnsAnyState : e->pv; }
 static int ens_full_pb(const s2d_ensemble* e) { return ens_pv(e) != 0; }
 static void ens_drop_graphs(s2d_ensemble* e) {
@@ -666,17 +670,21 @@ extern "C" int s2d_ensemble_step(s2d_ensemble* e, int steps, int use_graph) {
   cudaGetDevice(&prev);
   if (prev != e->dev) cudaSetDevice(e->dev);
   int rc = S2D_OK;
-  if (!e->packs_valid) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(e->stream, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone) e->caller_steps = true;
+  if (!e->packs_valid || e->packs_half != !ens_full_pb(e)) {
     const int sv = ens_sv(e);
     if (sv == 0) k_ens_band_flags<<<e->count, 128, 0, e->stream>>>(e->dinst, e->pool.row_nz);
     ens_launch_spec(-1, sv, e->work_b[sv], e->stream, e->dinst, e->pool, e->phase, ens_full_pb(e), e->err);
     if (cudaGetLastError() != cudaSuccess) rc = efail(S2D_ERR_CUDA, "prime launch failed");
     e->packs_valid = true;
+    e->packs_half = !ens_full_pb(e);
   }
   int done = 0;
   if (!rc && use_graph) {
     while (!rc && steps - done >= 3) {
-      auto it = e->graphs.find(e->phase);
+      const auto key = std::make_pair(e->phase, ens_dealiased(e));
+      auto it = e->graphs.find(key);
       if (it == e->graphs.end()) {
         const int p0 = e->phase;
         cudaGraph_t g = nullptr;
@@ -698,7 +706,7 @@ extern "C" int s2d_ensemble_step(s2d_ensemble* e, int steps, int use_graph) {
           rc = efail(S2D_ERR_CUDA, cudaGetErrorString(err));
           break;
         }
-        it = e->graphs.emplace(p0, std::make_pair(g, ge)).first;
+        it = e->graphs.emplace(key, std::make_pair(g, ge)).first;
       }
       cudaError_t err = cudaGraphLaunch(it->second.second, e->stream);
       if (err != cudaSuccess) { rc = efail(S2D_ERR_CUDA, cudaGetErrorString(err)); break; }

@@ -743,10 +743,12 @@ extern "C" int s2d_create(int n, int dye_scale, int fft_precision, int device, s
   for (cudaEvent_t& ev : s->upload_ev) TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "event");
   TRY(set_all_attrs(*ops), "kernel attributes");
   if (fft_precision == S2D_FFT_FP32) TRY(ops->step_attrs(&s->step_run), "kernel attributes");
+  // the limit is the kernel's, not the solver's: the most that any grid of the tile shape asks for
+  // (the velocity window grows with n / m, at most 1/2 under wide tiles)
   switch (dye_tile(n, s->m)) {
-    case 0: TRY(set_smem(k_dye_fused<DyeWide>, DyeWide::smem(n, s->m)), "dye kernel attributes"); break;
-    case 1: TRY(set_smem(k_dye_fused<DyeSquare>, DyeSquare::smem(n, s->m)), "dye kernel attributes"); break;
-    default: TRY(set_smem(k_dye_fused<DyeSmall>, DyeSmall::smem(n, s->m)), "dye kernel attributes"); break;
+    case 0: TRY(set_smem(k_dye_fused<DyeWide>, DyeWide::smem(1, 2)), "dye kernel attributes"); break;
+    case 1: TRY(set_smem(k_dye_fused<DyeSquare>, DyeSquare::smem(1, 1)), "dye kernel attributes"); break;
+    default: TRY(set_smem(k_dye_fused<DyeSmall>, DyeSmall::smem(1, 1)), "dye kernel attributes"); break;
   }
   if (fft_precision == S2D_FFT_TC_F16 && n == 1024) TRY(tc_attrs<tc::PrecF16>(), "tensor-core kernel attributes");
   if (fft_precision == S2D_FFT_TC_BF16 && n == 1024) TRY(tc_attrs<tc::PrecBF16>(), "tensor-core kernel attributes");

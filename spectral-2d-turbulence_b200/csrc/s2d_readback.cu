@@ -13,7 +13,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
-#include <system_error>
+#include <new>
 #include <thread>
 #include <vector>
 
@@ -94,9 +94,15 @@ cudaError_t read_direct(void* dst, const void* src, size_t bytes, cudaStream_t s
 
 void readback_retain(int dev) {
   std::lock_guard<std::mutex> lk(g_mu);
-  std::shared_ptr<Staging>& s = g_staging[dev];
-  if (!s) s = std::make_shared<Staging>();
-  ++s->refs;
+  auto it = g_staging.find(dev);
+  if (it == g_staging.end()) {
+    try {
+      it = g_staging.emplace(dev, std::make_shared<Staging>()).first;
+    } catch (const std::bad_alloc&) {
+      return;   // fields are then copied directly
+    }
+  }
+  ++it->second->refs;
 }
 
 void readback_release(int dev) {
@@ -151,7 +157,7 @@ cudaError_t read_back(int dev, void* dst, const void* src, size_t bytes, cudaStr
         cudaThreadExchangeStreamCaptureMode(&mode);
         run(t);
       });
-    } catch (const std::system_error&) {
+    } catch (...) {   // no thread to be had, or no memory for one: its share is done below
       break;
     }
   }

@@ -102,3 +102,38 @@ for r in reads:
     for w in writers:
         assert rec.ordered(r, w), (rec.ops[r], rec.ops[w])
 """)
+
+
+@pytest.mark.parametrize("after", [0, 1, 2])
+def test_a_read_goes_on_where_a_helper_thread_cannot_start(library, after):
+    """A field read by several threads, memory short as the second, third or fourth is made: their
+    shares fall to the threads that run, and no exception leaves the call."""
+    host_runtime.run(library, START + f"""
+s = solver(2048)
+want = np.arange(2048 * 2048, dtype=np.float32).astype(np.complex64).reshape(2048, 2048)
+want[683:1366], want[:, 683:1366] = 0, 0
+s.setBuffer("state0", want)
+assert np.array_equal(s.getBuffer("state0"), want)      # the slots are made
+pkg.host.host_fail_new({after})
+got = s.getBuffer("state0")
+pkg.host.host_fail_new(-1)
+assert np.array_equal(got, want)
+""")
+
+
+def test_a_solver_without_readback_slots_reads_directly(library):
+    """Memory short as the slots' holder is made (the second allocation of create): the solver works,
+    and so does one made and destroyed beside it."""
+    host_runtime.run(library, START + """
+pkg.host.host_fail_new(1)
+s = pkg.Solver.create(n=64, dyeScale=1)
+pkg.host.host_fail_new(-1)
+t = solver(2048)
+w = np.zeros((64, 64), np.complex64); w[1, 1] = 3
+s.setBuffer("state0", w)
+for _ in range(3):
+    assert np.array_equal(s.getBuffer("state0"), w) and t.getBuffer("state0").shape == (2048, 2048)
+s.destroy()
+assert t.getBuffer("state0").shape == (2048, 2048)
+t.destroy()
+""")

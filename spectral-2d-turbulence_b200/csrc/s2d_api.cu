@@ -149,6 +149,7 @@ static size_t diag_dt_offset(int nbins, int n) { return 2 * diag_block_stride(nb
 static size_t diag_alloc_bytes(int nbins, int n) { return diag_dt_offset(nbins, n) + 4 * sizeof(float); }
 
 constexpr int kGraphSteps = 6;   // substeps of a long run's graph (phases, dt slots and dye textures realign)
+constexpr int kGraphWorth = 60;  // substeps launched singly that cost what capturing such a graph does
 constexpr int kUploadSlots = 8;
 constexpr size_t kUploadSlotBytes = 512;
 // the parameter and splat blocks sit back to back in one device allocation, so that a
@@ -235,6 +236,7 @@ struct s2d_solver {
   bool latch_pending = false;   // S2D_STEP_RELATCH: the next step's first column kernel latches
   int phys_choice = 0, spec_choice = 0;   // stage-kernel shapes in use (ops->phys / ops->spec)
   std::map<GraphKey, GraphEntry> graphs;
+  int unaligned = 0;   // substeps launched singly for want of a graph of six (six_graph_from)
   // instrumentation: event pairs around launches, by kernel class
   bool profiling = false;
   std::vector<std::tuple<int, cudaEvent_t, cudaEvent_t>> prof_events;
@@ -1347,6 +1349,30 @@ extern "C" int s2d_step(s2d_solver* s, int substeps, unsigned flags) {
   return S2D_OK;
 }
 
+// the key of a graph that starts `ahead` substeps from here
+static GraphKey graph_key(const s2d_solver* s, unsigned flags, int ahead, int steps) {
+  return {(s->phase + ahead) % 3, s->slot ^ (flags & S2D_STEP_REDUCE ? ahead & 1 : 0),
+          s->dye_parity ^ (flags & S2D_STEP_DYE ? ahead & 1 : 0), flags, s->hs.count > 0 ? 1 : 0, stochastic(s),
+          s->profiling ? 1 : 0, dealiased(s) ? 1 : 0, steps};
+}
+// From which substep of a run on it takes graphs of six (`substeps`: none).  Capturing one takes as
+// long as 60 substeps gain by it (64^2, 256^2, 1024^2 with their dye: 0.2, 0.5-1, 0.25 ms), so the
+// first run captures one where it starts; a later run that starts elsewhere in the cycle of six goes
+// there by single substeps, and captures one of its own once 60 substeps have gone out singly.
+static int six_graph_from(s2d_solver* s, int substeps, unsigned flags) {
+  if (s->profiling || substeps < kGraphSteps) return substeps;
+  for (int ahead = 0; ahead < kGraphSteps; ++ahead) {
+    if (!s->graphs.count(graph_key(s, flags, ahead, kGraphSteps))) continue;
+    if (ahead == 0) return 0;
+    const bool reach = substeps - ahead >= kGraphSteps;
+    s->unaligned += reach ? ahead : substeps / kGraphSteps * kGraphSteps;
+    if (s->unaligned < kGraphWorth) return reach ? ahead : substeps;
+    break;
+  }
+  s->unaligned = 0;
+  return 0;
+}
+
 extern "C" int s2d_step_graph(s2d_solver* s, int substeps, unsigned flags) {
   S2D_USE_NOORDER(s);
   if (substeps < 0) return fail(S2D_ERR_ARG, "substeps < 0");
@@ -1359,15 +1385,15 @@ extern "C" int s2d_step_graph(s2d_solver* s, int substeps, unsigned flags) {
     if (int rc = enqueue_pack_prime(s)) return rc;
   if (flags & S2D_STEP_RELATCH)
     if (int rc = sync_step_counter(s)) return rc;
+  const int sixes = six_graph_from(s, substeps, flags);
   for (int i = 0; i < substeps;) {
     // Six substeps return phase, dt slot and dye texture to where they were, so one graph of six
     // serves a long run: a sixth of the launches, and within it the dye of a small texture runs
     // beside the next substep up to its velocity.  Beyond 1024^2 texels the dye fills the SMs
     // and gains nothing there (1024^2 grid, 2048^2 dye: 134.8 us either way; 256^2 and 512^2
     // dye: 29.8 -> 23.0 us, single launches 33.8; 512^2 and 1024^2 dye: 52.7 -> 49.2, 56.4).
-    const int count = !s->profiling && substeps - i >= kGraphSteps ? kGraphSteps : 1;
-    const GraphKey key{s->phase, s->slot, s->dye_parity, flags, s->hs.count > 0 ? 1 : 0, stochastic(s),
-                       s->profiling ? 1 : 0, dealiased(s) ? 1 : 0, count};
+    const int count = i >= sixes && substeps - i >= kGraphSteps ? kGraphSteps : 1;
+    const GraphKey key = graph_key(s, flags, 0, count);
     auto it = s->graphs.find(key);
     if (it == s->graphs.end()) {
       // capture the substeps from the current host state, then restore it

@@ -137,3 +137,25 @@ s.destroy()
 assert t.getBuffer("state0").shape == (2048, 2048)
 t.destroy()
 """)
+
+
+def test_short_runs_do_not_capture_at_every_place(library):
+    """Runs of seven substeps start at every place of the cycle of six: the first captures a graph of
+    six, the others go on with single ones, until these have cost what a capture does."""
+    host_runtime.run(library, START + """
+def calls(s, runs):
+    pkg.host.host_forget()
+    for n in runs:
+        s.step(n, graph=True)
+    lines = pkg.host.host_record().decode().splitlines()
+    return sum(l.startswith("captured") for l in lines), sum(l.startswith("graph") for l in lines)
+for scale in (1, 2):
+    s = solver(64, scale)
+    assert calls(s, [7]) == (2, 2)                   # six, one
+    assert calls(s, [7] * 5)[0] == 5                 # the single substeps of the other places
+    calls(s, [7] * 300)
+    assert calls(s, [7] * 6) == (0, 12)              # in the end a six and a single one each
+s = solver(256)
+assert calls(s, [100]) == (5, 20)                    # 16 sixes, four single ones, captured where they lie
+assert calls(s, [100]) == (2, 20)                    # two single ones to the graph, 16 sixes, two more
+""")

@@ -70,19 +70,38 @@ def _rows_in_band(n):
     return sum(1 for i in range(n) if abs(i if i < n // 2 else i - n) < kcut)
 
 
-def algorithmic_bytes(n, m):
+def pair_stages(tune):
+    """Whether the column and the row stage run as pair kernels, from autotune()'s report or --shapes."""
+    if "pinned" in tune:
+        col, row = tune["pinned"]["column"] == 0, tune["pinned"]["row"] == 0
+    else:
+        col, row = "pairs" in tune["choice"]["column"], "pairs" in tune["choice"]["row"]
+    return col and row, row           # pair columns read what pair rows write
+
+
+def algorithmic_bytes(n, m, pair_cols=True, pair_rows=True):
     """Per-launch algorithmic HBM bytes of each kernel class (averaged over the 3 stages)."""
     rb = _rows_in_band(n)
     c = 8 * n * n
-    phys = 2 * c + 8 * n * rb + c / 3.0                  # PA+PB read, in-band Z rows written, vel at stage 2
-    spec = 8 * n * rb + 4 * c + 2 * c / 3.0              # Z rows, wcur, wout, PA, PB; w0 at stages 1-2
+    half = 4 * n * rb                                    # PB's rows ky >= 0
+    z = 8 * n * rb                                       # in-band rows of Z, or of PA
+    vel = c / 3.0                                        # at stage 2
+    phys = z + half + z + vel if pair_cols else 2 * c + z + vel
+    if pair_rows:
+        spec = z + 64 * rb * rb / 3.0 + z + (half if pair_cols else z)   # Z, wcur, wout (w0 at stages 1-2), PA, PB
+    else:
+        spec = z + 4 * c + 2 * c / 3.0
     dye = 16 * m * m + 8 * n * n                         # one dye texture read + one written, velocity read
     return {"phys_cols": phys, "spec_rows": spec, "dye": dye}
 
 
-def step_algorithmic_bytes(n):
-    """Minimum-pass dataflow of one RK3 step, 232 N^2 bytes (dye and pointer forcing excluded)."""
-    return 232 * n * n
+def step_algorithmic_bytes(n, pairs=True, vel=True):
+    """Dataflow of one RK3 step (dye and pointer forcing excluded): the pair kernels' in-band cells, or
+    232 N^2 bytes of the kernels that take any state."""
+    if not pairs:
+        return 232 * n * n
+    b = algorithmic_bytes(n, n)
+    return 3 * (b["phys_cols"] + b["spec_rows"]) - (0 if vel else 8 * n * n)
 
 
 def load_peaks():
@@ -372,7 +391,7 @@ def run_ours(args):
     # pinned with --shapes (reproducible profiling)
     tune = pinned_shapes(solver, args.shapes) if args.shapes else solver.autotune(20)
 
-    # warm-up (also captures the graphs of the 6 (phase, dt slot, dye parity) combinations)
+    # warm-up (also captures the graph of six steps that the timed ones replay)
     solver.step(max(args.warmup, 6), dye=True, reduce=True, graph=True, relatch=True)
     solver.synchronize()
 
@@ -397,7 +416,7 @@ def run_ours(args):
     value = world * args.steps / (ms / 1e3)
 
     # ---- RK3-only (no dye) for reference
-    solver.step(3, dye=False, reduce=True, graph=True, relatch=True)
+    solver.step(6, dye=False, reduce=True, graph=True, relatch=True)    # captures their graph of six
     solver.synchronize()
     ev0.record(stream)
     solver.step(args.steps, dye=False, reduce=True, graph=True, relatch=True)
@@ -418,20 +437,23 @@ def run_ours(args):
         solver.step(ksteps, dye=True, reduce=True, graph=False, relatch=True)
         prof = solver.profileRead()
     solver.profile(False)
-    ab = algorithmic_bytes(N, N * DYE_SCALE)
+    pairs, pair_rows = pair_stages(tune)
+    ab = algorithmic_bytes(N, N * DYE_SCALE, pairs, pair_rows)
     hbm, bf16, peak_src = load_peaks()
     dom = max(("phys_cols", "spec_rows", "dye"), key=lambda k: prof[k][0])
     dom_ms, dom_n = prof[dom]
     avg_launch_s = dom_ms / 1e3 / max(dom_n, 1)
     achieved = ab[dom] / avg_launch_s / 1e9
-    kernel_names = {"phys_cols": "k_pair_cols", "spec_rows": "k_pair_rows", "dye": "k_dye_fused"}
-    traffic = committed_traffic(kernel_names[dom].split()[0])
+    kernel_names = {"phys_cols": "k_pair_cols" if pairs else "k_phys_cols",
+                    "spec_rows": "k_pair_rows" if pair_rows else "k_spec_rows", "dye": "k_dye_fused"}
+    traffic = committed_traffic(kernel_names[dom])
     step_ms = ms / args.steps if world == 1 else ms / args.steps
     roofline = {"bound": "hbm", "kernel": kernel_names[dom], "achieved": achieved, "peak": hbm, "unit": "GB/s",
                 "frac": achieved / hbm, "traffic": traffic, "peak_source": peak_src,
                 "algorithmic_bytes_per_launch": ab[dom], "avg_launch_ms": avg_launch_s * 1e3,
                 "per_kernel_ms_per_step": {k: prof[k][0] / ksteps for k in prof}}
-    step_roof = step_algorithmic_bytes(N) / ((ms_rk3 / args.steps) / 1e3) / 1e9
+    step_bytes = step_algorithmic_bytes(N, pairs)
+    step_roof = step_bytes / ((ms_rk3 / args.steps) / 1e3) / 1e9
 
     # ---- end to end through the public API: per step configure + splats + step + diagnostics
     # read.  Reads run one step behind, as the reference app's frame loop does (its
@@ -464,8 +486,8 @@ def run_ours(args):
     e2e_value = world * e2e_steps / e2e_s
     nb = N // 2 + 1
     h2d = 64 + 16 + 8 * 48
-    # two copies per step on the diagnostics stream: a diagnostics block (FP64 bins + u32
-    # bins (+ totals), the zonal mean) and the current [dt, speed] slot
+    # one copy per step on the diagnostics stream: a diagnostics block (FP64 bins + u32 bins
+    # (+ totals), the zonal mean, the current [dt, speed])
     d2h = (nb + 2) * 8 + (nb + 2) * 4 + N * 4 + 2 * 4
     finite = d is not None and all(map(lambda v: v == v, [d["energy"], d["enstrophy"], d["dt"]]))
     solver.destroy()
@@ -495,13 +517,13 @@ def run_ours(args):
                        "hyperviscosity": f"p=4, nu4={NU4:.3g} (rate {VISC_RATE} at the cutoff)",
                        "drag": 1e-2, "autotune": tune},
             "rk3_only_steps_per_s": world * args.steps / (ms_rk3 / 1e3),
-            "step_roofline": {"bytes_per_step": step_algorithmic_bytes(N), "achieved_gbs": step_roof,
-                              "frac": step_roof / hbm, "note": "232 N^2 algorithmic bytes per RK3 step (no dye)"},
+            "step_roofline": {"bytes_per_step": step_bytes, "achieved_gbs": step_roof, "frac": step_roof / hbm,
+                              "note": "bytes the chosen stage kernels cannot do without, per RK3 step (no dye)"},
             "roofline": roofline,
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                     "steps": e2e_steps, "diagnostics_finite": bool(finite)},
-            # per timed step: 3 k_pair_cols + 3 k_pair_rows + k_dye_fused (the CFL reduction
-            # and the stepIndex latch are fused into them)
+            # per timed step: 3 column and 3 row kernels and k_dye_fused (the CFL reduction and
+            # the stepIndex latch are fused into them)
             "gpu_launches": args.steps * 7,
             "clocks": clk,
             "cpu_baseline": cpu,
@@ -524,7 +546,7 @@ def pinned_shapes(solver, spec):
 
 
 def _timed_steps(solver, stream, torch, steps, dye):
-    solver.step(3, dye=dye, reduce=True, graph=True, relatch=True)
+    solver.step(6, dye=dye, reduce=True, graph=True, relatch=True)      # captures the graph of six
     solver.synchronize()
     ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     ev0.record(stream)
@@ -651,19 +673,19 @@ def run_ensemble(pkg, torch, world, rank, dev, args, groups=ENSEMBLE_256, seed=1
     e.destroy()
     hbm, _, _ = load_peaks()
     ens_steps_per_s = steps / (ms / 1e3)
-    bytes_step = sum(step_algorithmic_bytes(n) * c for n, c in groups)
+    pairs, _ = pair_stages(tune)
+    bytes_step = sum(step_algorithmic_bytes(n, pairs, vel=False) * c for n, c in groups)
     gbs = bytes_step * ens_steps_per_s / 1e9
     out = {"instances": count_total, "sizes": {str(n): c for n, c in groups},
            "n": groups[0][0] if len(groups) == 1 else None, "ensemble_steps_per_s": ens_steps_per_s,
            "instance_steps_per_s": ens_steps_per_s * count_total, "ms_per_ensemble_step": ms / steps,
            "achieved_gbs": gbs, "hbm_peak_gbs": hbm, "frac_of_hbm": gbs / hbm, "finite": ok, "autotune": tune,
-           "note": "232 N^2 algorithmic bytes per instance-step; per-instance nu, beta, drag; graph-replayed"}
-    # the DRAM bytes the kernels actually move (ncu, committed under profiles/; recorded
-    # for the 256 x 256^2 ensemble): the stage kernels move the band's half of the packs
-    # only, fewer bytes than the algorithmic count, and this fraction is the one
-    # that says how close to the bandwidth bound they run
+           "note": "bytes the chosen stage kernels cannot do without; per-instance nu, beta, drag; graph-replayed"}
+    # the DRAM bytes the pair kernels move (ncu, committed under profiles/; recorded for the
+    # 256 x 256^2 ensemble), fewer than that count where the packs are still in L2: this fraction
+    # is the one that says how close to the bandwidth bound they run
     spec_b, phys_b = committed_traffic("k_ens_pair_rows"), committed_traffic("k_ens_pair_cols")
-    if spec_b and phys_b and tuple(groups) == ENSEMBLE_256:
+    if pairs and spec_b and phys_b and tuple(groups) == ENSEMBLE_256:
         moved = 3 * (spec_b + phys_b)
         out["dram_traffic"] = {"bytes_per_ensemble_step": moved, "gbs": moved * ens_steps_per_s / 1e9,
                                "frac_of_hbm": moved * ens_steps_per_s / 1e9 / hbm,

@@ -254,9 +254,10 @@ int s2d_encode_reduce(s2d_solver* s);                                    /* solv
 /* `substeps` repetitions of encodeStep (+ encodeDye, + encodeReduce per flags),
  * priming first when needed: the body of main.js:409-419. */
 int s2d_step(s2d_solver* s, int substeps, unsigned flags);
-/* As s2d_step, replayed from captured CUDA graphs: one of six substeps for every six of a run
- * (the state ring, the dt slots and the dye textures are then back where they were), one of a
- * single substep for the rest; the same results bit for bit. */
+/* As s2d_step, replayed from captured CUDA graphs: of six substeps (the state ring, the dt slots
+ * and the dye textures are then back where they were) and of a single one; the same results bit
+ * for bit.  The first run of a kind captures its graph of six where it starts, later runs go there
+ * by single substeps, or capture another where such runs keep coming. */
 int s2d_step_graph(s2d_solver* s, int substeps, unsigned flags);
 
 /* ---------------------------------------------------------------- diagnostics */
@@ -267,9 +268,9 @@ int s2d_step_graph(s2d_solver* s, int substeps, unsigned flags);
  * step call waits for them unless it is one fused step right after them), so the
  * results are those of the state at this call. */
 int s2d_encode_diagnostics(s2d_solver* s);
-/* solver.js:560-568: on the diagnostics stream, behind the spectra and the work enqueued
- * so far, copies the block the last s2d_encode_diagnostics filled and the [dt, speed]
- * slot current now. */
+/* solver.js:560-568: takes the [dt, speed] slot current now, on the solver's stream, and copies
+ * it with the block the last s2d_encode_diagnostics filled, on the diagnostics stream, behind the
+ * spectra and the work enqueued so far. */
 int s2d_copy_diagnostics(s2d_solver* s);
 /* 1 when the copied diagnostics have landed in host memory, 0 otherwise. */
 int s2d_poll_diagnostics(s2d_solver* s);

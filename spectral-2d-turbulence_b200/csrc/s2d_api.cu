@@ -164,8 +164,8 @@ struct s2d_solver {
   // Diagnostics stream (low priority): the k-space spectra of encodeDiagnostics and the
   // readback copies run there, behind the work the main stream had enqueued, and alongside
   // the next step.  The spectra read state[phase] of the step before them, which the next
-  // fused step reads but does not write; every other call that enqueues device work first
-  // orders the main stream after them (diag_order).
+  // fused step reads but does not write, and the dye and the reduction do not touch; every other
+  // call that enqueues device work first orders the main stream after them (diag_order).
   cudaStream_t diag_stream = nullptr;
   cudaEvent_t diag_ready = nullptr;     // main-stream point the diagnostics stream waits for
   cudaEvent_t diag_done = nullptr;      // the last spectra launch has finished
@@ -395,8 +395,9 @@ static int diag_order(s2d_solver* s) {
 }
 // Every entry point that enqueues device work (or reads the device) flushes the host
 // blocks and orders the main stream after the outstanding spectra; the step entry points
-// order only where a step may write what the spectra read (diag_order_step), and the
-// readback calls, which use the diagnostics stream, do not order.
+// order only where a step may write what the spectra read (diag_order_step), the dye and the
+// reduction touch nothing of theirs, and the readback calls use the diagnostics stream: these
+// do not order.
 #define S2D_USE_NOORDER(s)                           \
   do {                                               \
     S2D_USE_HOST(s);                                 \

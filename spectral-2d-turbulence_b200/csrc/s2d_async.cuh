@@ -93,13 +93,16 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // Programmatic dependent launch: a stage kernel may start while the one before it drains.
 // pdl_wait returns once that kernel has finished (and its writes are visible); every kernel
 // lets its successor start only after its own wait, so whatever ran two or more launches
-// back is complete when a kernel starts -- its prologue may read that, and nothing newer.
+// back is complete when a kernel starts -- its prologue may read that, and nothing newer.  So what
+// a kernel reads ahead of its wait must not be written by the launch directly before it:
+// k_pair_rows reads the step size, the parameters and its first state cells there, and must follow
+// a column kernel (the prime, which follows whatever wrote the state, is launched in full order).
 __device__ __forceinline__ void pdl_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// a kernel that begins with pdl_wait, launched with programmatic stream serialisation
+// a kernel that calls pdl_wait, launched with programmatic stream serialisation
 template <class... P, class... A>
 inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, const A&... args) {
   cudaLaunchAttribute attr{};

@@ -97,7 +97,8 @@ struct PhysArgs {
 // the per-substep stepIndex latch (S2D_STEP_RELATCH): params.step_index = counter++,
 // the step index a configure() before this substep would latch (solver.js:316); done by
 // one thread of the first stage's column kernel, since nothing in that kernel reads
-// step_index and its first reader (the row kernel's stochastic forcing) is the next launch
+// step_index: its first reader, the row stage's stochastic forcing, is the next launch (or comes
+// behind a cluster barrier, in a step of one launch)
 __device__ __forceinline__ void phys_latch(const PhysArgs& a) {
   if (a.latch && blockIdx.x == 0 && threadIdx.x == 0) {
     const uint32_t k = *a.counter;

@@ -382,10 +382,12 @@ template <int NTHREADS> __device__ __forceinline__ void cols_speed_max(unsigned*
   if (threadIdx.x == 0) atomicMax(top, m);
 }
 
-// Bound by latency up to 1024^2 (one wave; see the head of this file), beyond that by shared
-// memory's wavefronts and, at 4096^2, HBM.  The stage is a run-time argument, as in the row
-// kernel: three copies of the code fetched anew by each launch cost more than the tests.
-// 1024^2 7.2 us a launch (k_phys_cols 14), 2048^2 33, 4096^2 109.
+// Bound by latency: up to 1024^2 one wave (see the head of this file); beyond, one CTA of 512
+// threads on an SM at 128 registers, whose loads, transforms and stores have nothing beside them
+// (cold, stage 1: 2048^2 L1 wavefronts 40 %, issue slots 34 %, HBM 10 %; 4096^2 56, 40 and 19 %).
+// The stage is a run-time argument, as in the row kernel: three copies of the code fetched anew by
+// each launch cost more than the tests.  1024^2 7.2 us a launch (k_phys_cols 14), 2048^2 33,
+// 4096^2 109.
 template <class TU>
 __global__ void __launch_bounds__(TU::THREADS, TU::MINB) k_pair_cols(PhysArgs a, int mode) {
   extern __shared__ __align__(16) float4 smem4[];

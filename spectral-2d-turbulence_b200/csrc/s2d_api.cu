@@ -656,9 +656,10 @@ static void pair_row_args(s2d_solver* s, SpecArgs* a) {
   a->dt_out = dt_slot(s, s->slot ^ 1);
   a->full_pb = pair_cols(s) ? 0 : 1;
 }
-// the row stage with the solver's chosen variant
-static void run_spec(s2d_solver* s, int mode, bool ptr, SpecArgs a) {
+// the row stage with the solver's chosen variant; `whole`: packs in rows, both halves of PB
+static void run_spec(s2d_solver* s, int mode, bool ptr, SpecArgs a, bool whole = false) {
   pair_row_args(s, &a);
+  if (whole) a.full_pb = 1;
   if (tc_rows(s)) {
     if (s->fft_precision == S2D_FFT_TC_BF16) tc_rows_launch<tc::PrecBF16>(mode, ptr, a, s->tctab, s->stream);
     else tc_rows_launch<tc::PrecF16>(mode, ptr, a, s->tctab, s->stream);
@@ -967,7 +968,7 @@ static int enqueue_fft2(s2d_solver* s, float2* buf, int sign) {
 }
 
 // prime packs from state[phase]: PA/PB = FFT_x^-1 of the scaled packs
-static int enqueue_pack_prime(s2d_solver* s) {
+static int enqueue_pack_prime(s2d_solver* s, bool whole = false) {
   SpecArgs a{};
   a.wcur = s->state[s->phase];
   a.pa = s->packA;
@@ -982,9 +983,13 @@ static int enqueue_pack_prime(s2d_solver* s) {
     k_band_flags<<<(s->n + 255) / 256, 256, 0, s->stream>>>(s->row_nz, s->n);
     S2D_LAUNCHED();
   }
-  run_spec(s, -1, false, a);
+  run_spec(s, -1, false, a, whole);
   S2D_LAUNCHED();
   mark_packs(s);
+  if (whole) {
+    s->packs_half = false;
+    s->packs_blocked = 0;
+  }
   return S2D_OK;
 }
 
@@ -1003,11 +1008,14 @@ static int unblock_pack_on_host(s2d_solver* s, float2* p) {
   return S2D_OK;
 }
 
-// Blocked packs to rows, in place.  The pair columns read blocks, so the packs no longer serve the
-// next step (it makes them again from the state); a pack is marked as its rewrite is enqueued, so
-// that a call after a failed one goes on with the other.
+// Blocked packs to rows: those of state[phase] formed again from it, the same bits (4096^2: 0.13 ms);
+// those that an earlier state left behind in place, through a second copy (2 ms, most of it the
+// allocation).  Either way they no longer serve the pair columns, which read blocks, and the next
+// step makes its own.  A pack is marked as its rewrite is enqueued, so that a call after a failed
+// one goes on with the other.
 static int unblock_packs(s2d_solver* s) {
   if (!s->packs_blocked) return S2D_OK;
+  if (packs_fit(s)) return enqueue_pack_prime(s, true);
   s->packs_valid = false;
   const size_t cbytes = (size_t)s->n * s->n * sizeof(float2);
   float2* tmp = nullptr;
@@ -1969,10 +1977,10 @@ extern "C" int s2d_velocity_pack(s2d_solver* s, int state_index) {
   S2D_USE(s);
   if (state_index < 0 || state_index > 2) return fail(S2D_ERR_ARG, "state index out of range");
   DeviceGuard guard(s->dev);
-  if (int rc = materialize_packs(s)) return rc;
   k_velocity_pack<<<cells_grid(s->n), 256, 0, s->stream>>>(s->state[state_index], s->packA, s->packB, s->n);
   S2D_LAUNCHED();
-  s->packs_valid = false;
+  s->packs_valid = s->packs_flagged = false;   // both packs are written whole
+  s->packs_blocked = 0;
   return S2D_OK;
 }
 

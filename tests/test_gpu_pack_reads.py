@@ -52,3 +52,24 @@ def test_a_second_read_returns_the_first(pkg):
         assert np.array_equal(first[1][1], np.conj(first[1][-1])) and np.any(first[1][1])
     finally:
         s.destroy()
+
+
+@pytest.mark.parametrize("n", [1024, 4096])
+def test_packs_of_an_earlier_state_are_kept(pkg, n):
+    """The packs as the last step left them, read at once and after the state they belong to has been
+    replaced: the same bits, whichever way the read puts them in rows."""
+    out = []
+    for stale in (False, True):
+        s = pkg.Solver.create(n=n, dyeScale=1)
+        try:
+            s.configure(config(viscosity=1.0, hyperP=2, dtMax=1e-3))
+            s.reset({"k0": 6, "amplitude": 3, "seed": 5, "dyePattern": "none"})
+            s.step(2, dye=False)
+            if stale:
+                s.setBuffer("state%d" % s.phase, np.zeros((n, n), np.complex64))
+            out.append([s.getBuffer("packA"), s.getBuffer("packB")])
+        finally:
+            s.destroy()
+    assert np.any(out[0][0]) and np.any(out[0][1])
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)

@@ -23,11 +23,13 @@ def kernels(rec):
 
 
 def test_a_pack_is_unblocked_once(library):
-    """4096^2, no room on the device and the second pack's transfer fails: the first pack, already in
-    rows, is not rewritten by the read that follows, and the next step makes the packs again."""
+    """4096^2, packs of an earlier phase, no room on the device and the second pack's transfer fails:
+    the first pack, already in rows, is not rewritten by the read that follows, and the next step
+    makes the packs again."""
     host_runtime.run(library, START + """
 s = solver(4096)
 s.step(1, dye=False)
+s.phase = 0
 def read(name):
     try:
         s.getBuffer(name)
@@ -51,6 +53,24 @@ names = kernels(Record(pkg.host))
 assert sum("k_pair_rows" in k for k in names) == 4, names    # three stages, and the packs before them
 s.encodeStep()
 assert sum("k_pair_rows" in k for k in kernels(Record(pkg.host))) == 7
+""")
+
+
+@pytest.mark.parametrize("call", ["s.getBuffer('packA')", "s.nlPack()", "s.fft.forward(None, 'packB')", "s.velocityPack(0)",
+                                  "s.seedPhysical(np.ones(4096 * 4096, np.float32))"])
+def test_calls_on_the_packs_allocate_nothing(library, call):
+    """4096^2, the packs of the current state: put in rows without device memory for a second copy and
+    without a way through host memory."""
+    host_runtime.run(library, START + f"""
+s = solver(4096)
+s.step(1, dye=False)
+pkg.host.host_fail(b"cudaMallocAsync", 0, 1)
+pkg.host.host_forget()
+{call}
+rec = Record(pkg.host)
+moved = [op for op in rec.ops if op[0] in ("upload", "copy") and int(op[2][2]) > 1 << 26]
+assert not moved, moved
+s.encodeStep()
 """)
 
 
